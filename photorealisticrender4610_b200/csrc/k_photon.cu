@@ -1410,10 +1410,13 @@ int prr_photon_emit(prr_photon_map *pmap, const prr_scene *scene, int64_t num_ph
     int64_t capacity = std::max<int64_t>(num_photons, 1 << 16);
     for (int attempt = 0; attempt < 2; attempt++) {
         const int64_t n2 = pow2_at_least(capacity);
-        PRR_CUDA_TRY(pm.scratch.ensure((size_t) capacity * 9 * sizeof(float) + n2 * 8 + 64));
+        // the 8-byte keys start on a 256-byte boundary whatever the record count
+        // (36 bytes a record: an odd capacity would leave them at 4 mod 8)
+        const size_t rec_bytes = ((size_t) capacity * 9 * sizeof(float) + 255) & ~size_t(255);
+        PRR_CUDA_TRY(pm.scratch.ensure(rec_bytes + (size_t) n2 * 8 + 64));
         float *rec = pm.scratch.as<float>();
         unsigned long long *keys =
-            reinterpret_cast<unsigned long long *>((char *) pm.scratch.ptr + capacity * 9 * 4);
+            reinterpret_cast<unsigned long long *>((char *) pm.scratch.ptr + rec_bytes);
         unsigned *count = reinterpret_cast<unsigned *>((char *) keys + n2 * 8);
         PRR_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(unsigned), st));
         EmitArgs a{num_photons, seed, max_depth, rec, keys, count, capacity, tcap};

@@ -372,3 +372,19 @@ def test_grid_large_map_sorted_in_stages(ref, cuda):
     n1 = small.launches()
     small.build(0.02)
     assert small.launches() - n1 <= 12  # one sort launch among the build's kernels
+
+
+@pytest.mark.parametrize("n", [65_537, 100_001])
+def test_emit_odd_photon_count(cuda, n):
+    """An odd number of photons (36-byte records, so the 8-byte sort keys
+    behind them need their own alignment): every photon's first stored record
+    is where a trace of one photon more puts it, up to the power's 1/n."""
+    s = prr.Scene.from_desc(scenes.caustics(64, 64, level=2))
+    recs, owners = zip(*(prr.PhotonMap().emit(s, m, seed=3).export() for m in (n, n + 1)))
+    firsts = [dict(zip(*np.unique(o, return_index=True))) for o in owners]
+    common = [k for k in firsts[0] if k in firsts[1]]
+    assert len(common) > 0.99 * len(firsts[0]) > 500
+    a = recs[0][[firsts[0][k] for k in common]]
+    b = recs[1][[firsts[1][k] for k in common]]
+    assert np.array_equal(a[:, :6].view(np.uint32), b[:, :6].view(np.uint32))
+    assert np.allclose(a[:, 6:], b[:, 6:] * ((n + 1) / n), rtol=1e-5)
