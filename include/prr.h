@@ -75,7 +75,8 @@ typedef struct prr_camera {
 /* Traversal launch shape (chosen by the autotuner; zero fields = defaults). */
 typedef struct prr_trace_config {
     int block_size;   /* threads per block (multiple of 32) */
-    int persistent;   /* 0: one ray per thread; 1: persistent grid, each warp
+    int persistent;   /* 0: by batch size (small ones spread over all warps, larger
+                         ones as mode 2); 1: persistent grid, each warp
                          takes 32 rays at a time; 2: persistent grid, lanes whose
                          ray finished take new rays as soon as `batch` lanes of the
                          warp are idle; 3: as 2, with postponed leaves (node and

@@ -49,6 +49,23 @@ struct alignas(64) WNode {
 };
 static_assert(sizeof(WNode) == 64, "WNode must be 64 bytes");
 
+// Four-wide node of a mesh BVH: two levels of the binary tree in one 128-byte
+// line, so a walk makes about half as many dependent fetches. Children 0 and 1
+// are those of the binary node's left child, 2 and 3 those of its right child;
+// a side that is a leaf (or whose box is not exactly the union of its
+// children's, see pack_quads) fills its first slot alone and its second slot
+// holds an inverted box (+inf..-inf, entered by no ray) and the first's
+// reference. Planes are stored axis by axis, the four minima then the four
+// maxima (32 bytes, one load), the order the four slab tests consume them in.
+// The walk over these nodes takes the same leaves in the same order as the
+// walk over the binary tree (trace.cuh, quad_test).
+struct alignas(128) QNode {
+    float plane[3][2][4]; // [axis][min, max][child]
+    uint32_t ref[4];      // interior: QNode index; leaf: mesh_leaf_ref
+    uint32_t pad[4];
+};
+static_assert(sizeof(QNode) == 128, "QNode must be 128 bytes");
+
 // One triangle in leaf order (orderedPrims order): v0, e1 = v1-v0, e2 = v2-v0
 // exactly as Triangle's constructor computes them (Triangle.hpp:27-31). The
 // intersection test reads 36 bytes: the first eight floats as one 32-byte
@@ -74,7 +91,7 @@ enum MaterialKind : int32_t { kMatDiffuse = 0, kMatEmissive = 1, kMatMirror = 2,
 struct alignas(16) DevObject {
     int32_t kind;
     int32_t material;
-    uint32_t root;      // mesh: root reference into nodes/tris
+    uint32_t root;      // mesh: root reference into nodes/tris (light sampling)
     int32_t tri_base;   // mesh: first triangle (global index)
     float root_box[6];  // own bounds (IntersectP tests the root box first)
     float area;         // MeshTriangle::area or Sphere::area
@@ -84,7 +101,8 @@ struct alignas(16) DevObject {
     int32_t depth;      // max leaf depth of the mesh BVH (stack bound)
     int32_t attr;       // mesh: kAttr* bits of the per-corner data it carries
     int32_t attr_base;  // mesh: its first record in DevScene::attr
-    int32_t pad[2];
+    uint32_t qroot;     // mesh: root reference into qnodes/tris (the traversals')
+    int32_t pad[1];
 };
 
 // Per-corner mesh data of Triangle (Triangle.hpp:17-23), one record of
@@ -134,6 +152,7 @@ struct DevEnv {
 
 struct DevScene {
     const WNode *nodes;
+    const QNode *qnodes;       // four-wide mesh nodes
     const Tri *tris;
     const float *tri_e2z;      // e2.z of each triangle (completes Tri)
     const TriMeta *tri_meta;   // input id and area of each triangle
@@ -153,12 +172,13 @@ struct DevScene {
     float tlas_box[6];
     int32_t tlas_depth;
     int32_t blas_depth;   // max over meshes
+    int32_t blas_stack;   // entries a mesh walk's stack may need, max over meshes
     float background[3];
     DevCamera camera;
     DevEnv env;
     // bounds of the node and triangle arrays and the scene's status words,
     // read only by the checked build (compiled with -DPRR_CHECKED)
-    uint32_t n_nodes, n_tris;
+    uint32_t n_nodes, n_qnodes, n_tris;
     uint32_t *check;
 };
 

@@ -311,12 +311,12 @@ __global__ void k_wf_begin(Wf w, int it) {
 // `refill` lanes of its warp are idle (one atomic per refill).
 // The scene-level stack of this thread (all in shared memory) and its mesh-level
 // stack (blas_sm entries in shared memory, the rest in the spill buffer).
-template <class E>
-__device__ __forceinline__ void make_stacks(const Wf &w, E *smem, StackCol<E> &tc,
-                                            StackCol<E> &bc) {
-    tc = StackCol<E>{smem + threadIdx.x, nullptr, w.tlas_cap, w.tlas_cap, w.check};
-    bc = StackCol<E>{smem + (size_t) w.tlas_cap * blockDim.x + threadIdx.x, (E *) w.spill,
-                     w.blas_sm, w.blas_cap, w.check};
+template <class E> __device__ __forceinline__ StackCol<E> scene_stack(const Wf &w, E *smem) {
+    return StackCol<E>(smem, nullptr, w.tlas_cap, w.tlas_cap, w.check);
+}
+template <class E> __device__ __forceinline__ StackCol<E> mesh_stack(const Wf &w, E *smem) {
+    return StackCol<E>(smem + (size_t) w.tlas_cap * blockDim.x, (E *) w.spill, w.blas_sm,
+                       w.blas_cap, w.check);
 }
 
 template <bool MULTI>
@@ -330,8 +330,7 @@ __device__ __forceinline__ const DevScene &lane_scene(const DevScene &S0, const 
 template <bool MULTI, bool STATS>
 __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int it, int refill) {
     extern __shared__ uint2 smem[];
-    StackCol<uint2> tc, bc;
-    make_stacks(w, smem, tc, bc);
+    const StackCol<uint2> tc = scene_stack(w, smem), bc = mesh_stack(w, smem);
     const int *qin = w.qray[it & 1];
     const int n = queue_len(w, w.cnt[kCntRay0 + (it & 1)], w.P);
     const unsigned full = 0xffffffffu;
@@ -339,7 +338,7 @@ __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int i
     int p = -1;
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    ClosestWalk cw;
+    ClosestWalk<STATS> cw;
     unsigned cnt_[6] = {0, 0, 0, 0, 0, 0}; // nodes, tris, objects, miss, delta, surface
     bool more = n > 0;
     if (!more)
@@ -374,7 +373,8 @@ __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int i
                     ls = w.reqs[r].scene;
                 }
                 const float4 o = w.ro[p], d = w.rd[p];
-                cw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z});
+                cw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z},
+                         tc);
             }
             if constexpr (MULTI)
                 count_req_rays(w, full, take, r, 0);
@@ -761,15 +761,14 @@ __global__ void __launch_bounds__(128, 8) k_wf_surface(DevScene S0, Wf w, int it
 template <bool MULTI, bool STATS>
 __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int refill) {
     extern __shared__ uint32_t smem32[];
-    StackCol<uint32_t> tc, bc;
-    make_stacks(w, smem32, tc, bc);
+    const StackCol<uint32_t> tc = scene_stack(w, smem32), bc = mesh_stack(w, smem32);
     const int n = queue_len(w, w.cnt[kCntShadowJobs], 2 * (int64_t) w.P);
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int job = -1;
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    AnyWalk aw;
+    AnyWalk<STATS> aw;
     bool more = n > 0;
     unsigned rays = 0;
     unsigned cnt_[3] = {0, 0, 0}; // nodes, tris, objects
@@ -799,7 +798,8 @@ __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int r
                 const float4 o = (job & 1) ? w.seo[p] : w.slo[p];
                 const float4 d = (job & 1) ? w.sed[p] : w.sld[p];
                 rays++;
-                if (!aw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z}, o.w)) {
+                if (!aw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z}, o.w,
+                              tc)) {
                     w.vis[job] = 1;
                     job = -1;
                 }
@@ -826,22 +826,21 @@ __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int r
                   (unsigned long long) rays);
 }
 
-// The traversal stages held to 48 registers (no spills): 10 resident blocks of
-// 128 (or 21 of 64) instead of 9 at the 54-56 they take otherwise; the
-// museum-like frame 216.6 -> 213.5 ms.
+// The traversal stages on the four-wide nodes, 64 registers at most (8 resident
+// blocks of 128). Tighter caps gain blocks but spill the four boxes' distances:
+// museum-like scene of 491,520 triangles at 960x540, 16 spp: 16.9 ms, 17.6 at
+// 56 registers, 19.0 at 48; 18.5 on the binary nodes (at their best cap, 48).
 template <bool MULTI, bool STATS = false>
-__global__ void __maxnreg__(48) k_wf_extend(DevScene S, Wf w, int it, int refill) {
+__global__ void __maxnreg__(64) k_wf_extend(DevScene S, Wf w, int it, int refill) {
     wf_extend<MULTI, STATS>(S, w, it, refill);
 }
 // The server's extend stage (paths of several requests; the request index
-// selects scene and camera), held to 48 registers like the others: 10
-// resident blocks of 128 instead of 8 at the 64 it takes otherwise (16 bytes
-// of spills).
-__global__ void __maxnreg__(48) k_wf_extend_multi(DevScene S, Wf w, int it, int refill) {
+// selects scene and camera).
+__global__ void __maxnreg__(64) k_wf_extend_multi(DevScene S, Wf w, int it, int refill) {
     wf_extend<true, false>(S, w, it, refill);
 }
 template <bool MULTI, bool STATS = false>
-__global__ void __maxnreg__(48) k_wf_shadow(DevScene S, Wf w, int refill) {
+__global__ void __maxnreg__(64) k_wf_shadow(DevScene S, Wf w, int refill) {
     wf_shadow<MULTI, STATS>(S, w, refill);
 }
 
@@ -1417,7 +1416,7 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.seed = rs.seed;
     w.sample_offset = rs.sample_offset;
     w.tlas_cap = S.tlas_depth + 1;
-    w.blas_cap = S.blas_depth + 1;
+    w.blas_cap = (s.wf_stats ? S.blas_depth : S.blas_stack) + 1;
     // paths per pass: whole samples of the window, about 8M paths in flight
     const int64_t target = s.wf_paths > 0 ? s.wf_paths : (int64_t) 1 << 23;
     int spp_pass = (int) std::max<int64_t>(1, target / std::max(1, w.npix));

@@ -89,6 +89,8 @@ struct HostObject {
     float area = 0.f;
     int tri_base = 0;
     uint32_t root = 0;
+    uint32_t qroot = 0; // root over the four-wide nodes
+    int qstack = 0;     // stack entries a walk over them may need
 };
 
 struct WavefrontPlan;
@@ -110,7 +112,7 @@ struct Scene {
     int64_t n_tris = 0;
     size_t device_bytes = 0;
 
-    DevBuf d_nodes, d_tris, d_tri_e2z, d_tri_meta, d_verts, d_normals, d_objects, d_materials,
+    DevBuf d_nodes, d_qnodes, d_tris, d_tri_e2z, d_tri_meta, d_verts, d_normals, d_objects, d_materials,
         d_emissives;
     std::vector<HostTexture> textures;
     DevBuf d_attr, d_texels, d_textures;

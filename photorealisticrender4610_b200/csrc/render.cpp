@@ -178,7 +178,7 @@ extern "C" int prr_autotune(prr_scene *scene, const prr_render_settings *setting
     };
     // stage 1: paths per pass x block size, ordered queues, 8 shared stack
     // entries (the rest of the L1 caches nodes and triangles)
-    const int stack1 = std::min(8, s.dev.blas_depth + 1);
+    const int stack1 = std::min(8, s.dev.blas_stack + 1);
     int64_t last = -1;
     for (int64_t cand : paths) {
         // a pass never holds more than the whole render
@@ -193,7 +193,7 @@ extern "C" int prr_autotune(prr_scene *scene, const prr_render_settings *setting
     // stage 2: at that shape, other shared stack depths (0: the whole stack)
     const prr_wavefront_config shape = best;
     for (int sk : {0, 16, 4, 2})
-        if (rc == PRR_OK && sk < s.dev.blas_depth + 1 && sk != stack1)
+        if (rc == PRR_OK && sk < s.dev.blas_stack + 1 && sk != stack1)
             trial(prr_wavefront_config{shape.paths_per_pass, shape.block_size, 1, sk, 1, 0});
     // stage 3: append-order queues
     const prr_wavefront_config shape2 = best;

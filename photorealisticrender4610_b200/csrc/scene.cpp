@@ -81,6 +81,101 @@ int pack_tree(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<WN
     return PRR_OK;
 }
 
+// Stack entries a walk over four-wide nodes may need before the mesh keeps
+// the binary shape (two children a node, one entry per level): the stacks of
+// the query kernels live in shared memory, which a deep tree's three entries
+// per two levels would outgrow sooner.
+constexpr int kMaxQuadStack = 64;
+
+// Collapse one mesh's tree into four-wide nodes (QNode) appended to `out`:
+// node, grandchildren, great-great-grandchildren and so on. A child is
+// collapsed when it is interior and its box is exactly the union of its
+// children's boxes, which the walk's exactness rests on (a NaN in a box fails
+// the comparison); otherwise it stays a child of its own. Returns the root
+// reference and how many entries a walk's stack can hold: every child of a
+// node but the one entered may wait on it.
+void pack_quads(const FlatBVH &f, int tri_base, std::vector<QNode> &out, uint32_t &root_ref,
+                int &stack) {
+    const size_t n = f.size();
+    auto count = [&](size_t i) { return f.meta[i] & 0x00FFFFFFu; };
+    auto leaf_ref = [&](size_t i) {
+        return mesh_leaf_ref((uint32_t) (tri_base + f.first_child[i]), count(i));
+    };
+    stack = 0;
+    if (n == 0 || count(0) > 0) {
+        root_ref = n ? leaf_ref(0) : 0;
+        return;
+    }
+    const float inf = std::numeric_limits<float>::infinity();
+    const size_t base = out.size();
+    for (const bool collapse : {true, false}) {
+        auto collapsible = [&](size_t i) {
+            if (!collapse || count(i) > 0)
+                return false;
+            const float *p = &f.bounds[i * 6], *l = &f.bounds[(i + 1) * 6],
+                        *r = &f.bounds[(size_t) f.first_child[i] * 6];
+            for (int k = 0; k < 6; k += 2)
+                if (!(p[k] == (l[k] < r[k] ? l[k] : r[k])) ||
+                    !(p[k + 1] == (l[k + 1] > r[k + 1] ? l[k + 1] : r[k + 1])) ||
+                    std::isnan(l[k]) || std::isnan(r[k]) || std::isnan(l[k + 1]) ||
+                    std::isnan(r[k + 1]))
+                    return false;
+            return true;
+        };
+        out.resize(base);
+        std::vector<size_t> todo{0};  // binary node of each four-wide node
+        todo.reserve(n / 3 + 1);
+        for (size_t w = 0; w < todo.size(); w++) {
+            const size_t i = todo[w];
+            QNode q;
+            std::memset(&q, 0, sizeof(q));
+            const size_t side[2] = {i + 1, f.first_child[i]};
+            for (int h = 0; h < 2; h++) {
+                size_t child[2] = {side[h], n};
+                if (collapsible(side[h])) {
+                    child[0] = side[h] + 1;
+                    child[1] = f.first_child[side[h]];
+                }
+                for (int c = 0; c < 2; c++) {
+                    const int slot = 2 * h + c;
+                    for (int a = 0; a < 3; a++) {
+                        q.plane[a][0][slot] = child[c] < n ? f.bounds[child[c] * 6 + 2 * a] : inf;
+                        q.plane[a][1][slot] =
+                            child[c] < n ? f.bounds[child[c] * 6 + 2 * a + 1] : -inf;
+                    }
+                    if (child[c] >= n) {
+                        q.ref[slot] = q.ref[slot - 1];
+                    } else if (count(child[c]) > 0) {
+                        q.ref[slot] = leaf_ref(child[c]);
+                    } else {
+                        q.ref[slot] = (uint32_t) (base + todo.size());
+                        todo.push_back(child[c]);
+                    }
+                }
+            }
+            out.push_back(q);
+        }
+        // children follow their parents, so a backward pass has theirs ready
+        std::vector<int> need(todo.size(), 0);
+        for (size_t w = todo.size(); w-- > 0;) {
+            const QNode &q = out[base + w];
+            int valid = 0, deepest = 0;
+            for (int c = 0; c < 4; c++) {
+                if ((c & 1) && q.ref[c] == q.ref[c - 1])
+                    continue; // an empty slot
+                valid++;
+                if (!(q.ref[c] & kLeafBit))
+                    deepest = std::max(deepest, need[q.ref[c] - base]);
+            }
+            need[w] = valid - 1 + deepest;
+        }
+        stack = need[0];
+        if (stack <= kMaxQuadStack)
+            break;
+    }
+    root_ref = (uint32_t) base;
+}
+
 template <class T> int upload(DevBuf &b, const std::vector<T> &v) {
     PRR_CUDA_TRY(b.alloc(std::max<size_t>(v.size() * sizeof(T), 16)));
     if (!v.empty())
@@ -209,6 +304,7 @@ int build_scene(Scene &s, cudaStream_t st) {
     std::vector<TriMeta> tri_meta;
     std::vector<float> verts, normals;
     std::vector<WNode> nodes;
+    std::vector<QNode> qnodes;
     int64_t ntri = 0;
     for (int k : meshes)
         ntri += (int64_t) s.objects[k].verts.size() / 9;
@@ -220,7 +316,7 @@ int build_scene(Scene &s, cudaStream_t st) {
     verts.resize((size_t) ntri * 9);
     normals.resize((size_t) ntri * 3);
     int base = 0;
-    int blas_depth = 0;
+    int blas_depth = 0, blas_stack = 0;
     for (int k : meshes) {
         HostObject &o = s.objects[k];
         o.tri_base = base;
@@ -275,6 +371,8 @@ int build_scene(Scene &s, cudaStream_t st) {
         }
         if (int rc = pack_tree(o.bvh, false, base, nodes, o.root))
             return rc;
+        pack_quads(o.bvh, base, qnodes, o.qroot, o.qstack);
+        blas_stack = std::max(blas_stack, o.qstack);
         blas_depth = std::max(blas_depth, o.bvh.max_depth);
         base += (int) nt;
     }
@@ -332,6 +430,7 @@ int build_scene(Scene &s, cudaStream_t st) {
         d.area = o.area;
         if (o.kind == kObjMesh) {
             d.root = o.root;
+            d.qroot = o.qroot;
             d.tri_base = o.tri_base;
             d.ntri = (int32_t) (o.verts.size() / 9);
             for (int q = 0; q < 6; q++)
@@ -404,6 +503,8 @@ int build_scene(Scene &s, cudaStream_t st) {
 
     if (int rc = upload(s.d_nodes, nodes))
         return rc;
+    if (int rc = upload(s.d_qnodes, qnodes))
+        return rc;
     if (int rc = upload(s.d_tris, tris))
         return rc;
     if (int rc = upload(s.d_tri_e2z, tri_e2z))
@@ -424,10 +525,12 @@ int build_scene(Scene &s, cudaStream_t st) {
     DevScene &D = s.dev;
     std::memset(&D, 0, sizeof(D));
     D.nodes = s.d_nodes.as<WNode>();
+    D.qnodes = s.d_qnodes.as<QNode>();
     D.tris = s.d_tris.as<Tri>();
     D.tri_e2z = s.d_tri_e2z.as<float>();
     D.tri_meta = s.d_tri_meta.as<TriMeta>();
     D.n_nodes = (uint32_t) nodes.size();
+    D.n_qnodes = (uint32_t) qnodes.size();
     D.n_tris = (uint32_t) ntri;
     // status words of the checked build's device-side tests (prr_check_status)
     PRR_CUDA_TRY(s.d_check.alloc(4 * sizeof(uint32_t)));
@@ -454,6 +557,7 @@ int build_scene(Scene &s, cudaStream_t st) {
             D.tlas_box[q] = s.tlas.bounds[q];
     D.tlas_depth = s.tlas.max_depth;
     D.blas_depth = blas_depth;
+    D.blas_stack = blas_stack;
     std::memcpy(D.background, s.background, sizeof(D.background));
 
     if (s.camera_set)
@@ -495,7 +599,7 @@ int build_scene(Scene &s, cudaStream_t st) {
     PRR_CUDA_TRY(cudaStreamSynchronize(st));
     s.n_tris = ntri;
     s.device_bytes = s.d_attr.bytes + s.d_texels.bytes + s.d_textures.bytes +
-                     s.d_nodes.bytes + s.d_tris.bytes + s.d_tri_e2z.bytes + s.d_tri_meta.bytes +
+                     s.d_nodes.bytes + s.d_qnodes.bytes + s.d_tris.bytes + s.d_tri_e2z.bytes + s.d_tri_meta.bytes +
                      s.d_verts.bytes + s.d_normals.bytes +
                      s.d_objects.bytes + s.d_materials.bytes + s.d_emissives.bytes +
                      s.d_env_px.bytes + s.d_env_cdf.bytes + s.d_env_marginal.bytes +
@@ -861,8 +965,8 @@ int prr_mesh_intersect(const prr_scene *scene, int object, const float *o, const
     if (n < 0 || (n > 0 && (!o || !d || !out_id || !out_t)))
         return fail(PRR_ERR_INVALID_ARGUMENT, "bad ray or output arrays");
     const Scene *s = S(scene);
-    return launch_mesh_closest(*s, object, o, d, n, out_id, out_t, out_t64,
-                               (unsigned *) s->d_counter.ptr, cfg, (cudaStream_t) stream);
+    return launch_mesh_closest(*s, object, o, d, n, out_id, out_t, out_t64, nullptr, cfg,
+                               (cudaStream_t) stream);
 }
 
 int prr_mesh_intersect_host(prr_scene *scene, int object, const float *o, const float *d,

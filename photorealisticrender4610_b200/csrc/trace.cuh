@@ -45,12 +45,12 @@ __device__ __forceinline__ void check_fail(uint32_t *status, uint32_t code, uint
 
 // What a checked fetch tests against.
 struct TraceBounds {
-    uint32_t n_nodes, n_tris;
+    uint32_t n_nodes, n_qnodes, n_tris;
     uint32_t *check;
 };
 
 __device__ __forceinline__ TraceBounds bounds_of(const DevScene &S) {
-    return TraceBounds{S.n_nodes, S.n_tris, S.check};
+    return TraceBounds{S.n_nodes, S.n_qnodes, S.n_tris, S.check};
 }
 
 struct RayD {
@@ -211,6 +211,173 @@ __device__ __forceinline__ NodeV load_node(const WNode *nodes, uint32_t idx) {
     return n;
 }
 
+// ---- four-wide nodes
+
+struct QuadV {
+    float4 mn[3], mx[3]; // per axis: the four children's minima, maxima
+    uint4 ref;
+};
+
+__device__ __forceinline__ QuadV load_quad(const QNode *nodes, uint32_t idx,
+                                           const TraceBounds &B) {
+    QuadV n;
+#ifdef PRR_CHECKED
+    if (idx >= B.n_qnodes) {
+        check_fail(B.check, kCheckNode, idx);
+        for (int a = 0; a < 3; a++) { // four empty boxes: no slab test enters them
+            n.mn[a] = make_float4(kInf, kInf, kInf, kInf);
+            n.mx[a] = make_float4(-kInf, -kInf, -kInf, -kInf);
+        }
+        n.ref = make_uint4(kLeafBit, kLeafBit, kLeafBit, kLeafBit);
+        return n;
+    }
+#endif
+    (void) B;
+    const float4 *q = reinterpret_cast<const float4 *>(nodes + idx);
+    ldg256(q, n.mn[0], n.mx[0]);
+    ldg256(q + 2, n.mn[1], n.mx[1]);
+    ldg256(q + 4, n.mn[2], n.mx[2]);
+    n.ref = __ldg(reinterpret_cast<const uint4 *>(q + 6));
+    return n;
+}
+
+// min that returns NaN when either operand is NaN
+__device__ __forceinline__ float fmin_nan(float a, float b) {
+    float d;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+
+// Distances to one axis's near and far planes of the four children, each the
+// float the binary slab() computes for that child.
+__device__ __forceinline__ void quad_axis(const float4 &mn, const float4 &mx, bool neg, float o,
+                                          float inv, float (&t0)[4], float (&t1)[4]) {
+    t0[0] = ((neg ? mx.x : mn.x) - o) * inv;
+    t0[1] = ((neg ? mx.y : mn.y) - o) * inv;
+    t0[2] = ((neg ? mx.z : mn.z) - o) * inv;
+    t0[3] = ((neg ? mx.w : mn.w) - o) * inv;
+    t1[0] = ((neg ? mn.x : mx.x) - o) * inv;
+    t1[1] = ((neg ? mn.y : mx.y) - o) * inv;
+    t1[2] = ((neg ? mn.z : mx.z) - o) * inv;
+    t1[3] = ((neg ? mn.w : mx.w) - o) * inv;
+}
+
+__device__ __forceinline__ void quad_axis(const float4 &mn, const float4 &mx, bool neg, float2 o,
+                                          float2 inv, float (&t0)[4], float (&t1)[4]) {
+    const float2 a = __fmul2_rn(fsub2(make_float2(neg ? mx.x : mn.x, neg ? mx.y : mn.y), o), inv);
+    const float2 b = __fmul2_rn(fsub2(make_float2(neg ? mx.z : mn.z, neg ? mx.w : mn.w), o), inv);
+    const float2 c = __fmul2_rn(fsub2(make_float2(neg ? mn.x : mx.x, neg ? mn.y : mx.y), o), inv);
+    const float2 d = __fmul2_rn(fsub2(make_float2(neg ? mn.z : mx.z, neg ? mn.w : mx.w), o), inv);
+    t0[0] = a.x;
+    t0[1] = a.y;
+    t0[2] = b.x;
+    t0[3] = b.y;
+    t1[0] = c.x;
+    t1[1] = c.y;
+    t1[2] = d.x;
+    t1[3] = d.y;
+}
+
+// Entry distances of the four children (slab() of each), and of the two
+// binary nodes between them and this one (e01 over children 0 and 1, e23 over
+// 2 and 3), which only decide the order the sides are walked in.
+//
+// Why a walk over these nodes equals the binary walk: a node's box is the
+// union of its children's, and rounding is monotone, so a child's entry
+// distance is never below its parent's and a child is entered only when its
+// parent is; whether a leaf's triangles are tested therefore depends on the
+// leaf's own distance and on the order of the leaves alone. The order comes
+// from comparing siblings' entry distances at each binary node: between the
+// grandchildren of a side those computed here, between the two sides e01 and
+// e23, the near distances of the union boxes -- per axis the smaller of the
+// children's near distances, or NaN (an axis without a bound) when one of
+// them is, since then the union's near plane is either at the ray's origin
+// too or behind it. Where a side's own box is missed its entry distance is
+// not the binary walk's +inf, but then none of its children is entered.
+__device__ __forceinline__ void quad_fold(const float (&x0)[4], const float (&x1)[4],
+                                          const float (&y0)[4], const float (&y1)[4],
+                                          const float (&z0)[4], const float (&z1)[4],
+                                          float (&t)[4], float &e01, float &e23) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float tmin = fmax3(fmaxf(0.f, x0[k]), y0[k], z0[k]);
+        // NaN when no axis bounds the exit: not tmin > tmax, as tmin <= +inf
+        const float tmax = fmin3(x1[k], y1[k], z1[k]);
+        t[k] = tmin > tmax ? kInf : tmin;
+    }
+    e01 = fmax3(fmaxf(0.f, fmin_nan(x0[0], x0[1])), fmin_nan(y0[0], y0[1]),
+                fmin_nan(z0[0], z0[1]));
+    e23 = fmax3(fmaxf(0.f, fmin_nan(x0[2], x0[3])), fmin_nan(y0[2], y0[3]),
+                fmin_nan(z0[2], z0[3]));
+}
+
+__device__ __forceinline__ void quad_test(const QuadV &n, const RayPre &p, float (&t)[4],
+                                          float &e01, float &e23) {
+    float x0[4], x1[4], y0[4], y1[4], z0[4], z1[4];
+    quad_axis(n.mn[0], n.mx[0], p.nx, p.ox, p.ix, x0, x1);
+    quad_axis(n.mn[1], n.mx[1], p.ny, p.oy, p.iy, y0, y1);
+    quad_axis(n.mn[2], n.mx[2], p.nz, p.oz, p.iz, z0, z1);
+    quad_fold(x0, x1, y0, y1, z0, z1, t, e01, e23);
+}
+
+__device__ __forceinline__ void quad_test(const QuadV &n, const RayPair &p, float (&t)[4],
+                                          float &e01, float &e23) {
+    float x0[4], x1[4], y0[4], y1[4], z0[4], z1[4];
+    quad_axis(n.mn[0], n.mx[0], p.nx, p.o2x, p.i2x, x0, x1);
+    quad_axis(n.mn[1], n.mx[1], p.ny, p.o2y, p.i2y, y0, y1);
+    quad_axis(n.mn[2], n.mx[2], p.nz, p.o2z, p.i2z, z0, z1);
+    quad_fold(x0, x1, y0, y1, z0, z1, t, e01, e23);
+}
+
+// The children of a four-wide node in walk order, with their entry distances
+// (t0 <= t1 and t2 <= t3).
+struct QuadOrder {
+    float t0, t1, t2, t3;
+    uint32_t r0, r1, r2, r3;
+    // whether some child is entered (its box nearer than best), and the first
+    __device__ __forceinline__ bool any(float best) const { return t0 < best || t2 < best; }
+    __device__ __forceinline__ uint32_t next(float best) const { return t0 < best ? r0 : r2; }
+    __device__ __forceinline__ float next_t(float best) const { return t0 < best ? t0 : t2; }
+    // push(ref, t) for the entered children but the first, last in walk order first
+    template <class Push> __device__ __forceinline__ void rest(float best, Push &&push) const {
+        if (t3 < best)
+            push(r3, t3);
+        if (t0 < best && t2 < best)
+            push(r2, t2);
+        if (t1 < best)
+            push(r1, t1);
+    }
+};
+
+template <class P>
+__device__ __forceinline__ QuadOrder quad_order(const QuadV &n, const P &p) {
+    float t[4], e01, e23;
+    quad_test(n, p, t, e01, e23);
+    const bool s0 = !(t[0] <= t[1]), s1 = !(t[2] <= t[3]), sw = !(e01 <= e23);
+    const float an = s0 ? t[1] : t[0], af = s0 ? t[0] : t[1];
+    const float bn = s1 ? t[3] : t[2], bf = s1 ? t[2] : t[3];
+    const uint32_t ar = s0 ? n.ref.y : n.ref.x, aq = s0 ? n.ref.x : n.ref.y;
+    const uint32_t br = s1 ? n.ref.w : n.ref.z, bq = s1 ? n.ref.z : n.ref.w;
+    QuadOrder q;
+    q.t0 = sw ? bn : an;
+    q.t1 = sw ? bf : af;
+    q.t2 = sw ? an : bn;
+    q.t3 = sw ? af : bf;
+    q.r0 = sw ? br : ar;
+    q.r1 = sw ? bq : aq;
+    q.r2 = sw ? ar : br;
+    q.r3 = sw ? aq : bq;
+    return q;
+}
+
+// True for a ray that an inverted box (+inf..-inf, an empty slot) does not
+// stop: on every axis its origin is NaN or its direction NaN or infinite. Such
+// a ray hits no triangle (its Möller-Trumbore t is NaN or 0), so mesh walks
+// are skipped for it, and empty slots are never entered.
+template <class P> __device__ __forceinline__ bool no_slab(const P &p) {
+    return slab(kInf, -kInf, kInf, -kInf, kInf, -kInf, p) < kInf;
+}
+
 struct TriV {
     float4 p, q, r;
 };
@@ -255,6 +422,10 @@ __device__ __forceinline__ TriV load_tri(const Tri *tris, const float *e2z, uint
 
 __device__ __forceinline__ NodeV load_node(const DevScene &S, uint32_t idx) {
     return load_node(S.nodes, idx, bounds_of(S));
+}
+
+__device__ __forceinline__ QuadV load_quad(const DevScene &S, uint32_t idx) {
+    return load_quad(S.qnodes, idx, bounds_of(S));
 }
 
 __device__ __forceinline__ TriV load_tri(const DevScene &S, uint32_t idx) {
@@ -308,47 +479,107 @@ __device__ __forceinline__ bool tri_occludes(const TriV &T, const RayD &r, float
            (t > 1e-3f && t < tmax);
 }
 
-// Per-thread stack with a bounded shared-memory part: entries [0, cap) in the
-// thread's shared-memory column (entry k at sm[k * blockDim.x]), deeper
-// entries in a global buffer laid out [entry - cap][grid thread], so a warp's
-// spills are coalesced. A walk pushes at most once per tree level, so tree
-// depth + 1 entries in the two parts together always suffice; the global part
-// is only reached deep in unbalanced subtrees and stays in L1/L2. Its address
-// is formed only on that cold path, so the stack costs two registers. `cap`
-// is a launch parameter: fewer shared entries leave more of the SM's L1 for
-// node and triangle fetches and let more blocks be resident.
+// Shared-memory accesses by 32-bit shared address (a pointer that may also
+// name global memory compiles to generic accesses, which cost the LSU more).
+__device__ __forceinline__ void sts(uint32_t a, uint2 v) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(v.x), "r"(v.y));
+}
+__device__ __forceinline__ void sts(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v));
+}
+__device__ __forceinline__ void lds(uint32_t a, uint2 &v) {
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+}
+__device__ __forceinline__ void lds(uint32_t a, uint32_t &v) {
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+}
+
+// Per-thread stack with a bounded shared-memory part. A position is the byte
+// address `top` of the next free entry of the thread's shared-memory column
+// (step bytes apart, [entry][thread], so a warp's pushes hit distinct banks);
+// positions at `limit` and beyond stand for entries of a global buffer laid
+// out [entry - cap][grid thread], so a warp's spills are coalesced. The bound
+// on a walk's entries is found when its tree is packed; the global part is
+// only reached deep in unbalanced subtrees and stays in L1/L2, and the code
+// for it sits behind one comparison per step. Fewer shared entries leave more
+// of the SM's L1 for node and triangle fetches and let more blocks be
+// resident.
 template <class E> struct StackCol {
-    E *sm;
+    uint32_t base, step, limit;
     E *gl;
-    int cap;
     int total = 1 << 30;     // entries in both parts (tested by the checked build)
     uint32_t *check = nullptr;
-    __device__ __forceinline__ E *spill_at(int k) const {
-        return gl + (size_t) (k - cap) * (gridDim.x * blockDim.x) + blockIdx.x * blockDim.x +
-               threadIdx.x;
+    __device__ __forceinline__ StackCol(E *sm, E *global, int cap, int total_, uint32_t *check_)
+        : base((uint32_t) __cvta_generic_to_shared(sm) + threadIdx.x * (uint32_t) sizeof(E)),
+          step(blockDim.x * (uint32_t) sizeof(E)), gl(global), total(total_), check(check_) {
+        limit = base + (uint32_t) cap * step;
     }
-    __device__ __forceinline__ void put(int k, E v) const {
+    __device__ __forceinline__ E *spill_at(uint32_t top) const {
+        return gl + (size_t) ((top - limit) / step) * (gridDim.x * blockDim.x) +
+               blockIdx.x * blockDim.x + threadIdx.x;
+    }
+    __device__ __forceinline__ bool ok(uint32_t top) const {
 #ifdef PRR_CHECKED
-        if (k >= total || k < 0) {
-            check_fail(check, kCheckStack, (uint32_t) k);
+        if (top < base || (top - base) / step >= (uint32_t) total) {
+            check_fail(check, kCheckStack, (top - base) / step);
+            return false;
+        }
+#endif
+        (void) top;
+        return true;
+    }
+    // three more entries fit in the shared part
+    __device__ __forceinline__ bool room3(uint32_t top) const { return top + 2 * step < limit; }
+    // an entry known to lie in the shared part
+    __device__ __forceinline__ void put_sm(uint32_t &top, E v) const {
+        if (!ok(top))
             return;
-        }
-#endif
-        if (k < cap)
-            sm[k * blockDim.x] = v;
+        sts(top, v);
+        top += step;
+    }
+    __device__ __forceinline__ void put(uint32_t &top, E v) const {
+        if (!ok(top))
+            return;
+        if (top < limit)
+            sts(top, v);
         else
-            *spill_at(k) = v;
+            *spill_at(top) = v;
+        top += step;
     }
-    __device__ __forceinline__ E get(int k) const {
-#ifdef PRR_CHECKED
-        if (k >= total || k < 0) {
-            check_fail(check, kCheckStack, (uint32_t) k);
-            return E{};
-        }
-#endif
-        return k < cap ? sm[k * blockDim.x] : *spill_at(k);
+    __device__ __forceinline__ E pop(uint32_t &top) const {
+        top -= step;
+        E v{};
+        if (!ok(top))
+            return v;
+        if (top < limit)
+            lds(top, v);
+        else
+            v = *spill_at(top);
+        return v;
     }
+    __device__ __forceinline__ bool empty(uint32_t top) const { return top == base; }
 };
+
+// Push a node's entered children but the first (closest hit: with their entry
+// distances; any hit: references alone).
+__device__ __forceinline__ void push_rest(const StackCol<uint2> &st, uint32_t &top,
+                                          const QuadOrder &q, float best) {
+    if (st.room3(top))
+        q.rest(best, [&](uint32_t c, float t) {
+            st.put_sm(top, make_uint2(c, __float_as_uint(t)));
+        });
+    else
+        q.rest(best, [&](uint32_t c, float t) {
+            st.put(top, make_uint2(c, __float_as_uint(t)));
+        });
+}
+__device__ __forceinline__ void push_rest(const StackCol<uint32_t> &st, uint32_t &top,
+                                          const QuadOrder &q, float tmax) {
+    if (st.room3(top))
+        q.rest(tmax, [&](uint32_t c, float) { st.put_sm(top, c); });
+    else
+        q.rest(tmax, [&](uint32_t c, float) { st.put(top, c); });
+}
 
 // Per-thread stack column in shared memory.
 struct SmemStack {
@@ -373,9 +604,61 @@ struct SmemStack {
     }
 };
 
-// BVHAccel::Intersect, triangle fast path (BVH.cpp:311-415) on one mesh BVH.
-// best_t enters as +inf (every mesh-level search starts fresh, BVH.cpp:331).
-// Returns the winning triangle's global leaf-order index, or -1.
+// BVHAccel::Intersect, triangle fast path (BVH.cpp:311-415) on one mesh's
+// four-wide nodes. best_t enters as +inf (every mesh-level search starts
+// fresh, BVH.cpp:331). Returns the winning triangle's global leaf-order index,
+// or -1.
+__device__ __forceinline__ int blas_closest_quad(const QNode *__restrict__ nodes,
+                                            const Tri *__restrict__ tris,
+                                            const float *__restrict__ e2z, uint32_t root,
+                                            const RayD &r, const RayPre &p, SmemStack &st,
+                                            float &best_t, float &best_u, float &best_v,
+                                            const TraceBounds &B) {
+    if (!(root & kLeafBit) && no_slab(p))
+        return -1;
+    const int sp0 = st.sp;
+    uint32_t ref = root;
+    int hit = -1;
+    for (;;) {
+        if (!(ref & kLeafBit)) {
+            const QuadOrder q = quad_order(load_quad(nodes, ref, B), p);
+            q.rest(best_t, [&](uint32_t c, float t) { st.push(c, t); });
+            if (q.any(best_t)) {
+                ref = q.next(best_t);
+                continue;
+            }
+        } else {
+            const uint32_t first = leaf_first(ref);
+            const uint32_t cnt = leaf_count(ref);
+            for (uint32_t i = 0; i < cnt; i++) {
+                const TriV T = load_tri(tris, e2z, first + i, B);
+                float t, u, v;
+                if (tri_hit(T, r, t, u, v) && t < best_t) {
+                    best_t = t;
+                    best_u = u;
+                    best_v = v;
+                    hit = (int) (first + i);
+                }
+            }
+        }
+        // pop the next entry whose box is still nearer than the closest hit
+        for (;;) {
+            if (st.sp == sp0)
+                return hit;
+            const uint2 e = st.pop();
+            if (__uint_as_float(e.y) < best_t) {
+                ref = e.x;
+                break;
+            }
+        }
+    }
+}
+
+// The same search on the binary nodes, for the kernels that run a whole path
+// per thread (plain renderer, photons, caustic samples): the four-wide step's
+// registers cost those more than its shorter walk saves (museum-like scene of
+// 122,880 triangles at 480x270, 16 spp: 12.4 ms, 14.4 four-wide; Cornell box
+// 2.2 against 2.7).
 __device__ __forceinline__ int blas_closest(const WNode *__restrict__ nodes,
                                             const Tri *__restrict__ tris,
                                             const float *__restrict__ e2z, uint32_t root,
@@ -432,10 +715,6 @@ __device__ __forceinline__ int blas_closest(const WNode *__restrict__ nodes,
     }
 }
 
-// BVHAccel::IntersectP (BVH.cpp:421-473) on one mesh BVH whose root box is
-// root_box: true when a triangle occludes within tmax. Child boxes are tested
-// where the reference tests them (far child at push, near child at the top of
-// the next iteration), so exactly the same subtrees are entered.
 __device__ __forceinline__ bool blas_occluded(const WNode *__restrict__ nodes,
                                               const Tri *__restrict__ tris,
                                               const float *__restrict__ e2z, uint32_t root,

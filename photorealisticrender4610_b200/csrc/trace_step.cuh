@@ -2,7 +2,7 @@
 // persistent kernels whose lanes take new rays as soon as theirs finish.
 // Each call to step() does one unit of work -- one interior node, one
 // triangle, one sphere, or entering a mesh -- in exactly the order of the
-// recursive walks in trace.cuh (scene_closest / scene_occluded, which restate
+// walks in trace.cuh (scene_closest / scene_occluded, which restate
 // BVH.cpp:311-473 over MeshTriangle and Sphere leaves), so results are
 // identical; only the scheduling of rays onto lanes changes.
 #pragma once
@@ -11,37 +11,40 @@
 namespace prr {
 
 // Closest hit: Scene::intersect -> scene BVH, general path; each mesh leaf is
-// searched from +inf on its own (BVH.cpp:359-369).
-struct ClosestWalk {
+// searched from +inf on its own (BVH.cpp:359-369). BINARY walks the binary
+// mesh nodes instead of the four-wide ones, a step being one of the
+// reference's interior visits: the counting variants of the wavefront stages
+// (prr_render_counts report the reference's traversal work).
+template <bool BINARY = false> struct ClosestWalk {
     RayD r;
     RayPre p;
     float closest;
     int hit_obj, hit_tri;
     uint32_t tref;
-    int tsp;
+    uint32_t tsp;
     bool in_mesh;
     int cur_obj;
     uint32_t bref, tri, ntri;
     float bbest;
     int bhit;
-    int bsp;
+    uint32_t bsp;
 
-    __device__ __forceinline__ void start(const DevScene &S, const RayD &ray) {
+    __device__ __forceinline__ void start(const DevScene &S, const RayD &ray,
+                                          const StackCol<uint2> &tc) {
         r = ray;
         p = precompute(ray);
         closest = kInf;
         hit_obj = hit_tri = -1;
         tref = S.tlas_root;
-        tsp = 0;
+        tsp = tc.base;
         in_mesh = false;
         ntri = 0;
     }
 
     // pops the scene-level stack; true when the walk is over
     __device__ __forceinline__ bool scene_pop(const StackCol<uint2> &tc) {
-        while (tsp > 0) {
-            --tsp;
-            const uint2 e = tc.get(tsp);
+        while (!tc.empty(tsp)) {
+            const uint2 e = tc.pop(tsp);
             if (__uint_as_float(e.y) < closest) {
                 tref = e.x;
                 return false;
@@ -75,31 +78,34 @@ struct ClosestWalk {
                 ntri--;
                 pop = ntri == 0;
             } else {
-                const NodeV n = load_node(S, bref);
-                const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-                const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-                if (tl <= tr) {
-                    if (tl < bbest) {
-                        if (tr < bbest)
-                            bc.put(bsp++, make_uint2(n.link.y, __float_as_uint(tr)));
-                        set_mesh_ref(n.link.x);
-                        return false;
-                    }
+                uint32_t next;
+                bool down;
+                if constexpr (BINARY) {
+                    const NodeV n = load_node(S, bref);
+                    const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
+                    const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
+                    const bool left = tl <= tr;
+                    down = (left ? tl : tr) < bbest;
+                    next = left ? n.link.x : n.link.y;
+                    if ((left ? tr : tl) < bbest)
+                        bc.put(bsp, make_uint2(left ? n.link.y : n.link.x,
+                                               __float_as_uint(left ? tr : tl)));
                 } else {
-                    if (tr < bbest) {
-                        if (tl < bbest)
-                            bc.put(bsp++, make_uint2(n.link.x, __float_as_uint(tl)));
-                        set_mesh_ref(n.link.y);
-                        return false;
-                    }
+                    const QuadOrder q = quad_order(load_quad(S, bref), p);
+                    push_rest(bc, bsp, q, bbest);
+                    down = q.any(bbest);
+                    next = q.next(bbest);
+                }
+                if (down) {
+                    set_mesh_ref(next);
+                    return false;
                 }
                 pop = true;
             }
             if (!pop)
                 return false;
-            while (bsp > 0) {
-                --bsp;
-                const uint2 e = bc.get(bsp);
+            while (!bc.empty(bsp)) {
+                const uint2 e = bc.pop(bsp);
                 if (__uint_as_float(e.y) < bbest) {
                     set_mesh_ref(e.x);
                     return false;
@@ -121,14 +127,14 @@ struct ClosestWalk {
             if (tl <= tr) {
                 if (tl < closest) {
                     if (tr < closest)
-                        tc.put(tsp++, make_uint2(n.link.y, __float_as_uint(tr)));
+                        tc.put(tsp, make_uint2(n.link.y, __float_as_uint(tr)));
                     tref = n.link.x;
                     return false;
                 }
             } else {
                 if (tr < closest) {
                     if (tl < closest)
-                        tc.put(tsp++, make_uint2(n.link.x, __float_as_uint(tl)));
+                        tc.put(tsp, make_uint2(n.link.x, __float_as_uint(tl)));
                     tref = n.link.y;
                     return false;
                 }
@@ -138,12 +144,14 @@ struct ClosestWalk {
         const int k = (int) (tref & ~kLeafBit);
         const DevObject &o = S.objects[k];
         if (o.kind == kObjMesh) {
+            if (!(o.qroot & kLeafBit) && no_slab(p))
+                return scene_pop(tc);
             in_mesh = true;
             cur_obj = k;
             bbest = kInf;
             bhit = -1;
-            bsp = 0;
-            set_mesh_ref(o.root);
+            bsp = bc.base;
+            set_mesh_ref(BINARY ? o.root : o.qroot);
             return false;
         }
         float t;
@@ -158,24 +166,26 @@ struct ClosestWalk {
 
 // Any hit: Scene::intersectP -> scene BVH IntersectP over MeshTriangle /
 // Sphere intersectT (BVH.cpp:421-473, Triangle.hpp:141-147, Object.hpp:24-29).
-struct AnyWalk {
+// BINARY as above: the reference's interior visits, in its order.
+template <bool BINARY = false> struct AnyWalk {
     RayD r;
     RayPair p;
     float tmax;
     uint32_t tref;
-    int tsp;
+    uint32_t tsp;
     bool in_mesh;
     uint32_t bref, tri, ntri;
-    int bsp;
+    uint32_t bsp;
     bool occluded;
 
     // false when the scene's root box already misses
-    __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray, float t_max) {
+    __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray, float t_max,
+                                          const StackCol<uint32_t> &tc) {
         r = ray;
         p = precompute_pair(ray);
         tmax = t_max;
         tref = S.tlas_root;
-        tsp = 0;
+        tsp = tc.base;
         in_mesh = false;
         ntri = 0;
         occluded = false;
@@ -193,10 +203,9 @@ struct AnyWalk {
     }
 
     __device__ __forceinline__ bool scene_pop(const StackCol<uint32_t> &tc) {
-        if (tsp == 0)
+        if (tc.empty(tsp))
             return true;
-        --tsp;
-        tref = tc.get(tsp);
+        tref = tc.pop(tsp);
         return false;
     }
 
@@ -221,25 +230,31 @@ struct AnyWalk {
                 if (ntri > 0)
                     return false;
             } else {
-                const NodeV n = load_node(S, bref);
-                const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-                const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-                const uint32_t axis = n.link.z;
-                const bool neg = axis == 0 ? p.nx : (axis == 1 ? p.ny : p.nz);
-                const uint32_t near_ref = neg ? n.link.y : n.link.x;
-                const uint32_t far_ref = neg ? n.link.x : n.link.y;
-                const float tnear = neg ? tr : tl;
-                const float tfar = neg ? tl : tr;
-                if (tfar < tmax)
-                    bc.put(bsp++, far_ref);
-                if (tnear < tmax) {
-                    set_mesh_ref(near_ref);
+                uint32_t next;
+                bool down;
+                if constexpr (BINARY) {
+                    const NodeV n = load_node(S, bref);
+                    const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
+                    const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
+                    const uint32_t axis = n.link.z;
+                    const bool neg = axis == 0 ? p.nx : (axis == 1 ? p.ny : p.nz);
+                    down = (neg ? tr : tl) < tmax; // octant 0 -> near = left
+                    next = neg ? n.link.y : n.link.x;
+                    if ((neg ? tl : tr) < tmax)
+                        bc.put(bsp, neg ? n.link.x : n.link.y);
+                } else {
+                    const QuadOrder q = quad_order(load_quad(S, bref), p);
+                    push_rest(bc, bsp, q, tmax);
+                    down = q.any(tmax);
+                    next = q.next(tmax);
+                }
+                if (down) {
+                    set_mesh_ref(next);
                     return false;
                 }
             }
-            if (bsp > 0) {
-                --bsp;
-                set_mesh_ref(bc.get(bsp));
+            if (!bc.empty(bsp)) {
+                set_mesh_ref(bc.pop(bsp));
                 return false;
             }
             in_mesh = false;
@@ -256,7 +271,7 @@ struct AnyWalk {
             const float tnear = neg ? tr : tl;
             const float tfar = neg ? tl : tr;
             if (tfar < tmax)
-                tc.put(tsp++, far_ref);
+                tc.put(tsp, far_ref);
             if (tnear < tmax) {
                 tref = near_ref;
                 return false;
@@ -266,10 +281,10 @@ struct AnyWalk {
         const DevObject &o = S.objects[tref & ~kLeafBit];
         if (o.kind == kObjMesh) {
             // the mesh's own IntersectP first tests its root box
-            if (slab6(o.root_box, p) < tmax) {
+            if (slab6(o.root_box, p) < tmax && ((o.qroot & kLeafBit) || !no_slab(p))) {
                 in_mesh = true;
-                bsp = 0;
-                set_mesh_ref(o.root);
+                bsp = bc.base;
+                set_mesh_ref(BINARY ? o.root : o.qroot);
                 return false;
             }
             return scene_pop(tc);
