@@ -116,8 +116,9 @@ typedef struct prr_render_settings {
 
 /* Wavefront launch shape (chosen by prr_autotune; zero fields = defaults). */
 typedef struct prr_wavefront_config {
-    int64_t paths_per_pass; /* paths in flight per pass (0: about 8M; at most 2^30; about
-                               320 bytes of device memory each) */
+    int64_t paths_per_pass; /* paths in flight per pass (0: up to 32M, fewer where device
+                               memory is short; at most 2^30; about 320 bytes of device
+                               memory each) */
     int block_size;         /* threads per block of the traversal stages (0: 128) */
     int use_graphs;         /* 1: replay each pass from one captured CUDA graph */
     int stack_smem;         /* mesh-BVH stack entries per thread kept in shared memory;
@@ -125,7 +126,7 @@ typedef struct prr_wavefront_config {
     int ordered;            /* 1: rebuild the stage queues in path order (stable partition,
                                next rays grouped by direction octant); 0: append order */
     int refill;             /* traversal stages: a warp takes new rays from its queue once
-                               this many of its lanes are idle (0: 8; at most 32) */
+                               this many of its lanes are idle (0: 12; at most 32) */
 } prr_wavefront_config;
 
 typedef struct prr_scene_stats {

@@ -306,6 +306,15 @@ __global__ void k_wf_begin(Wf w, int it) {
     }
 }
 
+// The lanes of a warp that take rays of a queue of n: all 32, or as many as
+// spread a short queue (a small frame, the last bounces) over every warp of
+// the grid. A short queue takes as long as its longest ray, and a warp steps
+// faster the fewer rays it holds.
+__device__ __forceinline__ int lanes_used(int n) {
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    return max(1, min(32, n / warps + 1));
+}
+
 // ---- extend: closest hit of the queued rays, then sort by material class.
 // Persistent: a lane whose ray is finished takes the next queued ray once
 // `refill` lanes of its warp are idle (one atomic per refill).
@@ -343,10 +352,14 @@ __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int i
     bool more = n > 0;
     if (!more)
         return;
+    // a lane without a ray has p = -1, or -2 when it takes none
+    refill = min(refill, lanes_used(n));
+    if (lane >= lanes_used(n))
+        p = -2;
     for (;;) {
-        const bool idle = p < 0;
+        const bool idle = p == -1;
         const unsigned im = __ballot_sync(full, idle);
-        if (!more && im == full) {
+        if (!more && __all_sync(full, p < 0)) {
             if constexpr (STATS) {
                 const unsigned a[3] = {cnt_[0], cnt_[1], cnt_[2]};
                 const unsigned b[3] = {cnt_[3], cnt_[4], cnt_[5]};
@@ -772,10 +785,13 @@ __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int r
     bool more = n > 0;
     unsigned rays = 0;
     unsigned cnt_[3] = {0, 0, 0}; // nodes, tris, objects
+    refill = min(refill, lanes_used(n)); // a lane that takes no rays: job = -2
+    if (lane >= lanes_used(n))
+        job = -2;
     for (;;) {
-        const bool idle = job < 0;
+        const bool idle = job == -1;
         const unsigned im = __ballot_sync(full, idle);
-        if (!more && im == full)
+        if (!more && __all_sync(full, job < 0))
             break;
         if (more && __popc(im) >= refill) {
             const int cnt = __popc(im);
@@ -1309,7 +1325,7 @@ int wf_shape(Wf &w, DevBuf &spill, int block_req, int stack_req, int refill_req,
                          carve_pref);
     cudaFuncSetAttribute((const void *) L.sh, cudaFuncAttributePreferredSharedMemoryCarveout,
                          carve_pref);
-    L.refill = refill_req > 0 ? std::min(refill_req, 32) : 8;
+    L.refill = refill_req > 0 ? std::min(refill_req, 32) : 12;
     int occ_ext = 1, occ_sh = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ext, (const void *) L.ext, L.block,
                                                   L.smem_ext);
@@ -1417,16 +1433,27 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.sample_offset = rs.sample_offset;
     w.tlas_cap = S.tlas_depth + 1;
     w.blas_cap = (s.wf_stats ? S.blas_depth : S.blas_stack) + 1;
-    // paths per pass: whole samples of the window, about 8M paths in flight
-    const int64_t target = s.wf_paths > 0 ? s.wf_paths : (int64_t) 1 << 23;
-    int spp_pass = (int) std::max<int64_t>(1, target / std::max(1, w.npix));
-    spp_pass = std::min(spp_pass, rs.max_spp);
-    while (rs.max_spp % spp_pass)
-        spp_pass--;
-    w.spp_pass = spp_pass;
-    w.P = spp_pass * w.npix;
-    if (int rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix))
-        return rc;
+    // Paths per pass: whole samples of the window, by default at most 32M in
+    // flight (10 GB of path state): every bounce of a pass ends in a tail of
+    // long rays, so fewer and larger passes pay it less often (museum-like
+    // scene at 480x270, adaptive up to 256 spp: 56.7 ms at 8M, 49.4 at 32M).
+    // Where that much memory is not free, half as much, down to 8M.
+    const int64_t kDefaultPaths = (int64_t) 1 << 25, kLeastPaths = (int64_t) 1 << 23;
+    int spp_pass = 1;
+    for (int64_t target = s.wf_paths > 0 ? s.wf_paths : kDefaultPaths;; target >>= 1) {
+        spp_pass = (int) std::max<int64_t>(1, target / std::max(1, w.npix));
+        spp_pass = std::min(spp_pass, rs.max_spp);
+        while (rs.max_spp % spp_pass)
+            spp_pass--;
+        w.spp_pass = spp_pass;
+        w.P = spp_pass * w.npix;
+        const int rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix);
+        if (rc == PRR_OK)
+            break;
+        if (rc != PRR_ERR_OUT_OF_MEMORY || s.wf_paths > 0 || target <= kLeastPaths)
+            return rc;
+        cudaGetLastError(); // the failed allocation
+    }
     w.ordered = s.wf_ordered ? 1 : 0;
     w.adaptive = rs.min_spp < rs.max_spp ? 1 : 0;
     w.min_spp = rs.min_spp;
@@ -1601,7 +1628,7 @@ int wavefront_step_multi(WfMultiState &ms, const WfStepReq *reqs, int n,
         if (int rc = wf_layout(ms.state, w, (size_t) maxP, 1))
             return rc;
         WfShape L;
-        if (int rc = wf_shape<true>(w, ms.spill, 128, 8, 8, L))
+        if (int rc = wf_shape<true>(w, ms.spill, 128, 8, 0, L))
             return rc;
         const WfParts parts = wf_parts(w);
         PRR_CUDA_TRY(cudaMemsetAsync(w.tag, 0xFF, (size_t) L.ntiles * kPartTile, st));
