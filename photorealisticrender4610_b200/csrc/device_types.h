@@ -49,7 +49,7 @@ struct alignas(64) WNode {
 };
 static_assert(sizeof(WNode) == 64, "WNode must be 64 bytes");
 
-// Four-wide node of a mesh BVH: two levels of the binary tree in one 128-byte
+// Four-wide node of a mesh BVH or of the scene BVH: two levels of the binary tree in one 128-byte
 // line, so a walk makes about half as many dependent fetches. Children 0 and 1
 // are those of the binary node's left child, 2 and 3 those of its right child;
 // a side that is a leaf (or whose box is not exactly the union of its
@@ -61,7 +61,7 @@ static_assert(sizeof(WNode) == 64, "WNode must be 64 bytes");
 // walk over the binary tree (trace.cuh, quad_test).
 struct alignas(128) QNode {
     float plane[3][2][4]; // [axis][min, max][child]
-    uint32_t ref[4];      // interior: QNode index; leaf: mesh_leaf_ref
+    uint32_t ref[4];      // interior: QNode index; leaf: mesh_leaf_ref / kLeafBit | object
     uint32_t pad[4];
 };
 static_assert(sizeof(QNode) == 128, "QNode must be 128 bytes");
@@ -152,7 +152,7 @@ struct DevEnv {
 
 struct DevScene {
     const WNode *nodes;
-    const QNode *qnodes;       // four-wide mesh nodes
+    const QNode *qnodes;       // four-wide nodes, of the meshes and the scene
     const Tri *tris;
     const float *tri_e2z;      // e2.z of each triangle (completes Tri)
     const TriMeta *tri_meta;   // input id and area of each triangle
@@ -168,9 +168,10 @@ struct DevScene {
     int32_t has_emissive_kind; // some material is of the emissive kind (hit-emission MIS
                                // then needs the previous hit point)
     float total_emit_area;
-    uint32_t tlas_root;
+    uint32_t tlas_root, tlas_qroot; // into nodes, qnodes
     float tlas_box[6];
     int32_t tlas_depth;
+    int32_t tlas_stack;   // entries the scene level of a walk's stack may need
     int32_t blas_depth;   // max over meshes
     int32_t blas_stack;   // entries a mesh walk's stack may need, max over meshes
     float background[3];

@@ -43,12 +43,11 @@ __device__ double tri_t64(const float *__restrict__ v, const RayD &r) {
 // What every query kernel needs besides its rays and outputs.
 struct TraceCfg {
     unsigned *counter;           // next ray to hand out (nullptr: fixed shares)
-    void *spill;                 // global part of the mesh stacks
+    void *spill;                 // global part of the stacks
     uint32_t share;              // rays of a warp's share: n over the grid's warps
     int lanes;                   // lanes of a warp that take rays: share, at most 32
     int refill;                  // idle lanes that trigger a refill (at most lanes)
-    int stack_sm, stack_cap;     // mesh-stack entries: in shared memory, in all
-    int tlas_cap;                // scene-stack entries (all in shared memory)
+    int stack_sm, stack_cap;     // stack entries: in shared memory, in all
 };
 
 struct MeshArgs {
@@ -453,44 +452,38 @@ struct SceneArgs {
 
 template <class E> __device__ __forceinline__ StackCol<E> scene_col(const DevScene &S,
                                                                     const TraceCfg &c, E *smem) {
-    return StackCol<E>(smem, nullptr, c.tlas_cap, c.tlas_cap, S.check);
-}
-template <class E> __device__ __forceinline__ StackCol<E> mesh_col(const DevScene &S,
-                                                                   const TraceCfg &c, E *smem) {
-    return StackCol<E>(smem + (size_t) c.tlas_cap * blockDim.x, (E *) c.spill, c.stack_sm,
-                       c.stack_cap, S.check);
+    return StackCol<E>(smem, (E *) c.spill, c.stack_sm, c.stack_cap, S.check);
 }
 
 // 2,000,003 rays on 122,880 triangles with geometry, half of them incoherent:
-// 0.58 ms against 0.74 for one ray per thread; any hit 0.33 against 0.81.
+// 0.50 ms against 0.74 for one ray per thread; any hit 0.35 against 0.81.
 struct SceneClosest {
     const DevScene &S;
     const SceneArgs &a;
     int32_t *out_obj, *out_prim;
     float *out_t;
     bool raw; // out_prim takes the leaf-order triangle index (k_scene_finish resolves it)
-    const StackCol<uint2> tc, bc;
+    const StackCol<uint2> col;
     uint32_t idx = 0;
-    ClosestWalk<false> w;
+    ClosestWalk w;
 
     __device__ __forceinline__ SceneClosest(const DevScene &scene, const SceneArgs &args,
                                             int32_t *obj, int32_t *prim, float *t, bool leaf_order,
                                             uint2 *smem)
         : S(scene), a(args), out_obj(obj), out_prim(prim), out_t(t), raw(leaf_order),
-          tc(scene_col(scene, args.c, smem)), bc(mesh_col(scene, args.c, smem)) {}
+          col(scene_col(scene, args.c, smem)) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
-        w.start(S, load_ray(a.O, a.D, i), tc);
-        if (S.n_objects > 0)
+        if (w.start(S, load_ray(a.O, a.D, i), col))
             return true;
         finish();
         return false;
     }
-    __device__ __forceinline__ bool step() { return w.step(S, tc, bc); }
+    __device__ __forceinline__ bool step() { return w.step(S, col); }
     __device__ __forceinline__ void finish() {
         out_obj[idx] = w.hit_obj;
-        out_t[idx] = w.closest;
+        out_t[idx] = w.best;
         int prim = w.hit_tri;
         if (!raw && w.hit_obj >= 0)
             prim = prim >= 0 ? __ldg(&S.tri_meta[prim].id) : 0;
@@ -575,23 +568,22 @@ struct SceneAny {
     const SceneArgs &a;
     const float *tmaxs;
     uint8_t *out;
-    const StackCol<uint32_t> tc, bc;
+    const StackCol<uint32_t> col;
     uint32_t idx = 0;
-    AnyWalk<false> w;
+    AnyWalk w;
 
     __device__ __forceinline__ SceneAny(const DevScene &scene, const SceneArgs &args,
                                         const float *tmax, uint8_t *hit, uint32_t *smem)
-        : S(scene), a(args), tmaxs(tmax), out(hit), tc(scene_col(scene, args.c, smem)),
-          bc(mesh_col(scene, args.c, smem)) {}
+        : S(scene), a(args), tmaxs(tmax), out(hit), col(scene_col(scene, args.c, smem)) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
-        if (w.start(S, load_ray(a.O, a.D, i), __ldg(tmaxs + i), tc))
+        if (w.start(S, load_ray(a.O, a.D, i), __ldg(tmaxs + i), col))
             return true;
         finish();
         return false;
     }
-    __device__ __forceinline__ bool step() { return w.step(S, tc, bc); }
+    __device__ __forceinline__ bool step() { return w.step(S, col); }
     __device__ __forceinline__ void finish() { out[idx] = w.occluded ? 1 : 0; }
 };
 
@@ -919,15 +911,14 @@ struct TraceLaunch {
     CallScratch scratch;
 };
 
-int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int mesh_cap, int tlas_cap,
-               size_t entry, int64_t n, int blocks_per_sm, int refill, bool counter_always,
+int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, size_t entry,
+               int64_t n, int blocks_per_sm, int refill, bool counter_always,
                unsigned *counter, bool in_capture, cudaStream_t st) {
-    c.stack_cap = mesh_cap;
-    c.stack_sm = in_capture ? mesh_cap : std::min(mesh_cap, kStackSm);
-    c.tlas_cap = tlas_cap;
+    c.stack_cap = cap;
+    c.stack_sm = in_capture ? cap : std::min(cap, kStackSm);
     c.counter = nullptr;
     c.spill = nullptr;
-    L.smem = (size_t) (tlas_cap + c.stack_sm) * block * entry;
+    L.smem = (size_t) c.stack_sm * block * entry;
     if (L.smem > 227 * 1024)
         return fail(PRR_ERR_UNSUPPORTED, "BVH too deep for the shared-memory stack");
     if (int rc = set_smem(fn, L.smem))
@@ -943,12 +934,12 @@ int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int mesh_
     const bool count = counter_always || (n > warps * 32 && !in_capture);
     size_t bytes = count && !counter ? 256 : 0;
     const size_t spill_at = bytes;
-    if (mesh_cap > c.stack_sm)
-        bytes += (size_t) (mesh_cap - c.stack_sm) * L.grid * block * entry;
+    if (cap > c.stack_sm)
+        bytes += (size_t) (cap - c.stack_sm) * L.grid * block * entry;
     if (bytes)
         if (int rc = L.scratch.alloc(bytes, st))
             return rc;
-    if (mesh_cap > c.stack_sm)
+    if (cap > c.stack_sm)
         c.spill = L.scratch.ptr + spill_at;
     if (count) {
         c.counter = counter ? counter : (unsigned *) L.scratch.ptr;
@@ -1006,7 +997,7 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     const int cap = stack_cap(obj.qstack);
     TraceLaunch L;
     // mode 1 keeps its whole stack in shared memory
-    if (int rc = plan_trace(L, a.c, fn, block, cap, 0, sizeof(uint2), n,
+    if (int rc = plan_trace(L, a.c, fn, block, cap, sizeof(uint2), n,
                             mode > 0 ? cfg->blocks_per_sm : 0, refill, mode > 0, counter,
                             in_capture || mode == 1, st))
         return rc;
@@ -1056,7 +1047,7 @@ int launch_mesh_occluded(const Scene &s, int object, const float *o, const float
     const int block = 128;
     TraceLaunch L;
     if (int rc = plan_trace(L, a.c, (const void *) k_mesh_occluded, block, stack_cap(obj.qstack),
-                            0, sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
+                            sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
     k_mesh_occluded<<<L.grid, block, L.smem, st>>>(a, box, tmax, hit);
     PRR_CUDA_TRY(cudaGetLastError());
@@ -1076,7 +1067,7 @@ int launch_scene_closest(const Scene &s, const float *o, const float *d, int64_t
     SceneArgs a{o, d, (uint32_t) n, {}};
     TraceLaunch L;
     if (int rc = plan_trace(L, a.c, (const void *) k_scene_closest, block,
-                            stack_cap(s.dev.blas_stack), stack_cap(s.dev.tlas_depth),
+                            stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
                             sizeof(uint2), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
     k_scene_closest<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo != nullptr);
@@ -1099,7 +1090,7 @@ int launch_scene_occluded(const Scene &s, const float *o, const float *d, const 
     SceneArgs a{o, d, (uint32_t) n, {}};
     TraceLaunch L;
     if (int rc = plan_trace(L, a.c, (const void *) k_scene_occluded, block,
-                            stack_cap(s.dev.blas_stack), stack_cap(s.dev.tlas_depth),
+                            stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
                             sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
     k_scene_occluded<<<L.grid, block, L.smem, st>>>(s.dev, a, tmax, hit);

@@ -59,9 +59,10 @@ struct Wf {
     int max_depth;
     float clamp;
     uint64_t seed;
-    int tlas_cap, blas_cap; // stack entries a walk may need (tree depth + 1)
+    int tlas_cap, blas_cap; // stack entries a walk may need at the scene and mesh level
     int blas_sm;            // mesh-stack entries kept in shared memory
-    void *spill;            // global part of the mesh stacks ([entry][grid thread])
+    int count_stack;        // binary-walk entries of the counting variants, both levels
+    void *spill;            // global part of the stacks ([entry][grid thread])
     // path state
     uint64_t *rng;
     float4 *ro, *rd;     // current ray
@@ -318,14 +319,11 @@ __device__ __forceinline__ int lanes_used(int n) {
 // ---- extend: closest hit of the queued rays, then sort by material class.
 // Persistent: a lane whose ray is finished takes the next queued ray once
 // `refill` lanes of its warp are idle (one atomic per refill).
-// The scene-level stack of this thread (all in shared memory) and its mesh-level
-// stack (blas_sm entries in shared memory, the rest in the spill buffer).
-template <class E> __device__ __forceinline__ StackCol<E> scene_stack(const Wf &w, E *smem) {
-    return StackCol<E>(smem, nullptr, w.tlas_cap, w.tlas_cap, w.check);
-}
-template <class E> __device__ __forceinline__ StackCol<E> mesh_stack(const Wf &w, E *smem) {
-    return StackCol<E>(smem + (size_t) w.tlas_cap * blockDim.x, (E *) w.spill, w.blas_sm,
-                       w.blas_cap, w.check);
+// This thread's stack: tlas_cap + blas_sm entries in shared memory, the rest in
+// the spill buffer.
+template <class E> __device__ __forceinline__ StackCol<E> path_stack(const Wf &w, E *smem) {
+    return StackCol<E>(smem, (E *) w.spill, w.tlas_cap + w.blas_sm, w.tlas_cap + w.blas_cap,
+                       w.check);
 }
 
 template <bool MULTI>
@@ -336,38 +334,57 @@ __device__ __forceinline__ const DevScene &lane_scene(const DevScene &S0, const 
         return S0;
 }
 
-template <bool MULTI, bool STATS>
+// A traced path's hit record and its place among the next stages: its class
+// as a tag (ordered queues) or an entry of its class's queue. All lanes of the
+// warp call it; cls < 0: nothing to write.
+__device__ __forceinline__ int hit_class(const DevScene &S, int obj) {
+    if (obj < 0)
+        return 0;
+    const int kind = S.materials[S.objects[obj].material].kind;
+    return (kind == kMatMirror || kind == kMatGlass) ? 1 : 2;
+}
+__device__ __forceinline__ void route_path(const Wf &w, int p, int cls) {
+    if (w.ordered) {
+        if (cls >= 0)
+            w.tag[p] = (uint8_t) cls;
+        return;
+    }
+    const int a = warp_append(w.cnt + kCntMiss, cls == 0);
+    const int b = warp_append(w.cnt + kCntDelta, cls == 1);
+    const int c = warp_append(w.cnt + kCntSurf, cls == 2);
+    if (cls == 0)
+        queue_put(w, w.qmiss, a, w.P, p);
+    else if (cls == 1)
+        queue_put(w, w.qdelta, b, w.P, p);
+    else if (cls == 2)
+        queue_put(w, w.qsurf, c, w.P, p);
+}
+
+template <bool MULTI>
 __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int it, int refill) {
     extern __shared__ uint2 smem[];
-    const StackCol<uint2> tc = scene_stack(w, smem), bc = mesh_stack(w, smem);
+    const StackCol<uint2> st = path_stack(w, smem);
     const int *qin = w.qray[it & 1];
     const int n = queue_len(w, w.cnt[kCntRay0 + (it & 1)], w.P);
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    // a lane without a ray has p = -1, or -2 when it takes none
     int p = -1;
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    ClosestWalk<STATS> cw;
-    unsigned cnt_[6] = {0, 0, 0, 0, 0, 0}; // nodes, tris, objects, miss, delta, surface
+    ClosestWalk cw;
     bool more = n > 0;
     if (!more)
         return;
-    // a lane without a ray has p = -1, or -2 when it takes none
     refill = min(refill, lanes_used(n));
     if (lane >= lanes_used(n))
         p = -2;
     for (;;) {
         const bool idle = p == -1;
         const unsigned im = __ballot_sync(full, idle);
-        if (!more && __all_sync(full, p < 0)) {
-            if constexpr (STATS) {
-                const unsigned a[3] = {cnt_[0], cnt_[1], cnt_[2]};
-                const unsigned b[3] = {cnt_[3], cnt_[4], cnt_[5]};
-                flush_stats(w.stats, kStatClosestNodes, a);
-                flush_stats(w.stats, kStatMiss, b);
-            }
+        if (!more && __all_sync(full, p < 0))
             break;
-        }
+        bool done = false;
         if (more && __popc(im) >= refill) {
             const int cnt = __popc(im);
             unsigned base = 0;
@@ -386,50 +403,53 @@ __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int i
                     ls = w.reqs[r].scene;
                 }
                 const float4 o = w.ro[p], d = w.rd[p];
-                cw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z},
-                         tc);
+                done = !cw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z},
+                                 st);
             }
             if constexpr (MULTI)
                 count_req_rays(w, full, take, r, 0);
         }
-        bool done = false;
         const DevScene &S = lane_scene<MULTI>(S0, ls);
-        if (p >= 0) {
-            if constexpr (STATS) {
-                if (S.n_objects > 0)
-                    cnt_[cw.in_mesh ? (cw.ntri > 0 ? 1 : 0) : ((cw.tref & kLeafBit) ? 2 : 0)]++;
-            }
-            done = S.n_objects == 0 || cw.step(S, tc, bc);
-        }
+        if (p >= 0 && !done)
+            done = cw.step(S, st);
         int cls = -1;
         if (done) {
-            w.hit[p] = make_int4(cw.hit_obj, cw.hit_tri, __float_as_int(cw.closest), 0);
-            if (cw.hit_obj < 0) {
-                cls = 0;
-            } else {
-                const int kind = S.materials[S.objects[cw.hit_obj].material].kind;
-                cls = (kind == kMatMirror || kind == kMatGlass) ? 1 : 2;
-            }
-            if constexpr (STATS)
-                cnt_[3 + cls]++;
+            w.hit[p] = make_int4(cw.hit_obj, cw.hit_tri, __float_as_int(cw.best), 0);
+            cls = hit_class(S, cw.hit_obj);
         }
-        if (w.ordered) {
-            if (cls >= 0)
-                w.tag[p] = (uint8_t) cls;
-        } else {
-            const int a = warp_append(w.cnt + kCntMiss, cls == 0);
-            const int b = warp_append(w.cnt + kCntDelta, cls == 1);
-            const int c = warp_append(w.cnt + kCntSurf, cls == 2);
-            if (cls == 0)
-                queue_put(w, w.qmiss, a, w.P, p);
-            else if (cls == 1)
-                queue_put(w, w.qdelta, b, w.P, p);
-            else if (cls == 2)
-                queue_put(w, w.qsurf, c, w.P, p);
-        }
+        route_path(w, p, cls);
         if (done)
             p = -1;
     }
+}
+
+// The counting form of the extend stage (prr_render_counts): the binary walk,
+// which visits the nodes the reference visits, one ray per thread.
+__global__ void k_wf_extend_count(DevScene S, Wf w, int it, int) {
+    extern __shared__ uint2 smem[];
+    SmemStack tst{smem + threadIdx.x, (int) blockDim.x, 0, S.tlas_depth + 1, w.check};
+    SmemStack bst{smem + (size_t) (S.tlas_depth + 1) * blockDim.x + threadIdx.x, (int) blockDim.x,
+                  0, S.blas_depth + 1, w.check};
+    const int n = queue_len(w, w.cnt[kCntRay0 + (it & 1)], w.P);
+    unsigned cls_n[3] = {0, 0, 0};
+    WalkCounts c;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const int k = base + threadIdx.x;
+        int p = 0, cls = -1;
+        if (k < n) {
+            p = w.qray[it & 1][k];
+            const float4 o = w.ro[p], d = w.rd[p];
+            const RayD r{o.x, o.y, o.z, d.x, d.y, d.z};
+            const SceneHit h = scene_closest<true>(S, r, precompute(r), tst, bst, &c);
+            w.hit[p] = make_int4(h.obj, h.tri, __float_as_int(h.t), 0);
+            cls = hit_class(S, h.obj);
+            cls_n[cls]++;
+        }
+        route_path(w, p, cls);
+    }
+    const unsigned work[3] = {c.nodes, c.tris, c.objects};
+    flush_stats(w.stats, kStatClosestNodes, work);
+    flush_stats(w.stats, kStatMiss, cls_n);
 }
 
 // Hit record -> Inter (Triangle::finalize / Sphere::getIntersection fields).
@@ -771,21 +791,31 @@ __global__ void __launch_bounds__(128, 8) k_wf_surface(DevScene S0, Wf w, int it
 }
 
 // ---- shadow: visibility of every queued NEE ray (persistent, per-lane refill)
-template <bool MULTI, bool STATS>
+// Adds up the rays each lane traced.
+__device__ __forceinline__ void count_shadow_rays(const Wf &w, unsigned rays) {
+    for (int off = 16; off > 0; off >>= 1)
+        rays += __shfl_down_sync(0xffffffffu, rays, off);
+    if ((threadIdx.x & 31) == 0 && rays)
+        atomicAdd(reinterpret_cast<unsigned long long *>(w.cnt + kCntShadowRays),
+                  (unsigned long long) rays);
+}
+
+template <bool MULTI>
 __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int refill) {
     extern __shared__ uint32_t smem32[];
-    const StackCol<uint32_t> tc = scene_stack(w, smem32), bc = mesh_stack(w, smem32);
+    const StackCol<uint32_t> st = path_stack(w, smem32);
     const int n = queue_len(w, w.cnt[kCntShadowJobs], 2 * (int64_t) w.P);
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int job = -1;
+    int job = -1; // -2: a lane that takes no rays
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    AnyWalk<STATS> aw;
+    AnyWalk aw;
     bool more = n > 0;
+    if (!more)
+        return;
     unsigned rays = 0;
-    unsigned cnt_[3] = {0, 0, 0}; // nodes, tris, objects
-    refill = min(refill, lanes_used(n)); // a lane that takes no rays: job = -2
+    refill = min(refill, lanes_used(n));
     if (lane >= lanes_used(n))
         job = -2;
     for (;;) {
@@ -815,49 +845,57 @@ __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int r
                 const float4 d = (job & 1) ? w.sed[p] : w.sld[p];
                 rays++;
                 if (!aw.start(lane_scene<MULTI>(S0, ls), RayD{o.x, o.y, o.z, d.x, d.y, d.z}, o.w,
-                              tc)) {
-                    w.vis[job] = 1;
+                              st)) {
+                    w.vis[job] = aw.occluded ? 0 : 1;
                     job = -1;
                 }
             }
             if constexpr (MULTI)
                 count_req_rays(w, full, take, r, 1);
         }
-        const DevScene &S = lane_scene<MULTI>(S0, ls);
-        if constexpr (STATS) {
-            if (job >= 0)
-                cnt_[aw.in_mesh ? (aw.ntri > 0 ? 1 : 0) : ((aw.tref & kLeafBit) ? 2 : 0)]++;
-        }
-        if (job >= 0 && aw.step(S, tc, bc)) {
+        if (job >= 0 && aw.step(lane_scene<MULTI>(S0, ls), st)) {
             w.vis[job] = aw.occluded ? 0 : 1;
             job = -1;
         }
     }
-    if constexpr (STATS)
-        flush_stats(w.stats, kStatShadowNodes, cnt_);
-    for (int off = 16; off > 0; off >>= 1)
-        rays += __shfl_down_sync(full, rays, off);
-    if (lane == 0 && rays)
-        atomicAdd(reinterpret_cast<unsigned long long *>(w.cnt + kCntShadowRays),
-                  (unsigned long long) rays);
+    count_shadow_rays(w, rays);
+}
+
+// The counting form, as k_wf_extend_count.
+__global__ void k_wf_shadow_count(DevScene S, Wf w, int) {
+    extern __shared__ uint2 smem[];
+    SmemStack tst{smem + threadIdx.x, (int) blockDim.x, 0, S.tlas_depth + 1, w.check};
+    SmemStack bst{smem + (size_t) (S.tlas_depth + 1) * blockDim.x + threadIdx.x, (int) blockDim.x,
+                  0, S.blas_depth + 1, w.check};
+    const int n = queue_len(w, w.cnt[kCntShadowJobs], 2 * (int64_t) w.P);
+    unsigned rays = 0;
+    WalkCounts c;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int job = w.qjob[k], p = job >> 1;
+        const float4 o = (job & 1) ? w.seo[p] : w.slo[p];
+        const float4 d = (job & 1) ? w.sed[p] : w.sld[p];
+        const RayD r{o.x, o.y, o.z, d.x, d.y, d.z};
+        rays++;
+        w.vis[job] = scene_occluded<true>(S, r, precompute(r), tst, bst, o.w, &c) ? 0 : 1;
+    }
+    const unsigned work[3] = {c.nodes, c.tris, c.objects};
+    flush_stats(w.stats, kStatShadowNodes, work);
+    count_shadow_rays(w, rays);
 }
 
 // The traversal stages on the four-wide nodes, 64 registers at most (8 resident
 // blocks of 128). Tighter caps gain blocks but spill the four boxes' distances:
-// museum-like scene of 491,520 triangles at 960x540, 16 spp: 16.9 ms, 17.6 at
-// 56 registers, 19.0 at 48; 18.5 on the binary nodes (at their best cap, 48).
-template <bool MULTI, bool STATS = false>
+// museum-like scene of 491,520 triangles at 960x540, 16 spp, append-order
+// queues: 16.9 ms, 17.6 at 56 registers, 19.0 at 48; 18.5 on the binary nodes
+// (at their best cap, 48). 13.2 ms with the default queues and one walk for
+// both levels.
+template <bool MULTI>
 __global__ void __maxnreg__(64) k_wf_extend(DevScene S, Wf w, int it, int refill) {
-    wf_extend<MULTI, STATS>(S, w, it, refill);
+    wf_extend<MULTI>(S, w, it, refill);
 }
-// The server's extend stage (paths of several requests; the request index
-// selects scene and camera).
-__global__ void __maxnreg__(64) k_wf_extend_multi(DevScene S, Wf w, int it, int refill) {
-    wf_extend<true, false>(S, w, it, refill);
-}
-template <bool MULTI, bool STATS = false>
+template <bool MULTI>
 __global__ void __maxnreg__(64) k_wf_shadow(DevScene S, Wf w, int refill) {
-    wf_shadow<MULTI, STATS>(S, w, refill);
+    wf_shadow<MULTI>(S, w, refill);
 }
 
 // ---- add the visible NEE contributions, light first, then env, as castRay
@@ -1300,12 +1338,18 @@ int wf_shape(Wf &w, DevBuf &spill, int block_req, int stack_req, int refill_req,
     w.blas_sm = std::max(1, std::min(w.blas_sm, max_sm_entries - w.tlas_cap));
     L.smem_ext = (size_t) (w.tlas_cap + w.blas_sm) * L.block * sizeof(uint2);
     L.smem_sh = (size_t) (w.tlas_cap + w.blas_sm) * L.block * sizeof(uint32_t);
-    L.ext = MULTI ? k_wf_extend_multi : k_wf_extend<false>;
+    L.ext = k_wf_extend<MULTI>;
     L.sh = k_wf_shadow<MULTI>;
     if constexpr (!MULTI) {
-        if (w.stats) { // the counting variants (a separate, untimed render)
-            L.ext = k_wf_extend<false, true>;
-            L.sh = k_wf_shadow<false, true>;
+        if (w.stats) {
+            // the counting variants (a separate, untimed render): whole binary
+            // stacks in shared memory, so one-warp blocks for deep trees
+            L.ext = k_wf_extend_count;
+            L.sh = k_wf_shadow_count;
+            L.block = 32;
+            L.smem_ext = L.smem_sh = (size_t) w.count_stack * L.block * sizeof(uint2);
+            if (L.smem_ext > 227 * 1024)
+                return fail(PRR_ERR_UNSUPPORTED, "BVH too deep for the counting render");
         }
     }
     if (L.smem_ext > 48 * 1024)
@@ -1431,8 +1475,9 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.clamp = rs.indirect_clamp;
     w.seed = rs.seed;
     w.sample_offset = rs.sample_offset;
-    w.tlas_cap = S.tlas_depth + 1;
-    w.blas_cap = (s.wf_stats ? S.blas_depth : S.blas_stack) + 1;
+    w.tlas_cap = S.tlas_stack + 1;
+    w.blas_cap = S.blas_stack + 1;
+    w.count_stack = S.tlas_depth + S.blas_depth + 2;
     // Paths per pass: whole samples of the window, by default at most 32M in
     // flight (10 GB of path state): every bounce of a pass ends in a tail of
     // long rays, so fewer and larger passes pay it less often (museum-like

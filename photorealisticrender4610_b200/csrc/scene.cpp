@@ -87,18 +87,20 @@ int pack_tree(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<WN
 // per two levels would outgrow sooner.
 constexpr int kMaxQuadStack = 64;
 
-// Collapse one mesh's tree into four-wide nodes (QNode) appended to `out`:
+// Collapse one tree (a mesh's, or the scene's over objects) into four-wide nodes (QNode) appended to `out`:
 // node, grandchildren, great-great-grandchildren and so on. A child is
 // collapsed when it is interior and its box is exactly the union of its
 // children's boxes, which the walk's exactness rests on (a NaN in a box fails
 // the comparison); otherwise it stays a child of its own. Returns the root
 // reference and how many entries a walk's stack can hold: every child of a
 // node but the one entered may wait on it.
-void pack_quads(const FlatBVH &f, int tri_base, std::vector<QNode> &out, uint32_t &root_ref,
-                int &stack) {
+void pack_quads(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<QNode> &out,
+                uint32_t &root_ref, int &stack) {
     const size_t n = f.size();
     auto count = [&](size_t i) { return f.meta[i] & 0x00FFFFFFu; };
     auto leaf_ref = [&](size_t i) {
+        if (object_leaves)
+            return kLeafBit | (uint32_t) f.ordered[f.first_child[i]];
         return mesh_leaf_ref((uint32_t) (tri_base + f.first_child[i]), count(i));
     };
     stack = 0;
@@ -371,7 +373,7 @@ int build_scene(Scene &s, cudaStream_t st) {
         }
         if (int rc = pack_tree(o.bvh, false, base, nodes, o.root))
             return rc;
-        pack_quads(o.bvh, base, qnodes, o.qroot, o.qstack);
+        pack_quads(o.bvh, false, base, qnodes, o.qroot, o.qstack);
         blas_stack = std::max(blas_stack, o.qstack);
         blas_depth = std::max(blas_depth, o.bvh.max_depth);
         base += (int) nt;
@@ -416,6 +418,9 @@ int build_scene(Scene &s, cudaStream_t st) {
     if (!s.objects.empty())
         if (int rc = pack_tree(s.tlas, true, 0, nodes, tlas_root))
             return rc;
+    uint32_t tlas_qroot = 0;
+    int tlas_stack = 0;
+    pack_quads(s.tlas, true, 0, qnodes, tlas_qroot, tlas_stack);
 
     // ---- objects, materials, emitters (Scene.cpp:19-26) ----
     std::vector<DevObject> dobj(s.objects.size());
@@ -552,6 +557,8 @@ int build_scene(Scene &s, cudaStream_t st) {
             D.has_emissive_kind = 1;
     D.total_emit_area = emit_area;
     D.tlas_root = tlas_root;
+    D.tlas_qroot = tlas_qroot;
+    D.tlas_stack = tlas_stack;
     if (!s.objects.empty())
         for (int q = 0; q < 6; q++)
             D.tlas_box[q] = s.tlas.bounds[q];

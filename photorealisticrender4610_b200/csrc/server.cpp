@@ -525,7 +525,7 @@ int prr_server_add_scene(prr_server *server, prr_scene *scene, int *out_id) {
     S.scenes.push_back(&sc);
     S.scene_bytes.push_back(sc.device_bytes);
     S.used += sc.device_bytes;
-    S.tlas_cap = std::max(S.tlas_cap, sc.dev.tlas_depth + 1);
+    S.tlas_cap = std::max(S.tlas_cap, std::max(sc.dev.tlas_depth, sc.dev.tlas_stack) + 1);
     S.blas_cap = std::max(S.blas_cap, std::max(sc.dev.blas_depth, sc.dev.blas_stack) + 1);
     std::vector<DevScene> all;
     for (Scene *p : S.scenes)

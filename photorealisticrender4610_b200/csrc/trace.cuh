@@ -604,6 +604,12 @@ struct SmemStack {
     }
 };
 
+// Work of a binary walk: interior nodes of either level, triangle tests, object
+// leaves (mesh entries and sphere tests).
+struct WalkCounts {
+    unsigned nodes = 0, tris = 0, objects = 0;
+};
+
 // BVHAccel::Intersect, triangle fast path (BVH.cpp:311-415) on one mesh's
 // four-wide nodes. best_t enters as +inf (every mesh-level search starts
 // fresh, BVH.cpp:331). Returns the winning triangle's global leaf-order index,
@@ -659,17 +665,20 @@ __device__ __forceinline__ int blas_closest_quad(const QNode *__restrict__ nodes
 // registers cost those more than its shorter walk saves (museum-like scene of
 // 122,880 triangles at 480x270, 16 spp: 12.4 ms, 14.4 four-wide; Cornell box
 // 2.2 against 2.7).
+template <bool COUNT = false>
 __device__ __forceinline__ int blas_closest(const WNode *__restrict__ nodes,
                                             const Tri *__restrict__ tris,
                                             const float *__restrict__ e2z, uint32_t root,
                                             const RayD &r, const RayPre &p, SmemStack &st,
                                             float &best_t, float &best_u, float &best_v,
-                                            const TraceBounds &B) {
+                                            const TraceBounds &B, WalkCounts *wc = nullptr) {
     const int sp0 = st.sp;
     uint32_t ref = root;
     int hit = -1;
     for (;;) {
         if (!(ref & kLeafBit)) {
+            if constexpr (COUNT)
+                wc->nodes++;
             const NodeV n = load_node(nodes, ref, B);
             const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
             const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
@@ -692,6 +701,8 @@ __device__ __forceinline__ int blas_closest(const WNode *__restrict__ nodes,
             const uint32_t first = leaf_first(ref);
             const uint32_t cnt = leaf_count(ref);
             for (uint32_t i = 0; i < cnt; i++) {
+                if constexpr (COUNT)
+                    wc->tris++;
                 const TriV T = load_tri(tris, e2z, first + i, B);
                 float t, u, v;
                 if (tri_hit(T, r, t, u, v) && t < best_t) {
@@ -715,18 +726,21 @@ __device__ __forceinline__ int blas_closest(const WNode *__restrict__ nodes,
     }
 }
 
+template <bool COUNT = false>
 __device__ __forceinline__ bool blas_occluded(const WNode *__restrict__ nodes,
                                               const Tri *__restrict__ tris,
                                               const float *__restrict__ e2z, uint32_t root,
                                               const float *root_box, const RayD &r,
                                               const RayPre &p, SmemStack &st, float tmax,
-                                              const TraceBounds &B) {
+                                              const TraceBounds &B, WalkCounts *wc = nullptr) {
     if (!(slab6(root_box, p) < tmax))
         return false;
     const int sp0 = st.sp;
     uint32_t ref = root;
     for (;;) {
         if (!(ref & kLeafBit)) {
+            if constexpr (COUNT)
+                wc->nodes++;
             const NodeV n = load_node(nodes, ref, B);
             const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
             const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
@@ -747,6 +761,8 @@ __device__ __forceinline__ bool blas_occluded(const WNode *__restrict__ nodes,
             const uint32_t first = leaf_first(ref);
             const uint32_t cnt = leaf_count(ref);
             for (uint32_t i = 0; i < cnt; i++) {
+                if constexpr (COUNT)
+                    wc->tris++;
                 const TriV T = load_tri(tris, e2z, first + i, B);
                 if (tri_occludes(T, r, tmax)) {
                     st.sp = sp0;
@@ -805,9 +821,10 @@ struct SceneHit {
 // Scene::intersect -> BVHAccel::Intersect, general path (BVH.cpp:359-369):
 // every scene-BVH leaf object is intersected on its own (meshes start their
 // own search at +inf) and replaces the winner when tnear < closestT.
+template <bool COUNT = false>
 __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD &r,
                                                   const RayPre &p, SmemStack &tst,
-                                                  SmemStack &bst) {
+                                                  SmemStack &bst, WalkCounts *wc = nullptr) {
     SceneHit h;
     h.obj = -1;
     h.tri = -1;
@@ -820,6 +837,8 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD 
     uint32_t ref = S.tlas_root;
     for (;;) {
         if (!(ref & kLeafBit)) {
+            if constexpr (COUNT)
+                wc->nodes++;
             const NodeV n = load_node(S, ref);
             const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
             const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
@@ -841,10 +860,12 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD 
         } else {
             const int k = (int) (ref & ~kLeafBit);
             const DevObject &o = S.objects[k];
+            if constexpr (COUNT)
+                wc->objects++;
             if (o.kind == kObjMesh) {
                 float t = kInf, u = 0.f, v = 0.f;
-                const int tri = blas_closest(S.nodes, S.tris, S.tri_e2z, o.root, r, p, bst, t, u, v,
-                                             bounds_of(S));
+                const int tri = blas_closest<COUNT>(S.nodes, S.tris, S.tri_e2z, o.root, r, p, bst, t, u, v,
+                                             bounds_of(S), wc);
                 if (tri >= 0 && t < closest) {
                     closest = t;
                     h.obj = k;
@@ -880,9 +901,10 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD 
 // occluder (Triangle.hpp:141-147) and Sphere falls back to
 // Object::intersectT (Object.hpp:24-29); the caller then requires
 // t >= 0 && t < tMax.
+template <bool COUNT = false>
 __device__ __forceinline__ bool scene_occluded(const DevScene &S, const RayD &r,
                                                const RayPre &p, SmemStack &tst, SmemStack &bst,
-                                               float tmax) {
+                                               float tmax, WalkCounts *wc = nullptr) {
     if (S.n_objects == 0)
         return false;
     if (!(slab6(S.tlas_box, p) < tmax))
@@ -891,6 +913,8 @@ __device__ __forceinline__ bool scene_occluded(const DevScene &S, const RayD &r,
     uint32_t ref = S.tlas_root;
     for (;;) {
         if (!(ref & kLeafBit)) {
+            if constexpr (COUNT)
+                wc->nodes++;
             const NodeV n = load_node(S, ref);
             const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
             const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
@@ -909,9 +933,11 @@ __device__ __forceinline__ bool scene_occluded(const DevScene &S, const RayD &r,
         } else {
             const DevObject &o = S.objects[ref & ~kLeafBit];
             bool occ;
+            if constexpr (COUNT)
+                wc->objects++;
             if (o.kind == kObjMesh) {
-                occ = blas_occluded(S.nodes, S.tris, S.tri_e2z, o.root, o.root_box, r, p, bst, tmax,
-                                    bounds_of(S)) &&
+                occ = blas_occluded<COUNT>(S.nodes, S.tris, S.tri_e2z, o.root, o.root_box, r, p, bst, tmax,
+                                    bounds_of(S), wc) &&
                       (1e-3f < tmax);
             } else {
                 float t;

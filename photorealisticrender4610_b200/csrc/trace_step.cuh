@@ -1,300 +1,224 @@
 // Two-level scene traversal as resumable per-lane state machines, for
 // persistent kernels whose lanes take new rays as soon as theirs finish.
-// Each call to step() does one unit of work -- one interior node, one
-// triangle, one sphere, or entering a mesh -- in exactly the order of the
+// Each call to step() does one unit of work -- one four-wide node of either
+// level, or one triangle -- and leaves are taken in exactly the order of the
 // walks in trace.cuh (scene_closest / scene_occluded, which restate
 // BVH.cpp:311-473 over MeshTriangle and Sphere leaves), so results are
 // identical; only the scheduling of rays onto lanes changes.
+//
+// Both levels are four-wide nodes, and one stack holds the entries of both:
+// those of the mesh being walked lie above the scene's (from `floor` up). So a
+// warp whose lanes are at scene nodes and mesh nodes runs one piece of code,
+// where separate levels, and entering an object as a step of its own, split
+// it four ways (museum-like 960x540, 16 spp: 14.2 -> 13.2 ms; 2,000,003
+// closest-hit rays on 122,880 triangles 0.58 -> 0.50 ms). Both walks take 64
+// registers without spills.
 #pragma once
 #include "trace.cuh"
 
 namespace prr {
 
 // Closest hit: Scene::intersect -> scene BVH, general path; each mesh leaf is
-// searched from +inf on its own (BVH.cpp:359-369). BINARY walks the binary
-// mesh nodes instead of the four-wide ones, a step being one of the
-// reference's interior visits: the counting variants of the wavefront stages
-// (prr_render_counts report the reference's traversal work).
-template <bool BINARY = false> struct ClosestWalk {
+// searched from +inf on its own (BVH.cpp:359-369).
+struct ClosestWalk {
     RayD r;
     RayPre p;
-    float closest;
+    float best;    // closest hit of the level being walked
+    float closest; // the scene's, while a mesh is walked
     int hit_obj, hit_tri;
-    uint32_t tref;
-    uint32_t tsp;
-    bool in_mesh;
-    int cur_obj;
-    uint32_t bref, tri, ntri;
-    float bbest;
-    int bhit;
-    uint32_t bsp;
+    int cur_obj;   // mesh being walked, -1 at the scene level
+    int bhit;      // its closest triangle
+    uint32_t ref;  // next node, or next triangle when ntri > 0
+    uint32_t ntri; // triangles left in the current leaf
+    uint32_t top, floor;
 
-    __device__ __forceinline__ void start(const DevScene &S, const RayD &ray,
-                                          const StackCol<uint2> &tc) {
+    // false when the ray is over at once (a miss)
+    __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray,
+                                          const StackCol<uint2> &st) {
         r = ray;
         p = precompute(ray);
-        closest = kInf;
-        hit_obj = hit_tri = -1;
-        tref = S.tlas_root;
-        tsp = tc.base;
-        in_mesh = false;
+        best = closest = kInf;
+        hit_obj = hit_tri = cur_obj = -1;
+        top = floor = st.base;
         ntri = 0;
+        if (S.n_objects == 0 || no_slab(p))
+            return false;
+        // a scene of one sphere is answered here
+        return go(S, S.tlas_qroot);
     }
 
-    // pops the scene-level stack; true when the walk is over
-    __device__ __forceinline__ bool scene_pop(const StackCol<uint2> &tc) {
-        while (!tc.empty(tsp)) {
-            const uint2 e = tc.pop(tsp);
-            if (__uint_as_float(e.y) < closest) {
-                tref = e.x;
+    // Moves on to a child reference: false when it is a sphere, tested here.
+    __device__ __forceinline__ bool go(const DevScene &S, uint32_t x) {
+        ref = x;
+        if (!(x & kLeafBit))
+            return true;
+        if (cur_obj < 0) {
+            const int k = (int) (x & ~kLeafBit);
+            const DevObject &o = S.objects[k];
+            if (o.kind != kObjMesh) {
+                float t;
+                if (sphere_hit(o, r, t) && t < best) {
+                    best = t;
+                    hit_obj = k;
+                    hit_tri = -1;
+                }
                 return false;
             }
+            cur_obj = k;
+            closest = best;
+            best = kInf;
+            bhit = -1;
+            floor = top;
+            ref = o.qroot;
+            if (!(ref & kLeafBit))
+                return true;
         }
+        ntri = leaf_count(ref);
+        ref = leaf_first(ref);
         return true;
     }
 
-    __device__ __forceinline__ void set_mesh_ref(uint32_t ref) {
-        if (ref & kLeafBit) {
-            tri = leaf_first(ref);
-            ntri = leaf_count(ref);
-        } else {
-            bref = ref;
-            ntri = 0;
-        }
-    }
-
-    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint2> &tc,
-                                         const StackCol<uint2> &bc) {
-        if (in_mesh) {
-            bool pop = false;
-            if (ntri > 0) {
-                const TriV T = load_tri(S, tri);
-                float t, u, v;
-                if (tri_hit(T, r, t, u, v) && t < bbest) {
-                    bbest = t;
-                    bhit = (int) tri;
-                }
-                tri++;
-                ntri--;
-                pop = ntri == 0;
-            } else {
-                uint32_t next;
-                bool down;
-                if constexpr (BINARY) {
-                    const NodeV n = load_node(S, bref);
-                    const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-                    const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-                    const bool left = tl <= tr;
-                    down = (left ? tl : tr) < bbest;
-                    next = left ? n.link.x : n.link.y;
-                    if ((left ? tr : tl) < bbest)
-                        bc.put(bsp, make_uint2(left ? n.link.y : n.link.x,
-                                               __float_as_uint(left ? tr : tl)));
-                } else {
-                    const QuadOrder q = quad_order(load_quad(S, bref), p);
-                    push_rest(bc, bsp, q, bbest);
-                    down = q.any(bbest);
-                    next = q.next(bbest);
-                }
-                if (down) {
-                    set_mesh_ref(next);
-                    return false;
-                }
-                pop = true;
+    // one unit of work; true when the walk is over
+    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint2> &st) {
+        bool down = false;
+        uint32_t x = 0;
+        if (ntri > 0) {
+            const TriV T = load_tri(S, ref);
+            float t, u, v;
+            if (tri_hit(T, r, t, u, v) && t < best) {
+                best = t;
+                bhit = (int) ref;
             }
-            if (!pop)
+            ref++;
+            if (--ntri > 0)
                 return false;
-            while (!bc.empty(bsp)) {
-                const uint2 e = bc.pop(bsp);
-                if (__uint_as_float(e.y) < bbest) {
-                    set_mesh_ref(e.x);
-                    return false;
+        } else {
+            const QuadOrder q = quad_order(load_quad(S, ref), p);
+            push_rest(st, top, q, best);
+            down = q.any(best);
+            x = q.next(best);
+        }
+        for (;;) {
+            if (!down) {
+                if (top == floor) {
+                    if (cur_obj < 0)
+                        return true;
+                    // mesh finished: MeshTriangle::getIntersection's answer
+                    if (bhit >= 0 && best < closest) {
+                        closest = best;
+                        hit_obj = cur_obj;
+                        hit_tri = bhit;
+                    }
+                    best = closest;
+                    cur_obj = -1;
+                    floor = st.base;
+                    continue;
                 }
+                const uint2 e = st.pop(top);
+                if (!(__uint_as_float(e.y) < best))
+                    continue;
+                x = e.x;
             }
-            // mesh finished: MeshTriangle::getIntersection's answer
-            if (bhit >= 0 && bbest < closest) {
-                closest = bbest;
-                hit_obj = cur_obj;
-                hit_tri = bhit;
-            }
-            in_mesh = false;
-            return scene_pop(tc);
+            if (go(S, x))
+                return false;
+            down = false;
         }
-        if (!(tref & kLeafBit)) {
-            const NodeV n = load_node(S, tref);
-            const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-            const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-            if (tl <= tr) {
-                if (tl < closest) {
-                    if (tr < closest)
-                        tc.put(tsp, make_uint2(n.link.y, __float_as_uint(tr)));
-                    tref = n.link.x;
-                    return false;
-                }
-            } else {
-                if (tr < closest) {
-                    if (tl < closest)
-                        tc.put(tsp, make_uint2(n.link.x, __float_as_uint(tl)));
-                    tref = n.link.y;
-                    return false;
-                }
-            }
-            return scene_pop(tc);
-        }
-        const int k = (int) (tref & ~kLeafBit);
-        const DevObject &o = S.objects[k];
-        if (o.kind == kObjMesh) {
-            if (!(o.qroot & kLeafBit) && no_slab(p))
-                return scene_pop(tc);
-            in_mesh = true;
-            cur_obj = k;
-            bbest = kInf;
-            bhit = -1;
-            bsp = bc.base;
-            set_mesh_ref(BINARY ? o.root : o.qroot);
-            return false;
-        }
-        float t;
-        if (sphere_hit(o, r, t) && t < closest) {
-            closest = t;
-            hit_obj = k;
-            hit_tri = -1;
-        }
-        return scene_pop(tc);
     }
 };
 
 // Any hit: Scene::intersectP -> scene BVH IntersectP over MeshTriangle /
 // Sphere intersectT (BVH.cpp:421-473, Triangle.hpp:141-147, Object.hpp:24-29).
-// BINARY as above: the reference's interior visits, in its order.
-template <bool BINARY = false> struct AnyWalk {
+// Leaves are taken near ones first rather than in the reference's order: the
+// answer is whether any of those entered before tmax occludes.
+struct AnyWalk {
     RayD r;
     RayPair p;
     float tmax;
-    uint32_t tref;
-    uint32_t tsp;
-    bool in_mesh;
-    uint32_t bref, tri, ntri;
-    uint32_t bsp;
-    bool occluded;
+    uint32_t ref, ntri;
+    uint32_t top, floor;
+    bool in_mesh, occluded;
 
-    // false when the scene's root box already misses
+    // false when the walk is over at once (nothing in the way, or a sphere)
     __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray, float t_max,
-                                          const StackCol<uint32_t> &tc) {
+                                          const StackCol<uint32_t> &st) {
         r = ray;
         p = precompute_pair(ray);
         tmax = t_max;
-        tref = S.tlas_root;
-        tsp = tc.base;
-        in_mesh = false;
+        top = floor = st.base;
         ntri = 0;
-        occluded = false;
-        return S.n_objects > 0 && slab6(S.tlas_box, p) < tmax;
+        in_mesh = occluded = false;
+        if (S.n_objects == 0 || !(slab6(S.tlas_box, p) < tmax) || no_slab(p))
+            return false;
+        return go(S, S.tlas_qroot);
     }
 
-    __device__ __forceinline__ void set_mesh_ref(uint32_t ref) {
-        if (ref & kLeafBit) {
-            tri = leaf_first(ref);
-            ntri = leaf_count(ref);
-        } else {
-            bref = ref;
-            ntri = 0;
-        }
-    }
-
-    __device__ __forceinline__ bool scene_pop(const StackCol<uint32_t> &tc) {
-        if (tc.empty(tsp))
+    // Moves on to a child reference: false when there is nothing to walk there
+    // (a sphere, tested here, or a mesh whose box is beyond tmax).
+    __device__ __forceinline__ bool go(const DevScene &S, uint32_t x) {
+        ref = x;
+        if (!(x & kLeafBit))
             return true;
-        tref = tc.pop(tsp);
-        return false;
+        if (!in_mesh) {
+            const DevObject &o = S.objects[x & ~kLeafBit];
+            if (o.kind != kObjMesh) {
+                float t;
+                occluded = sphere_hit(o, r, t) && t < tmax && t >= 0.f;
+                return false;
+            }
+            // the mesh's own IntersectP first tests its root box
+            if (!(slab6(o.root_box, p) < tmax))
+                return false;
+            in_mesh = true;
+            floor = top;
+            ref = o.qroot;
+            if (!(ref & kLeafBit))
+                return true;
+        }
+        ntri = leaf_count(ref);
+        ref = leaf_first(ref);
+        return true;
     }
 
     // one unit of work; true when the walk is over (result in `occluded`)
-    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint32_t> &tc,
-                                         const StackCol<uint32_t> &bc) {
-        if (in_mesh) {
-            if (ntri > 0) {
-                const TriV T = load_tri(S, tri);
-                if (tri_occludes(T, r, tmax)) {
-                    // MeshTriangle::intersectT answers 1e-3; the scene-level
-                    // caller then needs 1e-3 < tMax
-                    in_mesh = false;
-                    if (1e-3f < tmax) {
-                        occluded = true;
+    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint32_t> &st) {
+        bool down = false;
+        uint32_t x = 0;
+        if (ntri > 0) {
+            if (tri_occludes(load_tri(S, ref), r, tmax)) {
+                // MeshTriangle::intersectT answers 1e-3; the scene-level
+                // caller then needs 1e-3 < tMax
+                if (1e-3f < tmax) {
+                    occluded = true;
+                    return true;
+                }
+                ntri = 1;
+                top = floor;
+            }
+            ref++;
+            if (--ntri > 0)
+                return false;
+        } else {
+            const QuadOrder q = quad_order(load_quad(S, ref), p);
+            push_rest(st, top, q, tmax);
+            down = q.any(tmax);
+            x = q.next(tmax);
+        }
+        for (;;) {
+            if (!down) {
+                if (top == floor) {
+                    if (top == st.base)
                         return true;
-                    }
-                    return scene_pop(tc);
+                    in_mesh = false;
+                    floor = st.base;
                 }
-                tri++;
-                ntri--;
-                if (ntri > 0)
-                    return false;
-            } else {
-                uint32_t next;
-                bool down;
-                if constexpr (BINARY) {
-                    const NodeV n = load_node(S, bref);
-                    const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-                    const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-                    const uint32_t axis = n.link.z;
-                    const bool neg = axis == 0 ? p.nx : (axis == 1 ? p.ny : p.nz);
-                    down = (neg ? tr : tl) < tmax; // octant 0 -> near = left
-                    next = neg ? n.link.y : n.link.x;
-                    if ((neg ? tl : tr) < tmax)
-                        bc.put(bsp, neg ? n.link.x : n.link.y);
-                } else {
-                    const QuadOrder q = quad_order(load_quad(S, bref), p);
-                    push_rest(bc, bsp, q, tmax);
-                    down = q.any(tmax);
-                    next = q.next(tmax);
-                }
-                if (down) {
-                    set_mesh_ref(next);
-                    return false;
-                }
+                x = st.pop(top);
             }
-            if (!bc.empty(bsp)) {
-                set_mesh_ref(bc.pop(bsp));
+            if (go(S, x))
                 return false;
-            }
-            in_mesh = false;
-            return scene_pop(tc);
+            if (occluded)
+                return true;
+            down = false;
         }
-        if (!(tref & kLeafBit)) {
-            const NodeV n = load_node(S, tref);
-            const float tl = slab(n.a.x, n.a.y, n.a.z, n.a.w, n.b.x, n.b.y, p);
-            const float tr = slab(n.b.z, n.b.w, n.c.x, n.c.y, n.c.z, n.c.w, p);
-            const uint32_t axis = n.link.z;
-            const bool neg = axis == 0 ? p.nx : (axis == 1 ? p.ny : p.nz);
-            const uint32_t near_ref = neg ? n.link.y : n.link.x;
-            const uint32_t far_ref = neg ? n.link.x : n.link.y;
-            const float tnear = neg ? tr : tl;
-            const float tfar = neg ? tl : tr;
-            if (tfar < tmax)
-                tc.put(tsp, far_ref);
-            if (tnear < tmax) {
-                tref = near_ref;
-                return false;
-            }
-            return scene_pop(tc);
-        }
-        const DevObject &o = S.objects[tref & ~kLeafBit];
-        if (o.kind == kObjMesh) {
-            // the mesh's own IntersectP first tests its root box
-            if (slab6(o.root_box, p) < tmax && ((o.qroot & kLeafBit) || !no_slab(p))) {
-                in_mesh = true;
-                bsp = bc.base;
-                set_mesh_ref(BINARY ? o.root : o.qroot);
-                return false;
-            }
-            return scene_pop(tc);
-        }
-        float t;
-        if (sphere_hit(o, r, t) && t < tmax && t >= 0.f) {
-            occluded = true;
-            return true;
-        }
-        return scene_pop(tc);
     }
 };
 
