@@ -640,6 +640,8 @@ __device__ __forceinline__ int next_slab(const uint32_t *occ, int c, int hi) {
 template <class C>
 __device__ __forceinline__ void walk_columns(const GridView &v, const GridParams &g, int x0,
                                              int x1, int y0, int y1, int z0, int z1, C &&col) {
+    if (z0 > z1)
+        return; // beyond the grid along z: its columns are not this box's
     for (int cx = next_slab(g.occ[0], x0, x1); cx <= x1; cx = next_slab(g.occ[0], cx + 1, x1))
         for (int cy = next_slab(g.occ[1], y0, y1); cy <= y1;
              cy = next_slab(g.occ[1], cy + 1, y1)) {

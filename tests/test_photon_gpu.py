@@ -388,3 +388,17 @@ def test_emit_odd_photon_count(cuda, n):
     b = recs[1][[firsts[1][k] for k in common]]
     assert np.array_equal(a[:, :6].view(np.uint32), b[:, :6].view(np.uint32))
     assert np.allclose(a[:, 6:], b[:, 6:] * ((n + 1) / n), rtol=1e-5)
+
+
+def test_gather_outside_the_grid(cuda):
+    """Points beyond the photons along one axis, near or far, get nothing (the
+    cell table is not read outside its range)."""
+    rec, _ = random_photons(20000, 9)
+    pm = prr.PhotonMap().set(rec).build(0.05)
+    for k in (0, 16):
+        for axis in range(3):
+            for far in (3.0, -3.0, 1e5, -1e5, 1e30):
+                q = np.zeros((64, 3), np.float32)
+                q[:, (axis + 1) % 3] = np.linspace(-0.02, 0.02, 64)
+                q[:, axis] = far
+                assert not pm.gather(q, k_nearest=k).cpu().numpy().any(), (k, axis, far)
