@@ -778,37 +778,7 @@ __device__ __noinline__ V3 knn_estimate(const GridView &v, const GatherBox &b, V
     return ek / disc_area(rk);
 }
 
-// PhotonGrid::query + PhotonMap::estimateIrradiance (Photon.cpp:55-94). With
-// k_nearest > 0 and more than k photons inside the radius, the estimate uses
-// the k nearest -- the k smallest (distance, photon index) pairs, so ties at
-// the k-th distance keep the lower photon index whatever the walk order --
-// and the disc through the k-th one: sum / (pi r_k^2), the kept photons added
-// in the order the query walks them (as estimateIrradiance adds its photons).
-__device__ V3 irradiance(const GridView &v, V3 pos, int k_nearest, float *kd, int *kc) {
-    const GatherBox b = gather_box(*v.g, pos, v.radius);
-    int found = 0;
-    const V3 e = radius_sum(v, b, pos, found);
-    if (found == 0)
-        return v3(0.f);
-    if (!kd || found <= k_nearest)
-        return e / disc_area(v.radius);
-    return knn_estimate(v, b, pos, k_nearest, kd, kc);
-}
-
 constexpr int kMaxK = 64;
-
-__global__ void k_photon_gather(GridView v, const float *q, int64_t n, int k_nearest, float *out) {
-    const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    float kd[kMaxK];
-    int kc[kMaxK];
-    const V3 e = irradiance(v, v3(q[i * 3], q[i * 3 + 1], q[i * 3 + 2]), k_nearest,
-                            k_nearest > 0 ? kd : nullptr, kc);
-    out[i * 3] = e.x;
-    out[i * 3 + 1] = e.y;
-    out[i * 3 + 2] = e.z;
-}
 
 // Caustic render: per (pixel, sample), follow the camera ray through the
 // specular chain as castRay does (Integrator.cpp:143-169) and, at the first
@@ -909,13 +879,6 @@ __device__ uint32_t warp_radix_select(Walk &&walk, int lane, unsigned *bins, int
     return prefix;
 }
 
-// Candidates per warp that k_caustic_dense holds in shared memory (4 KB; at
-// 1,024 the 36 KB blocks left 6 resident per SM, at 512 the 20 KB blocks are
-// held to 7 by registers: 4% faster on the caustics frame).
-constexpr int kDenseCands = 512;
-// Collection walks k_caustic_dense tries before it selects by walking cells.
-constexpr int kDenseTries = 4;
-
 // The cells of `big` that can hold photons within t of pos: the cell box of
 // the disc of radius t, one cell wider on every side (so rounding in the cell
 // arithmetic cannot leave such a photon out), cut to `big`. Walked in the
@@ -933,173 +896,281 @@ __device__ __forceinline__ GatherBox sub_box(const GridParams &g, const GatherBo
     return b;
 }
 
-// The dense gathers of one launch, one warp each (4 per block of 128, the
-// next entry from a counter). The k-th smallest (distance, photon index)
-// pair, then the kept photons -- at or below that pair -- added in the
-// walk's order, as knn_estimate adds them; the item gets scale * E(x), the
-// product the render kernel forms for the other items.
+// The box's photons in walk order, 32 at a time: calls f(valid, s) with lane l
+// of the warp at item base + l of the list of all photons in the box's
+// columns, one column after the other. Up to 32 columns' slot ranges are read
+// at once, one per lane, and their lengths scanned, so the table reads of a
+// box overlap and short columns (a caustic's floor has about a photon per
+// column) fill whole rounds together. All lanes call f together.
+template <class F>
+__device__ __forceinline__ void walk_flat(const GridView &v, const GridParams &g,
+                                          const GatherBox &b, int lane, F &&f) {
+    const unsigned full = 0xffffffffu;
+    if (b.z0 > b.z1)
+        return;
+    const int y_first = next_slab(g.occ[1], b.y0, b.y1);
+    int cx = y_first <= b.y1 ? next_slab(g.occ[0], b.x0, b.x1) : b.x1 + 1;
+    int cy = y_first;
+    while (cx <= b.x1) {
+        int k0 = 0, cols = 0;
+        while (cols < 32 && cx <= b.x1) {
+            if (lane == cols)
+                k0 = b.z0 + cy * g.res + cx * g.res * g.res;
+            cols++;
+            cy = next_slab(g.occ[1], cy + 1, b.y1);
+            if (cy > b.y1) {
+                cy = y_first;
+                cx = next_slab(g.occ[0], cx + 1, b.x1);
+            }
+        }
+        int a = 0, len = 0;
+        if (lane < cols) {
+            a = v.first[k0];
+            len = max(0, v.first[k0 + (b.z1 - b.z0) + 1] - a);
+        }
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(full, incl, o);
+            if (lane >= o)
+                incl += y;
+        }
+        const int excl = incl - len;
+        const int total = __shfl_sync(full, incl, 31);
+        a -= excl; // slot of item j in this column: a + j
+        for (int base = 0; base < total; base += 32) {
+            const int j = base + lane;
+            int c = 0; // the last column starting at or before item j
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int e = __shfl_sync(full, excl, c + o);
+                if (e <= j)
+                    c += o;
+            }
+            f(j < total, __shfl_sync(full, a, c) + j);
+        }
+    }
+}
+
+// Candidates per warp held in shared memory (4 KB).
+constexpr int kDenseCands = 512;
+// Collection walks a warp tries before it selects by walking cells.
+constexpr int kDenseTries = 4;
+
+struct WarpScratch {
+    unsigned bins[256];
+    uint2 cand[kDenseCands]; // (distance bits, sorted slot)
+    float stage[96];
+};
+
+// Adds the powers of the lanes that keep theirs, in lane order, to the sum
+// whose channel c lane c holds (c < 3): through shared memory, so the three
+// channels' sums advance by one load and one add per photon.
+__device__ __forceinline__ void ordered_add(bool keep, const GridView &v, int s, int lane,
+                                            float *stage, float &acc) {
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+        const float4 pa = v.sorted[2 * s], pb = v.sorted[2 * s + 1];
+        float *q = stage + 3 * __popc(m & ((1u << lane) - 1u));
+        q[0] = pa.w;
+        q[1] = pb.x;
+        q[2] = pb.y;
+    }
+    __syncwarp();
+    if (lane < 3)
+        for (int n = __popc(m), q = 0; q < n; q++)
+            acc += stage[3 * q + lane];
+    __syncwarp();
+}
+
+// PhotonGrid::query + PhotonMap::estimateIrradiance (Photon.cpp:55-94) by one
+// warp, k > 0; lane c < 3 returns channel c. With more than k photons inside
+// the radius, the estimate uses the k nearest -- the k smallest
+// (distance, photon index) pairs, so ties at the k-th distance keep the lower
+// photon index whatever the walk order -- and the disc through the k-th one:
+// sum / (pi r_k^2), the kept photons added in the order the query walks them
+// (as estimateIrradiance adds its photons). `found` is the number of photons
+// inside the radius where the caller knows it to exceed k, else -1.
 //
-// Collection first: one walk over the cells that can hold photons within a
+// Collection: one walk over the cells that can hold photons within a
 // threshold t <= r stores every photon at distance <= t, in walk order, as
 // (distance bits, sorted slot) in the warp's shared memory. When at least k
 // photons lie within t, the k nearest within r are the k nearest of these
 // (any pair at or below the k-th has distance <= t), so the selection and
-// the ordered sum run over shared memory. t starts where about 3k of the
-// `found` photons inside r would lie if they were spread evenly over the
-// disc, and is widened (fewer than k within t) or narrowed (more than the
-// warp holds) for up to kDenseTries walks. Failing that the warp selects by
-// radix passes that walk the cells of the whole query box: one per byte of
-// the distance's bits (non-negative floats order as their bit patterns), one
-// more per byte of the photon index when several photons share the k-th
-// distance, and the ordered sum in a last walk, 32 photons tested per round.
-__global__ void __launch_bounds__(128) k_caustic_dense(GridView v, CausticArgs a) {
-    __shared__ unsigned bins_all[4][256];
-    __shared__ uint2 cand_all[4][kDenseCands];
-    unsigned *bins = bins_all[threadIdx.x >> 5];
-    uint2 *cand = cand_all[threadIdx.x >> 5];
-    const int64_t n = min((int64_t) *a.dense_count, a.dense_cap);
+// the ordered sum run over shared memory. t starts at r, or, once `found` is
+// known, where about 3k of the photons inside r would lie if they were spread
+// evenly over the disc, and is widened (fewer than k within t) or narrowed
+// (more than the warp holds) for up to kDenseTries walks. Failing that the
+// warp selects by radix passes that walk the cells of the whole query box:
+// one per byte of the distance's bits (non-negative floats order as their bit
+// patterns), one more per byte of the photon index when several photons share
+// the k-th distance, and the ordered sum in a last walk.
+__device__ float warp_estimate(const GridView &v, V3 pos, int k, int found, WarpScratch &w,
+                               int lane) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const float r = v.radius;
-    const int k = a.k_nearest;
     const GridParams &g = *v.g;
+    const GatherBox big = gather_box(g, pos, r);
+    auto dist_of = [&](int s) {
+        const float4 pa = v.sorted[2 * s];
+        const V3 d = v3(pa.x, pa.y, pa.z) - pos;
+        return sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+    };
+    float acc = 0.f;
+    auto guess = [&] { return r * sqrtf(fminf(1.f, 3.f * (float) k / (float) found)); };
+    float t = found < 0 ? r : guess();
+    int count = -1; // photons collected in shared memory (-1: none usable)
+    for (int attempt = 0; attempt < kDenseTries; attempt++) {
+        const GatherBox b = found < 0 ? big : sub_box(g, big, pos, t);
+        int c = 0;
+        walk_flat(v, g, b, lane, [&](bool valid, int s) {
+            float dist = 0.f;
+            bool take = false;
+            if (valid) {
+                dist = dist_of(s);
+                take = dist <= t;
+            }
+            const unsigned m = __ballot_sync(full, take);
+            const int at = c + __popc(m & ((1u << lane) - 1u));
+            if (take && at < kDenseCands)
+                w.cand[at] = make_uint2(__float_as_uint(dist), (unsigned) s);
+            c += __popc(m);
+        });
+        __syncwarp();
+        if (found < 0) { // the walk at t = r: every photon inside
+            found = c;
+            if (c <= k) { // the fixed-radius estimate (k <= kMaxK fit)
+                for (int base = 0; base < c; base += 32) {
+                    const int q = base + lane;
+                    ordered_add(q < c, v, q < c ? (int) w.cand[q].y : 0, lane, w.stage, acc);
+                }
+                return acc / disc_area(r);
+            }
+            if (c > kDenseCands) {
+                t = guess();
+                continue;
+            }
+        }
+        if (c >= k && c <= kDenseCands) {
+            count = c;
+            break;
+        }
+        if (c < k) {
+            if (t >= r)
+                break; // cannot happen while found > k
+            t = fminf(r, t * sqrtf(2.f * (float) k / (float) max(c, 1)));
+        } else {
+            t = t * sqrtf(0.5f * (float) kDenseCands / (float) c);
+        }
+    }
+    int want = k, equal = 0;
+    uint32_t dk;
+    int ik = 0x7fffffff;
+    if (count >= 0) {
+        auto walk = [&](auto &&f) {
+            for (int q = lane; q < count; q += 32)
+                f(q);
+        };
+        dk = warp_radix_select(walk, lane, w.bins, want, &equal, [&](int q, uint32_t &key) {
+            key = w.cand[q].x;
+            return true;
+        });
+        // of the photons at the k-th distance, keep the lowest `want` indices
+        if (equal > want) {
+            int eq2 = 0;
+            ik = (int) warp_radix_select(walk, lane, w.bins, want, &eq2,
+                                         [&](int q, uint32_t &key) {
+                                             key = (uint32_t) v.order[w.cand[q].y];
+                                             return w.cand[q].x == dk;
+                                         });
+        }
+        for (int base = 0; base < count; base += 32) {
+            const int q = base + lane;
+            const uint2 cq = q < count ? w.cand[q] : make_uint2(0xffffffffu, 0u);
+            const bool keep = cq.x < dk || (cq.x == dk && v.order[cq.y] <= ik);
+            ordered_add(keep, v, (int) cq.y, lane, w.stage, acc);
+        }
+    } else {
+        auto walk = [&](auto &&f) { walk_cells_warp(v, big, lane, f); };
+        dk = warp_radix_select(walk, lane, w.bins, want, &equal, [&](int s, uint32_t &key) {
+            const float dist = dist_of(s);
+            key = __float_as_uint(dist);
+            return dist <= r;
+        });
+        if (equal > want) {
+            int eq2 = 0;
+            ik = (int) warp_radix_select(walk, lane, w.bins, want, &eq2,
+                                         [&](int s, uint32_t &key) {
+                                             key = (uint32_t) v.order[s];
+                                             return __float_as_uint(dist_of(s)) == dk;
+                                         });
+        }
+        walk_flat(v, g, big, lane, [&](bool valid, int s) {
+            bool keep = false;
+            if (valid) {
+                const uint32_t db = __float_as_uint(dist_of(s));
+                keep = db < dk || (db == dk && v.order[s] <= ik);
+            }
+            ordered_add(keep, v, s, lane, w.stage, acc);
+        });
+    }
+    return acc / disc_area(__uint_as_float(dk));
+}
+
+// PhotonMap::estimateIrradiance of n points, a thread each: a sum in the
+// walk's order, which a warp per point only adds overhead to (60,013 points,
+// 40,000 photons: 99 us, 138 a warp each).
+__global__ void k_photon_gather(GridView v, const float *q, int64_t n, float *out) {
+    const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const V3 pos = v3(q[i * 3], q[i * 3 + 1], q[i * 3 + 2]);
+    int found = 0;
+    V3 e = radius_sum(v, gather_box(*v.g, pos, v.radius), pos, found);
+    e = found == 0 ? v3(0.f) : e / disc_area(v.radius);
+    out[i * 3] = e.x;
+    out[i * 3 + 1] = e.y;
+    out[i * 3 + 2] = e.z;
+}
+
+// The k-nearest estimate of n points, a warp each: with a thread each a warp
+// waited on its densest point, whose heap of k pairs lived in local memory
+// (60,013 points, 40,000 photons, radius 0.02: k = 64 606 -> 155 us, k = 8 476
+// -> 177; 2,000 points, 3,000 photons, k = 64 48 -> 40).
+__global__ void __launch_bounds__(128) k_photon_gather_knn(GridView v, const float *q, int64_t n,
+                                                           int k_nearest, float *out) {
+    __shared__ WarpScratch scratch[4];
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = ((int64_t) gridDim.x * blockDim.x) >> 5;
+    for (int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const V3 pos = v3(q[i * 3], q[i * 3 + 1], q[i * 3 + 2]);
+        const float e = warp_estimate(v, pos, k_nearest, -1, scratch[threadIdx.x >> 5], lane);
+        if (lane < 3)
+            out[i * 3 + lane] = e;
+    }
+}
+
+// The dense gathers of one launch of the caustic render, one warp each (4 per
+// block of 128, the next entry from a counter); the item gets scale * E(x),
+// the product the render kernel forms for the other items.
+__global__ void __launch_bounds__(128) k_caustic_dense(GridView v, CausticArgs a) {
+    __shared__ WarpScratch scratch[4];
+    const int64_t n = min((int64_t) *a.dense_count, a.dense_cap);
+    const int lane = threadIdx.x & 31;
     for (;;) {
         unsigned long long e = 0;
         if (lane == 0)
             e = atomicAdd(a.dense_next, 1ull);
-        e = __shfl_sync(full, e, 0);
+        e = __shfl_sync(0xffffffffu, e, 0);
         if ((int64_t) e >= n)
             break;
         const float4 p = a.dense[2 * e], sc = a.dense[2 * e + 1];
-        const V3 pos = v3(p.x, p.y, p.z);
-        const int found = __float_as_int(sc.w); // photons inside r (> k)
-        const GatherBox big = gather_box(g, pos, r);
-        auto dist_of = [&](int s) {
-            const float4 pa = v.sorted[2 * s];
-            const V3 d = v3(pa.x, pa.y, pa.z) - pos;
-            return sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
-        };
-        float t = r * sqrtf(fminf(1.f, 3.f * (float) k / (float) found));
-        int count = -1; // photons collected in shared memory (-1: none usable)
-        for (int attempt = 0; attempt < kDenseTries; attempt++) {
-            const GatherBox b = sub_box(g, big, pos, t);
-            int c = 0;
-            walk_columns(v, g, b.x0, b.x1, b.y0, b.y1, b.z0, b.z1, [&](int a0, int e0) {
-                for (int base = a0; base < e0; base += 32) {
-                    const int s = base + lane;
-                    float dist = 0.f;
-                    bool take = false;
-                    if (s < e0) {
-                        dist = dist_of(s);
-                        take = dist <= t;
-                    }
-                    const unsigned m = __ballot_sync(full, take);
-                    const int at = c + __popc(m & ((1u << lane) - 1u));
-                    if (take && at < kDenseCands)
-                        cand[at] = make_uint2(__float_as_uint(dist), (unsigned) s);
-                    c += __popc(m);
-                }
-            });
-            __syncwarp();
-            if (c >= k && c <= kDenseCands) {
-                count = c;
-                break;
-            }
-            if (c < k) {
-                if (t >= r)
-                    break; // cannot happen while found > k
-                t = fminf(r, t * sqrtf(2.f * (float) k / (float) max(c, 1)));
-            } else {
-                t = t * sqrtf(0.5f * (float) kDenseCands / (float) c);
-            }
-        }
-        int want = k, equal = 0;
-        uint32_t dk;
-        int ik = 0x7fffffff;
-        V3 ek = v3(0.f);
-        if (count >= 0) {
-            auto walk = [&](auto &&f) {
-                for (int q = lane; q < count; q += 32)
-                    f(q);
-            };
-            dk = warp_radix_select(walk, lane, bins, want, &equal, [&](int q, uint32_t &key) {
-                key = cand[q].x;
-                return true;
-            });
-            // of the photons at the k-th distance, keep the lowest `want` indices
-            if (equal > want) {
-                int eq2 = 0;
-                ik = (int) warp_radix_select(walk, lane, bins, want, &eq2,
-                                             [&](int q, uint32_t &key) {
-                                                 key = (uint32_t) v.order[cand[q].y];
-                                                 return cand[q].x == dk;
-                                             });
-            }
-            // the ordered sum of the kept powers (lane 0 holds it)
-            for (int base = 0; base < count; base += 32) {
-                const int q = base + lane;
-                bool keep = false;
-                V3 pw = v3(0.f);
-                if (q < count) {
-                    const uint2 cq = cand[q];
-                    keep = cq.x < dk || (cq.x == dk && v.order[cq.y] <= ik);
-                    if (keep) {
-                        const float4 pa = v.sorted[2 * cq.y];
-                        const float4 pb = v.sorted[2 * cq.y + 1];
-                        pw = v3(pa.w, pb.x, pb.y);
-                    }
-                }
-                for (unsigned km = __ballot_sync(full, keep); km; km &= km - 1) {
-                    const int l = __ffs(km) - 1;
-                    const V3 w = v3(__shfl_sync(full, pw.x, l), __shfl_sync(full, pw.y, l),
-                                    __shfl_sync(full, pw.z, l));
-                    ek = ek + w;
-                }
-            }
-        } else {
-            const GatherBox &b = big;
-            auto walk = [&](auto &&f) { walk_cells_warp(v, b, lane, f); };
-            dk = warp_radix_select(walk, lane, bins, want, &equal, [&](int s, uint32_t &key) {
-                const float dist = dist_of(s);
-                key = __float_as_uint(dist);
-                return dist <= r;
-            });
-            if (equal > want) {
-                int eq2 = 0;
-                ik = (int) warp_radix_select(walk, lane, bins, want, &eq2,
-                                             [&](int s, uint32_t &key) {
-                                                 key = (uint32_t) v.order[s];
-                                                 return __float_as_uint(dist_of(s)) == dk;
-                                             });
-            }
-            const float rk = __uint_as_float(dk);
-            walk_columns(v, g, b.x0, b.x1, b.y0, b.y1, b.z0, b.z1, [&](int a0, int e0) {
-                for (int base = a0; base < e0; base += 32) {
-                    const int s = base + lane;
-                    bool keep = false;
-                    V3 pw = v3(0.f);
-                    if (s < e0) {
-                        const float dist = dist_of(s);
-                        keep = dist < rk || (dist == rk && v.order[s] <= ik);
-                        if (keep) {
-                            const float4 pa = v.sorted[2 * s];
-                            const float4 pb = v.sorted[2 * s + 1];
-                            pw = v3(pa.w, pb.x, pb.y);
-                        }
-                    }
-                    for (unsigned km = __ballot_sync(full, keep); km; km &= km - 1) {
-                        const int l = __ffs(km) - 1;
-                        const V3 w = v3(__shfl_sync(full, pw.x, l), __shfl_sync(full, pw.y, l),
-                                        __shfl_sync(full, pw.z, l));
-                        ek = ek + w;
-                    }
-                }
-            });
-        }
-        if (lane == 0) {
-            const V3 c = v3(sc.x, sc.y, sc.z) * (ek / disc_area(__uint_as_float(dk)));
-            a.samples[__float_as_int(p.w)] = make_float4(c.x, c.y, c.z, 0.f);
-        }
+        const float x = warp_estimate(v, v3(p.x, p.y, p.z), a.k_nearest, __float_as_int(sc.w),
+                                      scratch[threadIdx.x >> 5], lane);
+        const float scale = lane == 0 ? sc.x : (lane == 1 ? sc.y : sc.z);
+        if (lane < 4)
+            reinterpret_cast<float *>(a.samples + __float_as_int(p.w))[lane] =
+                lane < 3 ? scale * x : 0.f;
         __syncwarp();
     }
 }
@@ -1585,8 +1656,18 @@ int prr_photon_gather(const prr_photon_map *pmap, const float *points, int64_t n
         PRR_CUDA_TRY(cudaMemsetAsync(out_rgb, 0, (size_t) n * 3 * sizeof(float), st));
         return PRR_OK;
     }
-    k_photon_gather<<<(unsigned) ((n + 127) / 128), 128, 0, st>>>(view(pm), points, n, k_nearest,
-                                                                   out_rgb);
+    if (k_nearest == 0) {
+        k_photon_gather<<<(unsigned) ((n + 127) / 128), 128, 0, st>>>(view(pm), points, n,
+                                                                       out_rgb);
+    } else {
+        // four rounds of resident blocks: dense and sparse points even out
+        int bps = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_photon_gather_knn, 128, 0);
+        const int64_t grid = std::min<int64_t>(
+            (n + 3) / 4, (int64_t) device_sm_count() * std::max(1, bps) * 4);
+        k_photon_gather_knn<<<(unsigned) grid, 128, 0, st>>>(view(pm), points, n, k_nearest,
+                                                             out_rgb);
+    }
     pm.launches++;
     PRR_CUDA_TRY(cudaGetLastError());
     return PRR_OK;

@@ -402,3 +402,21 @@ def test_gather_outside_the_grid(cuda):
                 q[:, (axis + 1) % 3] = np.linspace(-0.02, 0.02, 64)
                 q[:, axis] = far
                 assert not pm.gather(q, k_nearest=k).cpu().numpy().any(), (k, axis, far)
+
+
+@pytest.mark.parametrize("n, k, radius", [(1, 1, 0.02), (40, 8, 0.3), (3000, 64, 0.05),
+                                          (30000, 64, 0.3), (30000, 1, 0.3), (5000, 63, 2.0)])
+def test_knn_gather_against_restatement(port, cuda, n, k, radius):
+    """Warp-wide k-nearest gathers bit for bit against the C restatement: few
+    photons, every photon inside (more than a warp holds in shared memory, so
+    the threshold walks and the selection over cells run), columns beyond one
+    round of 32, and coinciding photons."""
+    rec, q = random_photons(n, n + k)
+    if n > 100:
+        rec[n // 2:n // 2 + 40, :3] = rec[:40, :3]
+        rec[100:n // 4, :3] = rec[99, :3]  # a pile larger than the candidate store
+        q[:64] = rec[99, :3]
+    q = q[:400]
+    got = prr.PhotonMap().set(rec).build(radius).gather(q, k_nearest=k).cpu().numpy()
+    want, inside = port.photon_estimate_knn(rec, radius, q, k)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
