@@ -669,79 +669,78 @@ __global__ void __launch_bounds__(128, 8) k_wf_surface(DevScene S0, Wf w, int it
                 const V3 cd = ld3(w.rd, p);
                 const V3 hp = in.p;
                 const V3 sn = dot(cd, in.n) < 0.f ? in.n : -in.n;
-                const Shading sd = build_shading(S, m, sn, in.a);
+                const Shading sd = build_shading<kCastOutline>(S, m, sn, in.a);
                 const V3 wo = -cd;
-                const bool indirect = it > 0;
-                // NEE towards emitters: the contribution is formed now and
-                // added by the shadow stage if the light is visible
-                float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), ld = lo, lc = lo;
-                if (S.total_emit_area > 0.f) {
-                    const LightPoint lp = sample_light(S, rng);
-                    const float pdf_area = 1.0f / S.total_emit_area;
-                    const V3 to = lp.p - hp;
-                    const float dist2 = dot(to, to);
-                    const float dist = sqrtf(dist2);
-                    const V3 wi = to / dist;
-                    const float cos_l = smax(0.f, dot(-wi, normalized(lp.n)));
-                    if (cos_l > 0.f) {
-                        const float pdf_sa = pdf_area * dist2 / cos_l;
-                        V3 f;
-                        float bp;
+                const float indirect = it > 0 ? 1.f : 0.f;
+                // The three directions that leave the hit: towards an emitter,
+                // towards the environment, and the BSDF sample. One loop, so the
+                // BSDF evaluation stands once in the code. The first two
+                // contributions are formed now and added by the shadow stage if
+                // their light is visible.
+                V3 wi = v3(0.f), f = v3(0.f);
+                float bp = 0.f;
+#pragma unroll 1
+                for (int d = 0; d < 3; d++) {
+                    float pdf = 0.f, tmax = kInf;
+                    V3 em = v3(0.f);
+                    bool ok = false;
+                    if (d == 0) {
+                        if (S.total_emit_area > 0.f) {
+                            const LightPoint lp = sample_light(S, rng);
+                            const float pdf_area = 1.0f / S.total_emit_area;
+                            const V3 to = lp.p - hp;
+                            const float dist2 = dot(to, to);
+                            const float dist = sqrtf(dist2);
+                            wi = to / dist;
+                            const float cos_l = smax(0.f, dot(-wi, normalized(lp.n)));
+                            ok = cos_l > 0.f;
+                            if (ok) {
+                                pdf = pdf_area * dist2 / cos_l;
+                                tmax = dist - 2.f * PRR_EPS;
+                                const DevMaterial &lm = S.materials[lp.material];
+                                em = v3(lm.emission[0], lm.emission[1], lm.emission[2]);
+                            }
+                        }
+                    } else if (d == 1) {
+                        if (S.env.loaded) {
+                            wi = env_importance(S.env, rng, pdf);
+                            ok = !(pdf < 1e-6f);
+                            if (ok)
+                                em = env_lookup(S.env, wi);
+                        }
+                    } else {
+                        ok = m.kind == kMatDiffuse && diffuse_direction(m, sd, wo, rng, wi);
+                    }
+                    f = v3(0.f);
+                    bp = 0.f;
+                    if (ok)
                         mat_eval_pdf(m, sd, wi, wo, &f, &bp);
-                        const DevMaterial &lm = S.materials[lp.material];
-                        V3 c = mis(pdf_sa, bp) * v3(lm.emission[0], lm.emission[1], lm.emission[2]) *
-                               f / pdf_sa;
+                    if (d < 2 && ok) {
+                        V3 c = mis(pdf, bp) * em * f / (d == 0 ? pdf : pdf + 1e-6f);
                         c = beta * c;
                         if (!(c.x == 0.f && c.y == 0.f && c.z == 0.f)) {
                             const V3 o = hp + wi * PRR_EPS;
-                            lo = make_float4(o.x, o.y, o.z, dist - 2.f * PRR_EPS);
-                            ld = make_float4(wi.x, wi.y, wi.z, 1.f);
-                            lc = make_float4(c.x, c.y, c.z, indirect ? 1.f : 0.f);
-                            shadow = true;
+                            (d == 0 ? w.slo : w.seo)[p] = make_float4(o.x, o.y, o.z, tmax);
+                            (d == 0 ? w.sld : w.sed)[p] = make_float4(wi.x, wi.y, wi.z, 1.f);
+                            (d == 0 ? w.slc : w.sec)[p] = make_float4(c.x, c.y, c.z, indirect);
+                            if (d == 0)
+                                jl = true;
+                            else
+                                je = true;
                         }
                     }
                 }
-                float4 eo = make_float4(0.f, 0.f, 0.f, 0.f), ed = eo, ec = eo;
-                if (S.env.loaded) {
-                    float pdf;
-                    const V3 dir = env_importance(S.env, rng, pdf);
-                    if (!(pdf < 1e-6f)) {
-                        const V3 em = env_lookup(S.env, dir);
-                        V3 f;
-                        float bp;
-                        mat_eval_pdf(m, sd, dir, wo, &f, &bp);
-                        V3 c = mis(pdf, bp) * em * f / (pdf + 1e-6f);
-                        c = beta * c;
-                        if (!(c.x == 0.f && c.y == 0.f && c.z == 0.f)) {
-                            const V3 o = hp + dir * PRR_EPS;
-                            eo = make_float4(o.x, o.y, o.z, kInf);
-                            ed = make_float4(dir.x, dir.y, dir.z, 1.f);
-                            ec = make_float4(c.x, c.y, c.z, indirect ? 1.f : 0.f);
-                            shadow = true;
-                        }
-                    }
-                }
-                if (shadow) {
-                    // a ray's direction carries its flag (w = 0: none); its
-                    // origin and contribution are read only when set
-                    w.sld[p] = ld;
-                    w.sed[p] = ed;
-                    if (ld.w != 0.f) {
-                        w.slo[p] = lo;
-                        w.slc[p] = lc;
-                    }
-                    if (ed.w != 0.f) {
-                        w.seo[p] = eo;
-                        w.sec[p] = ec;
-                    }
-                    jl = ld.w != 0.f;
-                    je = ed.w != 0.f;
-                }
+                // a ray's direction carries its flag (w = 0: none); its origin and
+                // contribution are read only when set
+                shadow = jl || je;
+                if (shadow && !jl)
+                    w.sld[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (shadow && !je)
+                    w.sed[p] = make_float4(0.f, 0.f, 0.f, 0.f);
                 BSDFSample bs;
-                if (m.kind == kMatDiffuse)
-                    bs = diffuse_sample(m, sd, wo, rng);
-                else
-                    bs.pdf = 0.f;
+                bs.wi = wi;
+                bs.pdf = bp;
+                bs.f = bp > 1e-6f ? f : v3(0.f); // DiffuseMaterial::sample
                 if (bs.pdf < 1e-6f) {
                     if (shadow) {
                         st3(w.L, p, L);

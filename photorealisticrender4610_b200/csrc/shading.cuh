@@ -170,16 +170,13 @@ __device__ __forceinline__ V3 f_schlick(float wodoth, V3 f0) { // :143-146
     const float t = powf(smax(0.f, 1.f - wodoth), 5.f);
     return f0 + (v3(1.f) - f0) * t;
 }
-// sampleGGX_VNDF (BRDFUtils.hpp:163-181), Heitz 2018
-__device__ __forceinline__ V3 sample_vndf(V3 wo, float alpha, float u1, float u2) {
+// sampleGGX_VNDF (BRDFUtils.hpp:163-181), Heitz 2018, from the disc point
+// t1 = sqrt(u1) cos(2 pi u2), t2 = sqrt(u1) sin(2 pi u2)
+__device__ __forceinline__ V3 sample_vndf(V3 wo, float alpha, float t1, float t2) {
     const V3 vh = normalize(v3(alpha * wo.x, alpha * wo.y, wo.z));
     const float lensq = vh.x * vh.x + vh.y * vh.y;
     const V3 T1 = lensq > 0.f ? v3(-vh.y, vh.x, 0.f) / sqrtf(lensq) : v3(1.f, 0.f, 0.f);
     const V3 T2 = cross(vh, T1);
-    const float r = sqrtf(u1);
-    const float phi = 2.f * PRR_PI * u2;
-    const float t1 = r * cosf(phi);
-    float t2 = r * sinf(phi);
     const float s = 0.5f * (1.f + vh.z);
     t2 = (1.f - s) * sqrtf(1.f - t1 * t1) + s * t2;
     const V3 nh = t1 * T1 + t2 * T2 + sqrtf(smax(0.f, 1.f - t1 * t1 - t2 * t2)) * vh;
@@ -445,44 +442,52 @@ __device__ __forceinline__ void mat_eval_pdf(const DevMaterial &m, const Shading
     }
 }
 
-// DiffuseMaterial::sample (Material.cpp:28-61): draws three numbers once the
-// outgoing direction is above the surface.
-__device__ __forceinline__ BSDFSample diffuse_sample(const DevMaterial &m, const Shading &sd, V3 wo,
-                                                     Rng &rng) {
-    BSDFSample s;
-    s.wi = v3(0.f);
-    s.f = v3(0.f);
-    s.pdf = 0.f;
+// The direction of DiffuseMaterial::sample (Material.cpp:28-61): draws three
+// numbers once wo is above the surface; false when the sample has no direction
+// (its pdf is 0). The sample's f and pdf are those of diffuse_eval_pdf.
+__device__ __forceinline__ bool diffuse_direction(const DevMaterial &m, const Shading &sd, V3 wo,
+                                                  Rng &rng, V3 &wi) {
     const float alpha = sd.roughness * sd.roughness;
     const V3 F0 = compute_f0(m.ior, sd.metallic, sd.base);
     const float F0max = max3(F0);
     const float sw = sd.metallic + (1.f - sd.metallic) * F0max;
     const V3 wol = to_local(sd.f, wo);
     if (wol.z <= 0.f)
-        return s;
+        return false;
     const float u0 = rng.next();
     const float u1 = rng.next();
     const float u2 = rng.next();
+    // both lobes start from the same point of the unit disc
+    const float r = sqrtf(u1);
+    const float phi = 2.f * PRR_PI * u2;
+    const float dx = r * cosf(phi), dy = r * sinf(phi);
     V3 wil;
     if (u0 < sw) {
-        const V3 H = sample_vndf(wol, alpha, u1, u2);
+        const V3 H = sample_vndf(wol, alpha, dx, dy);
         if (dot(H, H) < 1e-8f)
-            return s;
+            return false;
         wil = reflect(wol, H);
     } else {
-        const float r = sqrtf(u1);
-        const float phi = 2.f * PRR_PI * u2;
-        wil = v3(r * cosf(phi), r * sinf(phi), sqrtf(smax(0.f, 1.f - u1)));
+        wil = v3(dx, dy, sqrtf(smax(0.f, 1.f - u1)));
     }
     if (wil.z <= 0.f)
+        return false;
+    wi = to_world(sd.f, wil);
+    return true;
+}
+
+// DiffuseMaterial::sample (Material.cpp:28-61).
+__device__ __forceinline__ BSDFSample diffuse_sample(const DevMaterial &m, const Shading &sd, V3 wo,
+                                                     Rng &rng) {
+    BSDFSample s;
+    s.wi = v3(0.f);
+    s.f = v3(0.f);
+    s.pdf = 0.f;
+    if (!diffuse_direction(m, sd, wo, rng, s.wi))
         return s;
-    const V3 wi = to_world(sd.f, wil);
-    s.wi = wi;
-    float pdf;
-    diffuse_eval_pdf(m, sd, wi, wo, nullptr, &pdf);
-    s.pdf = pdf;
-    if (pdf > 1e-6f)
-        diffuse_eval_pdf(m, sd, wi, wo, &s.f, nullptr);
+    diffuse_eval_pdf(m, sd, s.wi, wo, &s.f, &s.pdf);
+    if (!(s.pdf > 1e-6f))
+        s.f = v3(0.f);
     return s;
 }
 
