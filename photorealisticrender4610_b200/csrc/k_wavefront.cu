@@ -43,7 +43,7 @@ enum : int {
 struct WfReq {
     const DevScene *scene;
     DevCamera camera;
-    int W, x0, y0, ww, npix;     // image width, window, window pixels
+    int W, x0, y0, ww, wh, npix; // image width, window, window pixels
     int s0, nspp;                // samples [s0, s0 + nspp) of every window pixel
     int max_depth;
     float clamp;
@@ -55,7 +55,7 @@ struct WfReq {
 
 struct Wf {
     int P, npix, spp_pass;
-    int W, x0, y0, ww;
+    int W, x0, y0, ww, wh;
     int max_depth;
     float clamp;
     uint64_t seed;
@@ -75,7 +75,7 @@ struct Wf {
     float4 *slo, *sld, *slc; // light shadow ray: origin+tmax, dir+valid, contribution
     float4 *seo, *sed, *sec; // env shadow ray
     float4 *result;      // final L per path
-    float3 *film;        // per pixel running sum
+    float3 *film;        // per pixel running sum, in path order (tile_pixel)
     // queues
     int *qray[2], *qmiss, *qdelta, *qsurf, *qshadow, *qjob;
     uint8_t *vis;        // per shadow job (2 per path): 1 when nothing occludes
@@ -238,6 +238,22 @@ __device__ __forceinline__ void finish(const Wf &w, int p, V3 L) {
     w.result[p] = make_float4(L.x, L.y, L.z, 0.f);
 }
 
+// Window pixel q in path order: tiles of 8x4 pixels (narrower at the right
+// edge, lower at the bottom), row by row of tiles, so a warp's 32 paths start
+// in a small square instead of a long row and stay closer together (1% on
+// every frame tried: museum-like 480x270, adaptive up to 256 spp, 44.0 -> 43.5
+// ms).
+__device__ __forceinline__ void tile_pixel(int q, int ww, int wh, int &x, int &y) {
+    const int strip = q / (4 * ww);
+    int r = q - strip * 4 * ww;
+    const int h = min(4, wh - strip * 4);
+    const int tx = r / (8 * h);
+    r -= tx * 8 * h;
+    const int tw = min(8, ww - tx * 8);
+    y = strip * 4 + r / tw;
+    x = tx * 8 + r % tw;
+}
+
 // ---- generate: camera rays for every (pixel, sample) of the pass
 template <bool MULTI> __global__ void k_wf_generate(DevScene S, Wf w) {
     const int base = MULTI ? 0 : *w.pass_base;
@@ -257,8 +273,9 @@ template <bool MULTI> __global__ void k_wf_generate(DevScene S, Wf w) {
             const WfReq &R = w.reqs[r];
             const int64_t o = p - R.path_base;
             const int q = (int) (o % R.npix);
-            i = R.x0 + q % R.ww;
-            j = R.y0 + q / R.ww;
+            tile_pixel(q, R.ww, R.wh, i, j);
+            i += R.x0;
+            j += R.y0;
             m = (uint32_t) i + (uint32_t) j * (uint32_t) R.W;
             sample = (uint32_t) (R.s0 + o / R.npix);
             seed = R.seed;
@@ -266,8 +283,9 @@ template <bool MULTI> __global__ void k_wf_generate(DevScene S, Wf w) {
             w.req[p] = r;
         } else {
             const int q = w.adaptive ? w.act[p % nq] : p % w.npix;
-            i = w.x0 + q % w.ww;
-            j = w.y0 + q / w.ww;
+            tile_pixel(q, w.ww, w.wh, i, j);
+            i += w.x0;
+            j += w.y0;
             m = (uint32_t) i + (uint32_t) j * (uint32_t) w.W;
             sample = (uint32_t) (w.sample_offset + base + p / nq);
             seed = w.seed;
@@ -1156,18 +1174,21 @@ __global__ void k_wf_adaptive_init(Wf w) {
 }
 
 // mean = sum / n per pixel (Renderer.cpp:98-99)
-__global__ void k_wf_resolve_adaptive(const float3 *film, const float4 *wel0, int npix, float *out,
-                                      int32_t *spp) {
+__global__ void k_wf_resolve_adaptive(const float3 *film, const float4 *wel0, int npix, int ww,
+                                      int wh, float *out, int32_t *spp) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= npix)
         return;
     const float3 f = film[q];
     const int n = (int) wel0[q].x;
-    out[(size_t) q * 3 + 0] = f.x / (float) n;
-    out[(size_t) q * 3 + 1] = f.y / (float) n;
-    out[(size_t) q * 3 + 2] = f.z / (float) n;
+    int x, y;
+    tile_pixel(q, ww, wh, x, y);
+    const size_t o = (size_t) y * ww + x;
+    out[o * 3 + 0] = f.x / (float) n;
+    out[o * 3 + 1] = f.y / (float) n;
+    out[o * 3 + 2] = f.z / (float) n;
     if (spp)
-        spp[q] = n;
+        spp[o] = n;
 }
 
 // ---- server step film: every request's window pixels take this step's
@@ -1179,7 +1200,10 @@ __global__ void k_wf_film_multi(Wf w, int64_t total_pixels) {
         const int r = find_req(w.reqs, w.n_reqs, t, true);
         const WfReq &R = w.reqs[r];
         const int q = (int) (t - R.pix_base);
-        float3 f = R.film[q];
+        int x, y;
+        tile_pixel(q, R.ww, R.wh, x, y);
+        float3 &film = R.film[(size_t) y * R.ww + x]; // row order
+        float3 f = film;
         for (int s = 0; s < R.nspp; s++) {
             const float4 v = w.result[R.path_base + (int64_t) s * R.npix + q];
             if (!(isnan(v.x) || isnan(v.y) || isnan(v.z))) {
@@ -1188,7 +1212,7 @@ __global__ void k_wf_film_multi(Wf w, int64_t total_pixels) {
                 f.z += v.z;
             }
         }
-        R.film[q] = f;
+        film = f;
     }
 }
 
@@ -1211,16 +1235,20 @@ __global__ void k_wf_film(Wf w) {
         *w.pass_base += w.spp_pass;
 }
 
-__global__ void k_wf_resolve(const float3 *film, int npix, int n, float *out, int32_t *spp) {
+__global__ void k_wf_resolve(const float3 *film, int npix, int ww, int wh, int n, float *out,
+                             int32_t *spp) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= npix)
         return;
     const float3 f = film[q];
-    out[(size_t) q * 3 + 0] = f.x / (float) n;
-    out[(size_t) q * 3 + 1] = f.y / (float) n;
-    out[(size_t) q * 3 + 2] = f.z / (float) n;
+    int x, y;
+    tile_pixel(q, ww, wh, x, y);
+    const size_t o = (size_t) y * ww + x;
+    out[o * 3 + 0] = f.x / (float) n;
+    out[o * 3 + 1] = f.y / (float) n;
+    out[o * 3 + 2] = f.z / (float) n;
     if (spp)
-        spp[q] = n;
+        spp[o] = n;
 }
 
 __global__ void k_wf_rays_out(const unsigned *cnt, unsigned long long *out) {
@@ -1468,8 +1496,8 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.x0 = rs.x0;
     w.y0 = rs.y0;
     w.ww = rs.x1 - rs.x0;
-    const int wh = rs.y1 - rs.y0;
-    w.npix = w.ww * wh;
+    w.wh = rs.y1 - rs.y0;
+    w.npix = w.ww * w.wh;
     w.max_depth = rs.max_depth;
     w.clamp = rs.indirect_clamp;
     w.seed = rs.seed;
@@ -1542,7 +1570,8 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     key = mix64(key ^ ((uint64_t) w.adaptive << 7) ^ ((uint64_t) w.min_spp << 24) ^
                 ((uint64_t) float_bits(w.threshold) << 28) ^ (uint64_t) w.max_spp);
     key = mix64(key ^ ((uint64_t) (uint32_t) w.x0 << 32 | (uint32_t) w.y0) ^
-                ((uint64_t) (uint32_t) w.ww << 16) ^ rs.seed ^ ((uint64_t) rs.sample_offset << 40) ^
+                ((uint64_t) (uint32_t) w.ww << 16) ^ (uint64_t) (uint32_t) w.wh ^ rs.seed ^
+                ((uint64_t) rs.sample_offset << 40) ^
                 (uint64_t) float_bits(w.clamp));
     if (!s.wf_plan)
         s.wf_plan = std::make_shared<WavefrontPlan>();
@@ -1580,10 +1609,10 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
                 return rc;
     }
     if (w.adaptive)
-        k_wf_resolve_adaptive<<<(w.npix + 255) / 256, 256, 0, st>>>(w.film, w.wel0, w.npix,
+        k_wf_resolve_adaptive<<<(w.npix + 255) / 256, 256, 0, st>>>(w.film, w.wel0, w.npix, w.ww, w.wh,
                                                                     out_rgb, out_spp);
     else
-        k_wf_resolve<<<(w.npix + 255) / 256, 256, 0, st>>>(w.film, w.npix, rs.max_spp, out_rgb,
+        k_wf_resolve<<<(w.npix + 255) / 256, 256, 0, st>>>(w.film, w.npix, w.ww, w.wh, rs.max_spp, out_rgb,
                                                             out_spp);
     PRR_CUDA_TRY(cudaGetLastError());
     if (out_rays) {
@@ -1637,6 +1666,7 @@ int wavefront_step_multi(WfMultiState &ms, const WfStepReq *reqs, int n,
         t.x0 = q.x0;
         t.y0 = q.y0;
         t.ww = q.ww;
+        t.wh = q.wh;
         t.npix = q.ww * q.wh;
         t.s0 = q.s0;
         t.nspp = q.nspp;
