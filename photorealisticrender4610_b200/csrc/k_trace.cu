@@ -139,8 +139,10 @@ __device__ __forceinline__ void trace_rays(Body &b, uint32_t n, const TraceCfg &
 // One ray of a closest-hit query on one mesh. A step is one four-wide node
 // (the slab tests of BVH.cpp:368-397 at two levels), or one triangle of the
 // current leaf (BVH.cpp:343-357), followed when needed by the pop of
-// BVH.cpp:400-407.
-struct MeshClosest {
+// BVH.cpp:400-407. FEW, here and below: the form for small batches, which
+// tests a leaf's triangles in one step, their loads under way together, and
+// asks for the children it pushes.
+template <bool FEW> struct MeshClosest {
     const MeshArgs &a;
     const StackCol<uint2> col;
     uint32_t idx = 0;
@@ -182,18 +184,38 @@ struct MeshClosest {
 
     __device__ __forceinline__ bool step() {
         if (ntri > 0) {
-            const TriV T = load_tri(a.tris, a.e2z, tri, a.B);
-            float t, u, v;
-            if (tri_hit(T, r, t, u, v) && t < best) {
-                best = t;
-                hit = (int) tri;
+            if constexpr (FEW) {
+                // the whole leaf, its loads under way together
+                TriV T[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    if (k < ntri)
+                        T[k] = load_tri(a.tris, a.e2z, tri + k, a.B);
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    if (k < ntri) {
+                        float t, u, v;
+                        if (tri_hit(T[k], r, t, u, v) && t < best) {
+                            best = t;
+                            hit = (int) (tri + k);
+                        }
+                    }
+            } else {
+                const TriV T = load_tri(a.tris, a.e2z, tri, a.B);
+                float t, u, v;
+                if (tri_hit(T, r, t, u, v) && t < best) {
+                    best = t;
+                    hit = (int) tri;
+                }
+                tri++;
+                ntri--;
+                if (ntri > 0)
+                    return false;
             }
-            tri++;
-            ntri--;
-            if (ntri > 0)
-                return false;
         } else {
             const QuadOrder q = quad_order(load_quad(a.nodes, ref, a.B), p);
+            if constexpr (FEW)
+                q.rest(best, [&](uint32_t x, float) { fetch_child(a.nodes, a.tris, x); });
             push_rest(col, top, q, best);
             if (q.any(best)) {
                 go(q.next(best));
@@ -221,7 +243,17 @@ struct MeshClosest {
 // against 3.09 for one ray per thread over the binary nodes.
 __global__ void __maxnreg__(64) k_mesh_closest_refill(const __grid_constant__ MeshArgs a) {
     extern __shared__ uint2 smem[];
-    MeshClosest b(a, smem);
+    MeshClosest<false> b(a, smem);
+    trace_rays(b, a.n, a.c);
+}
+
+// For batches that give each ray a lane of its own: the walk that keeps more
+// loads under way (92 registers, 5 blocks). 10,000 triangles, 4,099 rays 76 ->
+// 67 us, 40,000 rays 157 -> 126; 300,000 triangles, 1,000 rays 196 -> 161,
+// 40,000 rays 340 -> 285.
+__global__ void k_mesh_closest_few(const __grid_constant__ MeshArgs a) {
+    extern __shared__ uint2 smem[];
+    MeshClosest<true> b(a, smem);
     trace_rays(b, a.n, a.c);
 }
 
@@ -360,7 +392,7 @@ __global__ void __maxnreg__(64) k_mesh_closest_phased(MeshArgs a, int refill, in
 }
 
 // One ray of an any-hit query on one mesh (BVHAccel::IntersectP).
-struct MeshAny {
+template <bool FEW> struct MeshAny {
     const MeshArgs &a;
     const float *tmaxs;
     uint8_t *out;
@@ -406,16 +438,32 @@ struct MeshAny {
 
     __device__ __forceinline__ bool step() {
         if (ntri > 0) {
-            if (tri_occludes(load_tri(a.tris, a.e2z, tri, a.B), r, tmax)) {
-                occluded = true;
-                return true;
+            if constexpr (FEW) {
+                TriV T[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    if (k < ntri)
+                        T[k] = load_tri(a.tris, a.e2z, tri + k, a.B);
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    if (k < ntri && tri_occludes(T[k], r, tmax))
+                        occluded = true;
+                if (occluded)
+                    return true;
+            } else {
+                if (tri_occludes(load_tri(a.tris, a.e2z, tri, a.B), r, tmax)) {
+                    occluded = true;
+                    return true;
+                }
+                tri++;
+                ntri--;
+                if (ntri > 0)
+                    return false;
             }
-            tri++;
-            ntri--;
-            if (ntri > 0)
-                return false;
         } else {
             const QuadOrder q = quad_order(load_quad(a.nodes, ref, a.B), p);
+            if constexpr (FEW)
+                q.rest(tmax, [&](uint32_t x, float) { fetch_child(a.nodes, a.tris, x); });
             push_rest(col, top, q, tmax);
             if (q.any(tmax)) {
                 go(q.next(tmax));
@@ -435,11 +483,12 @@ struct MeshBox {
     float b[6];
 };
 
-__global__ void __maxnreg__(64) k_mesh_occluded(const __grid_constant__ MeshArgs a,
+template <bool FEW>
+__global__ void __maxnreg__(FEW ? 128 : 64) k_mesh_occluded(const __grid_constant__ MeshArgs a,
                                                 const __grid_constant__ MeshBox box,
                                                 const float *tmax, uint8_t *out) {
     extern __shared__ uint32_t smem32[];
-    MeshAny b(a, box.b, tmax, out, smem32);
+    MeshAny<FEW> b(a, box.b, tmax, out, smem32);
     trace_rays(b, a.n, a.c);
 }
 
@@ -457,7 +506,7 @@ template <class E> __device__ __forceinline__ StackCol<E> scene_col(const DevSce
 
 // 2,000,003 rays on 122,880 triangles with geometry, half of them incoherent:
 // 0.50 ms against 0.74 for one ray per thread; any hit 0.35 against 0.81.
-struct SceneClosest {
+template <bool FEW> struct SceneClosest {
     const DevScene &S;
     const SceneArgs &a;
     int32_t *out_obj, *out_prim;
@@ -465,7 +514,7 @@ struct SceneClosest {
     bool raw; // out_prim takes the leaf-order triangle index (k_scene_finish resolves it)
     const StackCol<uint2> col;
     uint32_t idx = 0;
-    ClosestWalk w;
+    ClosestWalk<FEW> w;
 
     __device__ __forceinline__ SceneClosest(const DevScene &scene, const SceneArgs &args,
                                             int32_t *obj, int32_t *prim, float *t, bool leaf_order,
@@ -491,11 +540,12 @@ struct SceneClosest {
     }
 };
 
-__global__ void __maxnreg__(64)
+template <bool FEW>
+__global__ void __maxnreg__(FEW ? 128 : 64)
     k_scene_closest(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
                     int32_t *out_obj, int32_t *out_prim, float *out_t, bool raw) {
     extern __shared__ uint2 smem[];
-    SceneClosest b(S, a, out_obj, out_prim, out_t, raw, smem);
+    SceneClosest<FEW> b(S, a, out_obj, out_prim, out_t, raw, smem);
     trace_rays(b, a.n, a.c);
 }
 
@@ -563,14 +613,14 @@ __global__ void __launch_bounds__(256)
     geo[i * 6 + 5] = nz;
 }
 
-struct SceneAny {
+template <bool FEW> struct SceneAny {
     const DevScene &S;
     const SceneArgs &a;
     const float *tmaxs;
     uint8_t *out;
     const StackCol<uint32_t> col;
     uint32_t idx = 0;
-    AnyWalk w;
+    AnyWalk<FEW> w;
 
     __device__ __forceinline__ SceneAny(const DevScene &scene, const SceneArgs &args,
                                         const float *tmax, uint8_t *hit, uint32_t *smem)
@@ -587,11 +637,12 @@ struct SceneAny {
     __device__ __forceinline__ void finish() { out[idx] = w.occluded ? 1 : 0; }
 };
 
-__global__ void __maxnreg__(64)
+template <bool FEW>
+__global__ void __maxnreg__(FEW ? 128 : 64)
     k_scene_occluded(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
                      const float *tmax, uint8_t *out) {
     extern __shared__ uint32_t smem32[];
-    SceneAny b(S, a, tmax, out, smem32);
+    SceneAny<FEW> b(S, a, tmax, out, smem32);
     trace_rays(b, a.n, a.c);
 }
 
@@ -902,6 +953,14 @@ int resident_blocks(const void *fn, int block, size_t smem) {
     return std::max(1, bps);
 }
 
+// Batches traced by the FEW form of a kernel: up to 640 rays per SM, what its
+// residents (5 blocks of 128) hold at once. Closest hit on one mesh takes it up
+// to twice that, its rays being slower apart than the larger batch's queueing
+// (100,000 triangles: 140,000 rays 454 -> 386 us, 180,000 479 -> 448, 250,000
+// 552 -> 546, 400,000 722 -> 753; scene level 100,000 rays 115 -> 108, 140,000
+// 115 -> 122).
+bool few_rays(int64_t n, int per_sm = 640) { return n <= (int64_t) device_sm_count() * per_sm; }
+
 // Launch shape of a query kernel over n rays: shared memory, grid, and the
 // scratch it needs (counter and stack spill). The grid is what the device
 // holds at once, less for batches that give its warps less than one ray each.
@@ -990,8 +1049,10 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     // allocate nothing; every other call gets its own
     if (in_capture && mode > 0 && !counter)
         counter = (unsigned *) s.d_counter.ptr;
+    const bool few = mode == 0 && few_rays(n, 1280);
     const void *fn = mode == 1   ? (const void *) k_mesh_closest_persistent
                      : mode == 3 ? (const void *) k_mesh_closest_phased
+                     : few         ? (const void *) k_mesh_closest_few
                                  : (const void *) k_mesh_closest_refill;
     const int refill = mode >= 2 && cfg->batch > 0 ? std::min(cfg->batch, 32) : 8;
     const int cap = stack_cap(obj.qstack);
@@ -1017,6 +1078,8 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     else if (mode == 3)
         k_mesh_closest_phased<<<L.grid, block, L.smem, st>>>(
             a, refill, cfg->leaf_batch > 0 ? std::min(cfg->leaf_batch, 32) : 16);
+    else if (few)
+        k_mesh_closest_few<<<L.grid, block, L.smem, st>>>(a);
     else
         k_mesh_closest_refill<<<L.grid, block, L.smem, st>>>(a);
     PRR_CUDA_TRY(cudaGetLastError());
@@ -1046,10 +1109,11 @@ int launch_mesh_occluded(const Scene &s, int object, const float *o, const float
         box.b[k] = obj.bvh.bounds[k];
     const int block = 128;
     TraceLaunch L;
-    if (int rc = plan_trace(L, a.c, (const void *) k_mesh_occluded, block, stack_cap(obj.qstack),
+    auto kern = few_rays(n) ? k_mesh_occluded<true> : k_mesh_occluded<false>;
+    if (int rc = plan_trace(L, a.c, (const void *) kern, block, stack_cap(obj.qstack),
                             sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
-    k_mesh_occluded<<<L.grid, block, L.smem, st>>>(a, box, tmax, hit);
+    kern<<<L.grid, block, L.smem, st>>>(a, box, tmax, hit);
     PRR_CUDA_TRY(cudaGetLastError());
     return PRR_OK;
 }
@@ -1066,11 +1130,12 @@ int launch_scene_closest(const Scene &s, const float *o, const float *d, int64_t
     const int block = 128;
     SceneArgs a{o, d, (uint32_t) n, {}};
     TraceLaunch L;
-    if (int rc = plan_trace(L, a.c, (const void *) k_scene_closest, block,
+    auto kern = few_rays(n) ? k_scene_closest<true> : k_scene_closest<false>;
+    if (int rc = plan_trace(L, a.c, (const void *) kern, block,
                             stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
                             sizeof(uint2), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
-    k_scene_closest<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo != nullptr);
+    kern<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo != nullptr);
     if (geo)
         k_scene_finish<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(s.dev, o, d, n, obj, prim, t,
                                                                      geo);
@@ -1089,11 +1154,12 @@ int launch_scene_occluded(const Scene &s, const float *o, const float *d, const 
     const int block = 128;
     SceneArgs a{o, d, (uint32_t) n, {}};
     TraceLaunch L;
-    if (int rc = plan_trace(L, a.c, (const void *) k_scene_occluded, block,
+    auto kern = few_rays(n) ? k_scene_occluded<true> : k_scene_occluded<false>;
+    if (int rc = plan_trace(L, a.c, (const void *) kern, block,
                             stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
                             sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
-    k_scene_occluded<<<L.grid, block, L.smem, st>>>(s.dev, a, tmax, hit);
+    kern<<<L.grid, block, L.smem, st>>>(s.dev, a, tmax, hit);
     PRR_CUDA_TRY(cudaGetLastError());
     return PRR_OK;
 }

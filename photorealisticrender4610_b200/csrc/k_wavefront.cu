@@ -390,7 +390,7 @@ __device__ __forceinline__ void wf_extend(const DevScene &S0, const Wf &w, int i
     int p = -1;
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    ClosestWalk cw;
+    ClosestWalk<> cw;
     bool more = n > 0;
     if (!more)
         return;
@@ -827,7 +827,7 @@ __device__ __forceinline__ void wf_shadow(const DevScene &S0, const Wf &w, int r
     int job = -1; // -2: a lane that takes no rays
     // this lane's ray's scene (server steps; a valid scene before the first ray)
     const DevScene *ls = MULTI ? w.reqs[0].scene : nullptr;
-    AnyWalk aw;
+    AnyWalk<> aw;
     bool more = n > 0;
     if (!more)
         return;

@@ -581,6 +581,15 @@ __device__ __forceinline__ void push_rest(const StackCol<uint32_t> &st, uint32_t
         q.rest(tmax, [&](uint32_t c, float) { st.put(top, c); });
 }
 
+// Asks for a child's first bytes in L1: for batches so small that memory is idle
+// and a walk waits on one fetch after another (a child waiting on the stack is
+// then at hand when it is popped).
+__device__ __forceinline__ void fetch_child(const QNode *nodes, const Tri *tris, uint32_t ref) {
+    const void *g = (ref & kLeafBit) ? (const void *) (tris + leaf_first(ref))
+                                     : (const void *) (nodes + ref);
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(g));
+}
+
 // Per-thread stack column in shared memory.
 struct SmemStack {
     uint2 *base; // &smem[tid]; entry k at base[k * stride]

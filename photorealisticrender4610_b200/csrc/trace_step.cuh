@@ -20,7 +20,9 @@ namespace prr {
 
 // Closest hit: Scene::intersect -> scene BVH, general path; each mesh leaf is
 // searched from +inf on its own (BVH.cpp:359-369).
-struct ClosestWalk {
+// FEW: the form for batches of few rays -- a step tests a leaf's triangles
+// together, their loads under way at once, and asks for the children it pushes.
+template <bool FEW = false> struct ClosestWalk {
     RayD r;
     RayPre p;
     float best;    // closest hit of the level being walked
@@ -82,7 +84,23 @@ struct ClosestWalk {
     __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint2> &st) {
         bool down = false;
         uint32_t x = 0;
-        if (ntri > 0) {
+        if (FEW && ntri > 0) {
+            TriV T[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < ntri)
+                    T[k] = load_tri(S, ref + k);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < ntri) {
+                    float t, u, v;
+                    if (tri_hit(T[k], r, t, u, v) && t < best) {
+                        best = t;
+                        bhit = (int) (ref + k);
+                    }
+                }
+            ntri = 0;
+        } else if (ntri > 0) {
             const TriV T = load_tri(S, ref);
             float t, u, v;
             if (tri_hit(T, r, t, u, v) && t < best) {
@@ -94,6 +112,8 @@ struct ClosestWalk {
                 return false;
         } else {
             const QuadOrder q = quad_order(load_quad(S, ref), p);
+            if (FEW && cur_obj >= 0)
+                q.rest(best, [&](uint32_t c, float) { fetch_child(S.qnodes, S.tris, c); });
             push_rest(st, top, q, best);
             down = q.any(best);
             x = q.next(best);
@@ -130,7 +150,7 @@ struct ClosestWalk {
 // Sphere intersectT (BVH.cpp:421-473, Triangle.hpp:141-147, Object.hpp:24-29).
 // Leaves are taken near ones first rather than in the reference's order: the
 // answer is whether any of those entered before tmax occludes.
-struct AnyWalk {
+template <bool FEW = false> struct AnyWalk {
     RayD r;
     RayPair p;
     float tmax;
@@ -183,7 +203,26 @@ struct AnyWalk {
     __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint32_t> &st) {
         bool down = false;
         uint32_t x = 0;
-        if (ntri > 0) {
+        if (FEW && ntri > 0) {
+            TriV T[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < ntri)
+                    T[k] = load_tri(S, ref + k);
+            bool found = false;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < ntri && tri_occludes(T[k], r, tmax))
+                    found = true;
+            ntri = 0;
+            if (found) {
+                if (1e-3f < tmax) { // as below
+                    occluded = true;
+                    return true;
+                }
+                top = floor;
+            }
+        } else if (ntri > 0) {
             if (tri_occludes(load_tri(S, ref), r, tmax)) {
                 // MeshTriangle::intersectT answers 1e-3; the scene-level
                 // caller then needs 1e-3 < tMax
@@ -199,6 +238,8 @@ struct AnyWalk {
                 return false;
         } else {
             const QuadOrder q = quad_order(load_quad(S, ref), p);
+            if (FEW && in_mesh)
+                q.rest(tmax, [&](uint32_t c, float) { fetch_child(S.qnodes, S.tris, c); });
             push_rest(st, top, q, tmax);
             down = q.any(tmax);
             x = q.next(tmax);

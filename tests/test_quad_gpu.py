@@ -184,7 +184,7 @@ def test_tree_deeper_than_the_collapse_limit(cuda):
         assert np.array_equal(bits(t.cpu().numpy()), bits(ts))
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 4_735, 4_737, 40_001, 170_499, 250_007])
+@pytest.mark.parametrize("n", [1, 31, 33, 4_735, 4_737, 40_001, 94_720, 94_721, 189_441, 250_007])
 def test_batch_sizes(port, cuda, n):
     verts = soup(300)
     o, d, tmax = rays(verts, n, n)
