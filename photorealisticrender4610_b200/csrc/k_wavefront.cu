@@ -1285,21 +1285,22 @@ struct WavefrontPlan {
 
 namespace {
 
-// Bytes of the path-state layout for P paths and npix film pixels.
-size_t wf_bytes(size_t P, int npix) {
+// Bytes of the path-state layout for P paths, npix film pixels and the stacks'
+// spilled entries.
+size_t wf_bytes(size_t P, int npix, size_t spill) {
     const int ntiles = (int) ((P + kPartTile - 1) / kPartTile);
     const int ptiles = (npix + kPartTile - 1) / kPartTile;
     return 256 * 48 + P * (8 + 16 * 16 + 4 * 2 + 4 * 9 + 2 + 4) + (size_t) ntiles * kPartTile +
            (size_t) npix * (16 + 8 + 32) + (size_t) ptiles * kPartTile +
-           (size_t) std::max(ntiles, ptiles) * 32 + 4096;
+           (size_t) std::max(ntiles, ptiles) * 32 + 4096 + spill;
 }
 
 // Carves the per-path arrays, queues, counters and partition buffers of P
 // paths and npix pixels out of `buf` (grown as needed).
-int wf_layout(DevBuf &buf, Wf &w, size_t P, int npix) {
+int wf_layout(DevBuf &buf, Wf &w, size_t P, int npix, size_t spill) {
     const int ntiles = (int) ((P + kPartTile - 1) / kPartTile);
     const int ptiles = (npix + kPartTile - 1) / kPartTile;
-    const size_t bytes = wf_bytes(P, npix);
+    const size_t bytes = wf_bytes(P, npix, spill);
     PRR_CUDA_TRY(buf.ensure(bytes));
     char *cur = (char *) buf.ptr;
     w.rng = carve<uint64_t>(cur, P);
@@ -1338,21 +1339,22 @@ int wf_layout(DevBuf &buf, Wf &w, size_t P, int npix) {
     w.ptag = carve<uint8_t>(cur, (size_t) ptiles * kPartTile);
     w.wel0 = carve<float4>(cur, (size_t) npix);
     w.wel1 = carve<float4>(cur, (size_t) npix);
+    w.spill = carve<char>(cur, spill);
     if ((size_t) (cur - (char *) buf.ptr) > bytes)
         return fail(PRR_ERR_INTERNAL, "wavefront buffer layout overflow");
     return PRR_OK;
 }
 
-// Launch shape of one bounce: traversal grids, stack split, spill buffer.
+// Launch shape of one bounce: traversal grids, stack split, spill size.
 struct WfShape {
     int block, refill, g_ext, g_sh, g_shade, g_gen, ntiles, ptiles;
-    size_t smem_ext, smem_sh;
+    size_t smem_ext, smem_sh, spill_bytes;
     void (*ext)(DevScene, Wf, int, int);
     void (*sh)(DevScene, Wf, int);
 };
 
 template <bool MULTI>
-int wf_shape(Wf &w, DevBuf &spill, int block_req, int stack_req, int refill_req, WfShape &L) {
+int wf_shape(Wf &w, int block_req, int stack_req, int refill_req, WfShape &L) {
     const int sms = device_sm_count();
     L.block = block_req > 0 ? block_req : 128;
     // Stacks: the scene-level one wholly in shared memory, the mesh one up to
@@ -1405,11 +1407,9 @@ int wf_shape(Wf &w, DevBuf &spill, int block_req, int stack_req, int refill_req,
     L.g_ext = sms * std::max(1, occ_ext);
     L.g_sh = sms * std::max(1, occ_sh);
     const size_t spill_entries = (size_t) (w.blas_cap - w.blas_sm);
-    const size_t spill_bytes =
+    L.spill_bytes =
         spill_entries * std::max((size_t) L.g_ext * L.block * sizeof(uint2),
                                  (size_t) L.g_sh * L.block * sizeof(uint32_t));
-    PRR_CUDA_TRY(spill.ensure(spill_bytes));
-    w.spill = spill.ptr;
     L.g_shade = sms * 8;
     L.g_gen = (int) std::min<int64_t>(((int64_t) w.P + 255) / 256, (int64_t) sms * 16);
     L.ntiles = (int) (((size_t) w.P + kPartTile - 1) / kPartTile);
@@ -1505,6 +1505,14 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.tlas_cap = S.tlas_stack + 1;
     w.blas_cap = S.blas_stack + 1;
     w.count_stack = S.tlas_depth + S.blas_depth + 2;
+    w.ordered = s.wf_ordered ? 1 : 0;
+    w.adaptive = rs.min_spp < rs.max_spp ? 1 : 0;
+    w.min_spp = rs.min_spp;
+    w.max_spp = rs.max_spp;
+    w.threshold = rs.variance_threshold;
+    w.stats = s.wf_stats;
+    w.check = S.check;
+    WfShape L{};
     // Paths per pass: whole samples of the window, by default at most 32M in
     // flight (10 GB of path state): every bounce of a pass ends in a tail of
     // long rays, so fewer and larger passes pay it less often (museum-like
@@ -1519,23 +1527,15 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
             spp_pass--;
         w.spp_pass = spp_pass;
         w.P = spp_pass * w.npix;
-        const int rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix);
+        int rc = wf_shape<false>(w, s.wf_block, s.wf_stack, s.wf_refill, L);
+        if (rc == PRR_OK)
+            rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix, L.spill_bytes);
         if (rc == PRR_OK)
             break;
         if (rc != PRR_ERR_OUT_OF_MEMORY || s.wf_paths > 0 || target <= kLeastPaths)
             return rc;
         cudaGetLastError(); // the failed allocation
     }
-    w.ordered = s.wf_ordered ? 1 : 0;
-    w.adaptive = rs.min_spp < rs.max_spp ? 1 : 0;
-    w.min_spp = rs.min_spp;
-    w.max_spp = rs.max_spp;
-    w.threshold = rs.variance_threshold;
-    w.stats = s.wf_stats;
-    w.check = S.check;
-    WfShape L;
-    if (int rc = wf_shape<false>(w, s.d_wf_spill, s.wf_block, s.wf_stack, s.wf_refill, L))
-        return rc;
     const WfParts parts = wf_parts(w);
 
     PRR_CUDA_TRY(cudaMemsetAsync(w.film, 0, (size_t) w.npix * sizeof(float3), st));
@@ -1699,10 +1699,10 @@ int wavefront_step_multi(WfMultiState &ms, const WfStepReq *reqs, int n,
         w.n_reqs = x.b - x.a;
         w.tlas_cap = tlas_cap;
         w.blas_cap = blas_cap;
-        if (int rc = wf_layout(ms.state, w, (size_t) maxP, 1))
+        WfShape L{};
+        if (int rc = wf_shape<true>(w, 128, 8, 0, L))
             return rc;
-        WfShape L;
-        if (int rc = wf_shape<true>(w, ms.spill, 128, 8, 0, L))
+        if (int rc = wf_layout(ms.state, w, (size_t) maxP, 1, L.spill_bytes))
             return rc;
         const WfParts parts = wf_parts(w);
         PRR_CUDA_TRY(cudaMemsetAsync(w.tag, 0xFF, (size_t) L.ntiles * kPartTile, st));

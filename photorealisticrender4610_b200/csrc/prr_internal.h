@@ -91,6 +91,7 @@ struct HostObject {
     uint32_t root = 0;
     uint32_t qroot = 0; // root over the four-wide nodes
     int qstack = 0;     // stack entries a walk over them may need
+    std::vector<QNode> quads; // its four-wide nodes, while the scene is built
 };
 
 struct WavefrontPlan;
@@ -121,7 +122,7 @@ struct Scene {
     DevBuf d_render, d_render_spp; // per-slice partial sums / adaptive spp
     DevBuf d_counter;      // persistent-kernel work counters
     DevBuf d_check;        // status words of the checked build's device-side tests
-    DevBuf d_wavefront;    // wavefront path state, queues and film
+    DevBuf d_wavefront;    // wavefront path state, queues, film and stack spill
     std::shared_ptr<WavefrontPlan> wf_plan; // captured pass graph
     int64_t wf_paths = 0;  // paths in flight per pass (0 = automatic)
     int wf_block = 0;      // extend / shadow block size (0 = 128)
@@ -133,7 +134,6 @@ struct Scene {
     // queues 16.2, both 16.7).
     int wf_stack = 8;      // mesh-stack entries per thread in shared memory (0 = whole stack)
     bool wf_ordered = true; // queues rebuilt in path order by a stable partition
-    DevBuf d_wf_spill;     // global part of the traversal stacks
     unsigned long long *wf_stats = nullptr; // set by prr_render_counts: count traversal work
     int64_t last_launches = 0; // kernels the last prr_render launched
     // Renders reuse the scratch above; each render waits for the previous
@@ -188,10 +188,10 @@ struct WfStepReq {
     uint64_t seed;
     float3 *film; // ww*wh running sums (device)
 };
-// Buffers a server keeps across its wavefront steps: path state, stack
-// spill, and the request table (device, and pinned host for the upload).
+// Buffers a server keeps across its wavefront steps: path state (with the stack
+// spill), and the request table (device, and pinned host for the upload).
 struct WfMultiState {
-    DevBuf state, spill, reqs;
+    DevBuf state, reqs;
     void *h_table = nullptr;
     size_t h_cap = 0;
     WfMultiState() = default;

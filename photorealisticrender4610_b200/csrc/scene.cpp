@@ -125,8 +125,9 @@ void pack_quads(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<
             return true;
         };
         out.resize(base);
+        out.reserve(base + n / 4 + 1);
         std::vector<size_t> todo{0};  // binary node of each four-wide node
-        todo.reserve(n / 3 + 1);
+        todo.reserve(n / 4 + 1);
         for (size_t w = 0; w < todo.size(); w++) {
             const size_t i = todo[w];
             QNode q;
@@ -176,6 +177,23 @@ void pack_quads(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<
             break;
     }
     root_ref = (uint32_t) base;
+}
+
+// Appends one mesh's four-wide nodes, packed with references from 0, to the
+// scene's: moves node references by the nodes before them and leaf references
+// by the mesh's first triangle.
+void append_quads(const std::vector<QNode> &quads, uint32_t &root_ref, int tri_base,
+                  std::vector<QNode> &out) {
+    const uint32_t node_base = (uint32_t) out.size(), leaf_base = (uint32_t) tri_base << 2;
+    auto moved = [&](uint32_t r) { return r + ((r & kLeafBit) ? leaf_base : node_base); };
+    root_ref = moved(root_ref);
+    out.resize(out.size() + quads.size());
+    QNode *q = out.data() + node_base;
+    for (size_t k = 0; k < quads.size(); k++) {
+        q[k] = quads[k];
+        for (uint32_t &r : q[k].ref)
+            r = moved(r);
+    }
 }
 
 template <class T> int upload(DevBuf &b, const std::vector<T> &v) {
@@ -270,6 +288,7 @@ int build_scene(Scene &s, cudaStream_t st) {
         for (float x : pa)
             a += x;
         o.area = a;
+        pack_quads(o.bvh, false, 0, o.quads, o.qroot, o.qstack);
     };
     {
         // big meshes get the threads; small ones run side by side
@@ -373,7 +392,8 @@ int build_scene(Scene &s, cudaStream_t st) {
         }
         if (int rc = pack_tree(o.bvh, false, base, nodes, o.root))
             return rc;
-        pack_quads(o.bvh, false, base, qnodes, o.qroot, o.qstack);
+        append_quads(o.quads, o.qroot, base, qnodes);
+        std::vector<QNode>().swap(o.quads);
         blas_stack = std::max(blas_stack, o.qstack);
         blas_depth = std::max(blas_depth, o.bvh.max_depth);
         base += (int) nt;
