@@ -35,6 +35,9 @@ PRR_HD inline uint32_t mesh_leaf_ref(uint32_t first, uint32_t count) {
 }
 PRR_HD inline uint32_t leaf_first(uint32_t ref) { return (ref & ~kLeafBit) >> 2; }
 PRR_HD inline uint32_t leaf_count(uint32_t ref) { return (ref & 3u) + 1u; }
+// The leaf reference without its first triangle; 0 (no leaf reference) when
+// that was the last.
+PRR_HD inline uint32_t leaf_rest(uint32_t ref) { return (ref & 3u) ? ref + 3u : 0u; }
 
 // One interior node: boxes of its left (reference idx+1) and right
 // (reference first_child) children, interleaved [minX,maxX,minY,maxY,minZ,maxZ]

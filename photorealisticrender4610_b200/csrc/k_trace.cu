@@ -150,22 +150,12 @@ template <bool FEW> struct MeshClosest {
     RayPair p;
     float best = 0.f;
     int hit = -1;
-    uint32_t ref = 0, tri = 0, ntri = 0;
+    uint32_t ref = 0; // next node, or the leaf triangles left to test (a leaf reference)
     uint32_t top = 0;
 
     __device__ __forceinline__ MeshClosest(const MeshArgs &args, uint2 *smem)
         : a(args), col(smem, (uint2 *) args.c.spill, args.c.stack_sm, args.c.stack_cap,
                        args.B.check) {}
-
-    __device__ __forceinline__ void go(uint32_t x) {
-        if (x & kLeafBit) {
-            tri = leaf_first(x);
-            ntri = leaf_count(x);
-        } else {
-            ref = x;
-            ntri = 0;
-        }
-    }
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = ray_at(a, i);
@@ -178,13 +168,15 @@ template <bool FEW> struct MeshClosest {
             finish();
             return false;
         }
-        go(a.root);
+        ref = a.root;
         return true;
     }
 
     __device__ __forceinline__ bool step() {
-        if (ntri > 0) {
+        if (ref & kLeafBit) {
+            const uint32_t tri = leaf_first(ref);
             if constexpr (FEW) {
+                const uint32_t ntri = leaf_count(ref);
                 // the whole leaf, its loads under way together
                 TriV T[4];
 #pragma unroll
@@ -207,9 +199,8 @@ template <bool FEW> struct MeshClosest {
                     best = t;
                     hit = (int) tri;
                 }
-                tri++;
-                ntri--;
-                if (ntri > 0)
+                ref = leaf_rest(ref);
+                if (ref)
                     return false;
             }
         } else {
@@ -218,14 +209,14 @@ template <bool FEW> struct MeshClosest {
                 q.rest(best, [&](uint32_t x, float) { fetch_child(a.nodes, a.tris, x); });
             push_rest(col, top, q, best);
             if (q.any(best)) {
-                go(q.next(best));
+                ref = q.next(best);
                 return false;
             }
         }
         while (!col.empty(top)) {
             const uint2 e = col.pop(top);
             if (__uint_as_float(e.y) < best) {
-                go(e.x);
+                ref = e.x;
                 return false;
             }
         }
@@ -236,7 +227,7 @@ template <bool FEW> struct MeshClosest {
 };
 
 // 56 registers, so 9 resident blocks of 128 with 24 stack entries in shared
-// memory. 1M triangles, 4,194,304 reordered rays: 3.27 ms against 3.64 over the
+// memory. 1M triangles, 4,194,304 reordered rays: 3.21 ms against 3.64 over the
 // binary nodes (634M against 791M warp instructions for 1M rays: bound by issue
 // and the latency of L2; whole stacks in shared memory, 6 blocks, gave 3.70).
 // 300,000 triangles, 1,500,007 rays in input order, default call: 1.67 ms
@@ -294,6 +285,7 @@ __global__ void k_mesh_closest_persistent(MeshArgs a) {
 // older closest hit only add leaves that this re-test then drops, since a
 // box contains the boxes below it and the slab entry distance is monotone in
 // the box.
+
 constexpr uint32_t kNoRef = 0xFFFFFFFFu;
 
 __global__ void __maxnreg__(64) k_mesh_closest_phased(MeshArgs a, int refill, int tri_min) {
@@ -402,7 +394,7 @@ template <bool FEW> struct MeshAny {
     RayD r;
     RayPair p;
     float tmax = 0.f;
-    uint32_t ref = 0, tri = 0, ntri = 0;
+    uint32_t ref = 0; // as in MeshClosest
     uint32_t top = 0;
     bool occluded = false;
 
@@ -410,16 +402,6 @@ template <bool FEW> struct MeshAny {
                                        const float *tmax_, uint8_t *hit, uint32_t *smem)
         : a(args), tmaxs(tmax_), out(hit), box(root_box),
           col(smem, (uint32_t *) args.c.spill, args.c.stack_sm, args.c.stack_cap, args.B.check) {}
-
-    __device__ __forceinline__ void go(uint32_t x) {
-        if (x & kLeafBit) {
-            tri = leaf_first(x);
-            ntri = leaf_count(x);
-        } else {
-            ref = x;
-            ntri = 0;
-        }
-    }
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
@@ -432,13 +414,15 @@ template <bool FEW> struct MeshAny {
             finish();
             return false;
         }
-        go(a.root);
+        ref = a.root;
         return true;
     }
 
     __device__ __forceinline__ bool step() {
-        if (ntri > 0) {
+        if (ref & kLeafBit) {
+            const uint32_t tri = leaf_first(ref);
             if constexpr (FEW) {
+                const uint32_t ntri = leaf_count(ref);
                 TriV T[4];
 #pragma unroll
                 for (uint32_t k = 0; k < 4; k++)
@@ -455,9 +439,8 @@ template <bool FEW> struct MeshAny {
                     occluded = true;
                     return true;
                 }
-                tri++;
-                ntri--;
-                if (ntri > 0)
+                ref = leaf_rest(ref);
+                if (ref)
                     return false;
             }
         } else {
@@ -466,13 +449,13 @@ template <bool FEW> struct MeshAny {
                 q.rest(tmax, [&](uint32_t x, float) { fetch_child(a.nodes, a.tris, x); });
             push_rest(col, top, q, tmax);
             if (q.any(tmax)) {
-                go(q.next(tmax));
+                ref = q.next(tmax);
                 return false;
             }
         }
         if (col.empty(top))
             return true;
-        go(col.pop(top));
+        ref = col.pop(top);
         return false;
     }
 
