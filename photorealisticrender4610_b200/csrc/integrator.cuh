@@ -44,11 +44,13 @@ __device__ __forceinline__ void finalize_attr(const DevScene &S, const DevObject
     }
 }
 
+// OOL: spheres tested out of line.
+template <bool OOL = false>
 __device__ __forceinline__ Inter intersect(const DevScene &S, const Ray3 &ray, SmemStack &tst,
                                            SmemStack &bst) {
     RayD r{ray.o.x, ray.o.y, ray.o.z, ray.d.x, ray.d.y, ray.d.z};
     const RayPre p = precompute(r);
-    const SceneHit h = scene_closest(S, r, p, tst, bst);
+    const SceneHit h = scene_closest<false, OOL>(S, r, p, tst, bst);
     Inter in;
     in.hit = h.obj >= 0;
     in.a = no_attr();
@@ -73,11 +75,12 @@ __device__ __forceinline__ Inter intersect(const DevScene &S, const Ray3 &ray, S
     return in;
 }
 
+template <bool OOL = false>
 __device__ __forceinline__ bool occluded(const DevScene &S, V3 o, V3 d, float tmax, SmemStack &tst,
                                          SmemStack &bst) {
     RayD r{o.x, o.y, o.z, d.x, d.y, d.z};
     const RayPre p = precompute(r);
-    return scene_occluded(S, r, p, tst, bst, tmax);
+    return scene_occluded<false, OOL>(S, r, p, tst, bst, tmax);
 }
 
 __device__ __forceinline__ float mis(float a, float b) { return (a * a) / (a * a + b * b + 1e-6f); }
@@ -105,38 +108,60 @@ struct PathCounters {
 // twice in the code instead of two to four times: with them inlined at every
 // use the megakernels stalled on instruction fetch (9 warps of every issue
 // cycle; Cornell box 256x256, 16 spp, 2.18 ms).
+//
+// SYNC: every thread of the block calls it together, with run = false for
+// those without a path, and the block starts each iteration together. Its
+// warps then read the same instructions at about the same time, which pays
+// where the rays' walks are short (Cornell box 2.05 -> 1.44 ms in blocks of
+// 384) and costs where they are long and uneven (see render_plain).
+template <bool SYNC = false>
 static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float clamp, Rng &rng,
-                       SmemStack &tst, SmemStack &bst, PathCounters &cnt) {
+                              SmemStack &tst, SmemStack &bst, PathCounters &cnt,
+                              bool run = true) {
     enum { kFirst, kSpecular, kPending };
     V3 L = v3(0.f), beta = v3(1.f);
     Ray3 cur = ray;
     const DevEnv &env = S.env;
     const V3 bg = v3(S.background[0], S.background[1], S.background[2]);
+// the path has ended: the loop is left, or (SYNC) gone through idle
+#define PRR_PATH_END                                                                               \
+    if constexpr (SYNC)                                                                            \
+        continue;                                                                                  \
+    else                                                                                           \
+        break
     int bounce = 0;
     int from = kFirst;                     // what spawned the ray
     V3 scale = v3(0.f), prev = v3(0.f);    // pending bounce: f / pdf, the hit it left from
     float bpdf = 0.f;                      // its pdf
+    (void) run; // only SYNC reads it
     for (;;) {
-        const Inter in = intersect(S, cur, tst, bst);
+        if constexpr (SYNC) {
+            if (!__syncthreads_or(run))
+                break;
+            if (!run)
+                continue;
+            run = false; // set again where the path goes on
+        }
+        const Inter in = intersect<SYNC>(S, cur, tst, bst);
         cnt.closest++;
         const bool lit = !in.hit || S.materials[in.mat].kind == kMatEmissive;
         if (from != kFirst && !(from == kPending && lit)) {
             if (from == kPending) {
                 beta = beta * scale;
                 if (!finite3(beta))
-                    break;
+                    PRR_PATH_END;
                 // Russian roulette from bounce 3 (Integrator.cpp:250-256)
                 if (bounce >= 3) {
                     const float mc = max3(beta);
                     const float q = smax(0.05f, 1.f - mc);
                     if (rng.next() < q)
-                        break;
+                        PRR_PATH_END;
                     beta = beta * (1.f / (1.f - q));
                 }
             }
             bounce++;
             if (bounce >= max_depth)
-                break;
+                PRR_PATH_END;
         }
         if (lit && (from == kPending || bounce == 0 || from == kSpecular)) {
             // light reached: seen directly (Integrator.cpp:119-139), or by the
@@ -164,10 +189,10 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
             }
             L = L + ((bounce > 0) ? clamp_indirect(c, clamp) : c);
             if (from == kPending)
-                break;
+                PRR_PATH_END;
         }
         if (!in.hit)
-            break;
+            PRR_PATH_END;
         const DevMaterial &m = S.materials[in.mat];
         const V3 hp = in.p;
         const V3 gn = in.n;
@@ -179,7 +204,7 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
             // delta chain (Integrator.cpp:143-169)
             const BSDFSample bs = delta_sample(m, sd, wo, rng);
             if (bs.pdf < 1e-6f)
-                break;
+                PRR_PATH_END;
             beta = beta * bs.f / bs.pdf;
             const bool trans = dot(bs.wi, gn) < 0.f;
             const V3 off = trans ? -gn : gn;
@@ -187,6 +212,8 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
             if (trans)
                 beta = beta * sd.base;
             from = kSpecular;
+            if constexpr (SYNC)
+                run = true;
             continue;
         }
         const bool indirect = bounce > 0;
@@ -239,14 +266,14 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
                 V3 c = beta * (mis(pdf, bp) * em * f / (d == 0 ? pdf : pdf + 1e-6f));
                 if (!(c.x == 0.f && c.y == 0.f && c.z == 0.f)) {
                     cnt.shadow++;
-                    if (occluded(S, hp + wi * PRR_EPS, wi, tmax, tst, bst))
+                    if (occluded<SYNC>(S, hp + wi * PRR_EPS, wi, tmax, tst, bst))
                         c = v3(0.f);
                 }
                 L = L + (indirect ? clamp_indirect(c, clamp) : c);
             }
         }
         if (bp < 1e-6f)
-            break;
+            PRR_PATH_END;
         if (!(bp > 1e-6f)) // DiffuseMaterial::sample leaves f at 0 there
             f = v3(0.f);
         scale = f / bp;
@@ -255,7 +282,10 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
         const V3 off = dot(wi, sd.f.N) >= 0.f ? sd.f.N : -sd.f.N;
         cur = Ray3{hp + off * PRR_EPS, wi};
         from = kPending;
+        if constexpr (SYNC)
+            run = true;
     }
+#undef PRR_PATH_END
     if (!finite3(L))
         return v3(0.f);
     return L;

@@ -51,7 +51,17 @@ __device__ __forceinline__ void count_rays(unsigned long long *rays, const PathC
     }
 }
 
-__global__ void __launch_bounds__(kTileW *kTileH) k_render_plain(DevScene S, RenderArgs a) {
+// SYNC: blocks of 16x24 pixels whose warps start each path segment together
+// (cast_ray); a slice's samples are as many for every pixel, so all threads
+// make the same calls. 384 threads at 80 registers, 2 blocks per SM: 128, 256
+// and 512 threads gave 1.91, 1.63 and 1.44 ms on the Cornell box, 512 less than
+// 384 on every other scene.
+constexpr int kSyncTileH = 24;
+constexpr int kSyncDepth = 9; // levels of the deepest mesh it is used for
+
+template <bool SYNC>
+__global__ void __launch_bounds__(kTileW *(SYNC ? kSyncTileH : kTileH))
+    k_render_plain(DevScene S, RenderArgs a) {
     extern __shared__ uint2 smem[];
     SmemStack tst{smem + threadIdx.x, (int) blockDim.x, 0, S.tlas_depth + 1, S.check};
     SmemStack bst{smem + (size_t) a.tlas_cap * blockDim.x + threadIdx.x, (int) blockDim.x, 0,
@@ -59,10 +69,10 @@ __global__ void __launch_bounds__(kTileW *kTileH) k_render_plain(DevScene S, Ren
     const int tiles_x = (a.ww + kTileW - 1) / kTileW;
     const int tile = blockIdx.x;
     const int lx = (tile % tiles_x) * kTileW + (int) (threadIdx.x % kTileW);
-    const int ly = (tile / tiles_x) * kTileH + (int) (threadIdx.x / kTileW);
+    const int ly = (tile / tiles_x) * (SYNC ? kSyncTileH : kTileH) + (int) (threadIdx.x / kTileW);
     const bool active = lx < a.ww && ly < a.wh;
     PathCounters cnt{0, 0};
-    if (active) {
+    if (SYNC || active) {
         const int i = a.x0 + lx, j = a.y0 + ly;
         const uint32_t m = (uint32_t) i + (uint32_t) j * (uint32_t) a.W;
         const int q = lx + ly * a.ww;
@@ -76,12 +86,13 @@ __global__ void __launch_bounds__(kTileW *kTileH) k_render_plain(DevScene S, Ren
             const float xo = rng.next();
             const float yo = rng.next();
             const Ray3 ray = generate_ray(S.camera, i, j, xo, yo, rng);
-            V3 s = cast_ray(S, ray, a.max_depth, a.clamp, rng, tst, bst, cnt);
+            V3 s = cast_ray<SYNC>(S, ray, a.max_depth, a.clamp, rng, tst, bst, cnt, active);
             if (isnan(s.x) || isnan(s.y) || isnan(s.z))
                 s = v3(0.f);
             acc = acc + s;
         }
-        a.partial[(size_t) slice * a.ww * a.wh + q] = make_float3(acc.x, acc.y, acc.z);
+        if (active)
+            a.partial[(size_t) slice * a.ww * a.wh + q] = make_float3(acc.x, acc.y, acc.z);
     }
     count_rays(a.rays, cnt);
 }
@@ -149,6 +160,32 @@ __global__ void k_render_resolve(const float3 *__restrict__ partial, int npix, i
         spp_out[q] = n;
 }
 
+// Launches k_render_plain over the window and its slices. Blocks that keep their
+// warps together pay on scenes of small meshes, with enough blocks to go round:
+// 480x270, 16 spp, on museum-like scenes of 480 triangles 6.1 -> 5.5 ms (6
+// levels a mesh), 1,920 triangles 6.4 -> 6.1 (8), but 7,680 triangles 7.1 -> 7.2
+// (10), 30,720 triangles 7.8 -> 8.3 (12); Cornell box 256x256 2.06 -> 1.44, and
+// 61x47, 3 spp, 0.163 -> 0.202. Their stacks are three times a small block's.
+int launch_plain(const DevScene &S, const RenderArgs &a, cudaStream_t st) {
+    const auto blocks = [&](int h) {
+        return (int64_t) ((a.ww + kTileW - 1) / kTileW) * ((a.wh + h - 1) / h) * a.slices;
+    };
+    const auto stacks = [&](int h) {
+        return (size_t) (a.tlas_cap + S.blas_depth + 1) * kTileW * h * sizeof(uint2);
+    };
+    const bool sync = S.blas_depth <= kSyncDepth && stacks(kSyncTileH) <= 96 * 1024 &&
+                      blocks(kSyncTileH) >= 2 * device_sm_count();
+    const int h = sync ? kSyncTileH : kTileH;
+    const size_t smem = stacks(h);
+    auto kern = sync ? k_render_plain<true> : k_render_plain<false>;
+    if (smem > 48 * 1024)
+        PRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int) smem));
+    kern<<<dim3((unsigned) (blocks(h) / a.slices), a.slices), kTileW * h, smem, st>>>(S, a);
+    PRR_CUDA_TRY(cudaGetLastError());
+    return PRR_OK;
+}
+
 } // namespace
 
 int render_plain(Scene &s, const prr_render_settings &rs, float *out_rgb, int32_t *out_spp,
@@ -197,15 +234,16 @@ int render_plain(Scene &s, const prr_render_settings &rs, float *out_rgb, int32_
     }
     if (out_rays)
         PRR_CUDA_TRY(cudaMemsetAsync(out_rays, 0, 2 * sizeof(unsigned long long), st));
-    const int tiles = ((a.ww + kTileW - 1) / kTileW) * ((a.wh + kTileH - 1) / kTileH);
-    const void *fn = adaptive ? (const void *) k_render_adaptive : (const void *) k_render_plain;
-    if (smem > 48 * 1024)
-        PRR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    if (adaptive)
+    if (adaptive) {
+        const int tiles = ((a.ww + kTileW - 1) / kTileW) * ((a.wh + kTileH - 1) / kTileH);
+        if (smem > 48 * 1024)
+            PRR_CUDA_TRY(cudaFuncSetAttribute(
+                k_render_adaptive, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
         k_render_adaptive<<<tiles, kTileW * kTileH, smem, st>>>(S, a);
-    else
-        k_render_plain<<<dim3(tiles, slices), kTileW * kTileH, smem, st>>>(S, a);
-    PRR_CUDA_TRY(cudaGetLastError());
+        PRR_CUDA_TRY(cudaGetLastError());
+    } else if (int rc = launch_plain(S, a, st)) {
+        return rc;
+    }
     k_render_resolve<<<(npix + 255) / 256, 256, 0, st>>>(a.partial, npix, slices,
                                                           adaptive ? a.spp_out : nullptr,
                                                           rs.max_spp, out_rgb, out_spp);
@@ -336,12 +374,8 @@ extern "C" int prr_render_noalloc(prr_scene *scene, const prr_render_settings *s
     std::lock_guard<std::mutex> g(s.mu);
     if (out_rays)
         PRR_CUDA_TRY(cudaMemsetAsync(out_rays, 0, 2 * sizeof(uint64_t), st));
-    if (smem > 48 * 1024)
-        PRR_CUDA_TRY(cudaFuncSetAttribute(k_render_plain,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    const int tiles = ((ww + kTileW - 1) / kTileW) * ((wh + kTileH - 1) / kTileH);
-    k_render_plain<<<dim3(tiles, slices), kTileW * kTileH, smem, st>>>(S, a);
-    PRR_CUDA_TRY(cudaGetLastError());
+    if (int rc = launch_plain(S, a, st))
+        return rc;
     k_render_resolve<<<(int) ((npix + 255) / 256), 256, 0, st>>>(partial, (int) npix, slices,
                                                                   nullptr, rs.max_spp, out_rgb,
                                                                   nullptr);

@@ -821,6 +821,12 @@ __device__ __forceinline__ bool sphere_hit(const DevObject &s, const RayD &r, fl
     return true;
 }
 
+// sphere_hit called out of line, for walks inlined in a kernel that waits on
+// instruction fetch: its double-precision steps are long and rarely run.
+static __device__ __noinline__ bool sphere_hit_ool(const DevObject &s, const RayD &r, float &t) {
+    return sphere_hit(s, r, t);
+}
+
 struct SceneHit {
     int obj;      // object index, -1 on a miss
     int tri;      // global leaf-order triangle index (meshes), -1 for spheres
@@ -830,7 +836,7 @@ struct SceneHit {
 // Scene::intersect -> BVHAccel::Intersect, general path (BVH.cpp:359-369):
 // every scene-BVH leaf object is intersected on its own (meshes start their
 // own search at +inf) and replaces the winner when tnear < closestT.
-template <bool COUNT = false>
+template <bool COUNT = false, bool OOL = false>
 __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD &r,
                                                   const RayPre &p, SmemStack &tst,
                                                   SmemStack &bst, WalkCounts *wc = nullptr) {
@@ -885,7 +891,7 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD 
                 }
             } else {
                 float t;
-                if (sphere_hit(o, r, t) && t < closest) {
+                if ((OOL ? sphere_hit_ool(o, r, t) : sphere_hit(o, r, t)) && t < closest) {
                     closest = t;
                     h.obj = k;
                     h.tri = -1;
@@ -910,7 +916,7 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene &S, const RayD 
 // occluder (Triangle.hpp:141-147) and Sphere falls back to
 // Object::intersectT (Object.hpp:24-29); the caller then requires
 // t >= 0 && t < tMax.
-template <bool COUNT = false>
+template <bool COUNT = false, bool OOL = false>
 __device__ __forceinline__ bool scene_occluded(const DevScene &S, const RayD &r,
                                                const RayPre &p, SmemStack &tst, SmemStack &bst,
                                                float tmax, WalkCounts *wc = nullptr) {
@@ -950,7 +956,7 @@ __device__ __forceinline__ bool scene_occluded(const DevScene &S, const RayD &r,
                       (1e-3f < tmax);
             } else {
                 float t;
-                occ = sphere_hit(o, r, t) && t < tmax && t >= 0.f;
+                occ = (OOL ? sphere_hit_ool(o, r, t) : sphere_hit(o, r, t)) && t < tmax && t >= 0.f;
             }
             if (occ) {
                 tst.sp = sp0;
