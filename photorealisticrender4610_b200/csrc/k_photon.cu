@@ -783,7 +783,29 @@ constexpr int kMaxK = 64;
 // Caustic render: per (pixel, sample), follow the camera ray through the
 // specular chain as castRay does (Integrator.cpp:143-169) and, at the first
 // non-delta hit, estimate the caustic radiance baseColor/pi * E(x).
+// Division of n < 2^31 by a fixed d >= 1: with s = ceil(log2 d) and m =
+// ceil(2^(31 + s) / d) < 2^32, n / d = (n m) >> (31 + s) (Granlund and
+// Montgomery 1994, theorem 4.2 for 31-bit n: m d - 2^(31 + s) < d <= 2^s). The
+// sample kernel's two divisions per item (one of them in 64 bits) were 3% of it.
+struct FastDiv {
+    uint32_t d = 1, m = 0, shift = 0; // m = 0: division by 1
+    FastDiv() = default;
+    explicit FastDiv(uint32_t by) : d(by) {
+        uint32_t s = 0;
+        while ((uint64_t(1) << s) < by)
+            s++;
+        if (s > 0) {
+            m = (uint32_t) (((uint64_t(1) << (31 + s)) + by - 1) / by);
+            shift = s - 1;
+        }
+    }
+    __device__ __forceinline__ uint32_t div(uint32_t n) const {
+        return m ? __umulhi(n, m) >> shift : n;
+    }
+};
+
 struct CausticArgs {
+    FastDiv by_npix, by_ww;
     int W, x0, y0, ww, wh, spp, max_depth, k_nearest, tlas_cap;
     uint64_t seed;
     int sample_offset;
@@ -1207,10 +1229,11 @@ __global__ void __launch_bounds__(128, 8) k_caustic_samples(DevScene S, GridView
         const int64_t t = (int64_t) base + lane;
         if (t >= total)
             continue;
-        const int nc = (int) (t / npix);
-        const int q = (int) (t - (int64_t) nc * npix);
-        const int n = a.s0 + nc;
-        const int i = a.x0 + q % a.ww, j = a.y0 + q / a.ww;
+        const uint32_t nc = a.by_npix.div((uint32_t) t); // t < kCausticItems, or one sample
+        const uint32_t q = (uint32_t) t - nc * a.by_npix.d;
+        const int n = a.s0 + (int) nc;
+        const uint32_t row = a.by_ww.div(q);
+        const int i = a.x0 + (int) (q - row * a.by_ww.d), j = a.y0 + (int) row;
         const uint32_t m = (uint32_t) i + (uint32_t) j * (uint32_t) a.W;
         Rng rng{path_state(a.seed, m, (uint32_t) (a.sample_offset + n))};
         const float xo = rng.next();
@@ -1222,7 +1245,7 @@ __global__ void __launch_bounds__(128, 8) k_caustic_samples(DevScene S, GridView
         for (int d = 0; d < a.max_depth; d++) {
             tst.sp = 0;
             bst.sp = 0;
-            const Inter in = intersect(S, ray, tst, bst);
+            const Inter in = intersect<true>(S, ray, tst, bst);
             if (!in.hit)
                 break;
             if constexpr (COUNT)
@@ -1373,6 +1396,8 @@ int render_caustics(const prr_scene *scene, const prr_photon_map *pmap,
     a.sample_offset = rs.sample_offset;
     a.out = out_rgb;
     a.stats = stats;
+    a.by_npix = FastDiv((uint32_t) (a.ww * a.wh));
+    a.by_ww = FastDiv((uint32_t) a.ww);
     a.tlas_cap = s.dev.tlas_depth + 1;
     const int block = 128;
     const size_t smem = (size_t) (a.tlas_cap + s.dev.blas_depth + 1) * block * sizeof(uint2);

@@ -420,3 +420,18 @@ def test_knn_gather_against_restatement(port, cuda, n, k, radius):
     got = prr.PhotonMap().set(rec).build(radius).gather(q, k_nearest=k).cpu().numpy()
     want, inside = port.photon_estimate_knn(rec, radius, q, k)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("size", [(61, 37), (64, 32), (1, 130), (97, 1)])
+def test_caustic_windows(cuda, size):
+    """The caustic render numbers its (sample, pixel) items by division: any
+    window of any size gives the full image's pixels."""
+    w, h = size
+    s = prr.Scene.from_desc(scenes.caustics(w, h, level=2))
+    pm = prr.PhotonMap().emit(s, 50_000, seed=1).build(0.05)
+    full = pm.render_caustics(s, 3, k_nearest=16).cpu().numpy()
+    assert full.shape == (h, w, 3)
+    for x0, y0, x1, y1 in [(0, 0, 1, 1), (w // 3, h // 3, w, h), (0, h // 2, (w + 1) // 2, h)]:
+        part = pm.render_caustics(s, 3, k_nearest=16, window=(x0, y0, x1, y1)).cpu().numpy()
+        assert np.array_equal(part.view(np.uint32),
+                              np.ascontiguousarray(full[y0:y1, x0:x1]).view(np.uint32))
