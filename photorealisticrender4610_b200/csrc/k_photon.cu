@@ -805,12 +805,12 @@ struct FastDiv {
 };
 
 struct CausticArgs {
-    FastDiv by_npix, by_ww;
+    FastDiv by_chunk, by_ww;
     int W, x0, y0, ww, wh, spp, max_depth, k_nearest, tlas_cap;
     uint64_t seed;
     int sample_offset;
     float *out;
-    float4 *samples; // npix x chunk contributions, sample-major
+    float4 *samples; // npix x chunk contributions, a pixel's in a row
     float4 *acc;     // npix running sums across chunks
     int s0, chunk;   // this launch's samples [s0, s0 + chunk) of each pixel
     unsigned long long *stats; // counting variant: camera hits, gathers, photons
@@ -1198,9 +1198,13 @@ __global__ void __launch_bounds__(128) k_caustic_dense(GridView v, CausticArgs a
 }
 
 // One (pixel, sample) item per thread at a time: sample n of window pixel q is
-// item n * npix + q, so a warp's lanes trace neighbouring pixels; its result
-// goes to slot n * npix + q, so the image does not depend on which thread
-// took which item. Held to 64 registers (8 resident blocks of 128 instead of
+// item q * chunk + n, so a warp's lanes trace samples of the same or the next
+// pixels: they meet the same surfaces and gather from the same cells (the
+// kernel issues in 77% of its cycles, so lanes that part cost most; a warp of
+// one sample of 32 pixels: 1024x1024, 32 spp, 2M photons, k = 64, frame 3.50
+// ms, 3.16 in this order). Its
+// result goes to the slot of the item's number, so the image does not depend
+// on which thread took which item. Held to 64 registers (8 resident blocks of 128 instead of
 // 7; the in-place k-nearest arrays live in local memory either way).
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 8) k_caustic_samples(DevScene S, GridView v, CausticArgs a) {
@@ -1229,8 +1233,8 @@ __global__ void __launch_bounds__(128, 8) k_caustic_samples(DevScene S, GridView
         const int64_t t = (int64_t) base + lane;
         if (t >= total)
             continue;
-        const uint32_t nc = a.by_npix.div((uint32_t) t); // t < kCausticItems, or one sample
-        const uint32_t q = (uint32_t) t - nc * a.by_npix.d;
+        const uint32_t q = a.by_chunk.div((uint32_t) t); // t < kCausticItems, or one sample
+        const uint32_t nc = (uint32_t) t - q * a.by_chunk.d;
         const int n = a.s0 + (int) nc;
         const uint32_t row = a.by_ww.div(q);
         const int i = a.x0 + (int) (q - row * a.by_ww.d), j = a.y0 + (int) row;
@@ -1316,20 +1320,49 @@ __global__ void __launch_bounds__(128, 8) k_caustic_samples(DevScene S, GridView
 // the chunks before (a sample without a diffuse hit adds zero, which leaves
 // the non-negative sum unchanged), so the image is the one a per-pixel loop
 // over its samples produces; the last chunk writes the mean.
-__global__ void k_caustic_film(CausticArgs a) {
+//
+// A pixel's contributions lie in a row. Warps bring them in eight at a time
+// for 32 pixels, 128 contiguous bytes a pixel, and turn them in shared memory
+// (rows of nine: no bank conflicts); short rows are read by their own thread.
+constexpr int kFilmBlock = 128, kFilmTile = 8;
+__global__ void __launch_bounds__(kFilmBlock) k_caustic_film(CausticArgs a) {
+    __shared__ float4 stage[kFilmBlock / 32][32][kFilmTile + 1];
     const int64_t npix = (int64_t) a.ww * a.wh;
     const int64_t q = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix)
+    const int lane = threadIdx.x & 31;
+    const int64_t q0 = q - lane; // the warp's first pixel
+    if (q0 >= npix)
         return;
+    const bool mine = q < npix;
     V3 acc = v3(0.f);
-    if (a.s0 > 0) {
+    if (a.s0 > 0 && mine) {
         const float4 p = a.acc[q];
         acc = v3(p.x, p.y, p.z);
     }
-    for (int n = 0; n < a.chunk; n++) {
-        const float4 c = a.samples[(int64_t) n * npix + q];
-        acc = acc + v3(c.x, c.y, c.z);
+    if (a.chunk < kFilmTile) {
+        for (int n = 0; mine && n < a.chunk; n++) {
+            const float4 c = a.samples[q * a.chunk + n];
+            acc = acc + v3(c.x, c.y, c.z);
+        }
+    } else {
+        float4(*tile)[kFilmTile + 1] = stage[threadIdx.x >> 5];
+        const int n_in = lane % kFilmTile, q_in = lane / kFilmTile;
+        for (int n0 = 0; n0 < a.chunk; n0 += kFilmTile) {
+#pragma unroll
+            for (int r = 0; r < 32; r += 32 / kFilmTile)
+                if (q0 + r + q_in < npix && n0 + n_in < a.chunk)
+                    tile[r + q_in][n_in] = a.samples[(q0 + r + q_in) * a.chunk + n0 + n_in];
+            __syncwarp();
+            if (mine)
+                for (int n = 0; n < min(kFilmTile, a.chunk - n0); n++) {
+                    const float4 c = tile[lane][n];
+                    acc = acc + v3(c.x, c.y, c.z);
+                }
+            __syncwarp();
+        }
     }
+    if (!mine)
+        return;
     if (a.s0 + a.chunk < a.spp) {
         a.acc[q] = make_float4(acc.x, acc.y, acc.z, 0.f);
         return;
@@ -1396,7 +1429,6 @@ int render_caustics(const prr_scene *scene, const prr_photon_map *pmap,
     a.sample_offset = rs.sample_offset;
     a.out = out_rgb;
     a.stats = stats;
-    a.by_npix = FastDiv((uint32_t) (a.ww * a.wh));
     a.by_ww = FastDiv((uint32_t) a.ww);
     a.tlas_cap = s.dev.tlas_depth + 1;
     const int block = 128;
@@ -1440,6 +1472,7 @@ int render_caustics(const prr_scene *scene, const prr_photon_map *pmap,
     for (int s0 = 0; s0 < a.spp && e == cudaSuccess; s0 += chunk) {
         a.s0 = s0;
         a.chunk = std::min(chunk, a.spp - s0);
+        a.by_chunk = FastDiv((uint32_t) a.chunk);
         const int64_t total = npix * a.chunk;
         const int64_t grid = std::min<int64_t>((total + block - 1) / block,
                                                (int64_t) device_sm_count() * std::max(1, bps));
@@ -1456,7 +1489,8 @@ int render_caustics(const prr_scene *scene, const prr_photon_map *pmap,
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
-            k_caustic_film<<<(unsigned) ((npix + 255) / 256), 256, 0, st>>>(a);
+            k_caustic_film<<<(unsigned) ((npix + kFilmBlock - 1) / kFilmBlock), kFilmBlock, 0, st>>>(
+                a);
             pm.launches++;
             e = cudaGetLastError();
         }

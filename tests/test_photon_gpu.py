@@ -435,3 +435,23 @@ def test_caustic_windows(cuda, size):
         part = pm.render_caustics(s, 3, k_nearest=16, window=(x0, y0, x1, y1)).cpu().numpy()
         assert np.array_equal(part.view(np.uint32),
                               np.ascontiguousarray(full[y0:y1, x0:x1]).view(np.uint32))
+
+
+@pytest.mark.parametrize("spp", [1, 2, 7, 8, 9, 33])
+def test_caustic_film_of_any_sample_count(cuda, spp):
+    """A pixel's samples lie in a row and its sum takes them in order: every
+    sample count gives the float32 sum of the one-sample images, bit for bit."""
+    import ctypes as C
+    from photorealisticrender4610_b200._lib import check
+    s = prr.Scene.from_desc(scenes.caustics(45, 7, level=2))
+    pm = prr.PhotonMap().emit(s, 50_000, seed=1).build(0.05)
+    got = pm.render_caustics(s, spp, k_nearest=16).cpu().numpy()
+    acc = np.zeros((7, 45, 3), np.float32)
+    for n in range(spp):
+        rs = s._settings(1, 8, 1, None, 0.05, "plain", None, 10.0, n, 0)
+        one = torch.empty(7, 45, 3, dtype=torch.float32, device="cuda")
+        check(s.lib.prr_render_caustics(s.h, pm.h, C.byref(rs), 16, C.c_void_p(one.data_ptr()),
+                                        None))
+        torch.cuda.synchronize()
+        acc += one.cpu().numpy()
+    assert np.array_equal(got.view(np.uint32), (acc / np.float32(spp)).view(np.uint32))
