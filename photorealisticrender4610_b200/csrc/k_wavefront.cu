@@ -254,6 +254,14 @@ __device__ __forceinline__ void finish(const Wf &w, int p, V3 L) {
     w.result[p] = make_float4(L.x, L.y, L.z, 0.f);
 }
 
+// The paths of a pass: a pixel's samples in a row, pixel after pixel, so the 32
+// paths a warp starts share one or two pixels, and after a bounce, sorted by
+// octant, they still leave from the same surfaces: fewer nodes, triangles and
+// texels per warp than with one sample of 32 pixels (museum-like 960x540, 16
+// spp 12.12 -> 11.66 ms; adaptive 320x180, up to 64 spp, 6.30 -> 5.95; eight
+// served frames 9.77 -> 9.29). The film stages then read a pixel's samples
+// from a row each; that is 0.2% of the frame either way.
+//
 // Window pixel q in path order: tiles of 8x4 pixels (narrower at the right
 // edge, lower at the bottom), row by row of tiles, so a warp's 32 paths start
 // in a small square instead of a long row and stay closer together (1% on
@@ -287,23 +295,24 @@ template <bool MULTI> __global__ void k_wf_generate(DevScene S, Wf w) {
         if constexpr (MULTI) {
             const int r = find_req(w.reqs, w.n_reqs, p, false);
             const WfReq &R = w.reqs[r];
-            const int64_t o = p - R.path_base;
-            const int q = (int) (o % R.npix);
+            const int o = (int) (p - R.path_base);
+            const int q = o / R.nspp;
             tile_pixel(q, R.ww, R.wh, i, j);
             i += R.x0;
             j += R.y0;
             m = (uint32_t) i + (uint32_t) j * (uint32_t) R.W;
-            sample = (uint32_t) (R.s0 + o / R.npix);
+            sample = (uint32_t) (R.s0 + (o - q * R.nspp));
             seed = R.seed;
             cam = &R.camera;
             w.req[p] = r;
         } else {
-            const int q = w.adaptive ? w.act[p % nq] : p % w.npix;
+            const int a = p / w.spp_pass;
+            const int q = w.adaptive ? w.act[a] : a;
             tile_pixel(q, w.ww, w.wh, i, j);
             i += w.x0;
             j += w.y0;
             m = (uint32_t) i + (uint32_t) j * (uint32_t) w.W;
-            sample = (uint32_t) (w.sample_offset + base + p / nq);
+            sample = (uint32_t) (w.sample_offset + base + (p - a * w.spp_pass));
             seed = w.seed;
             cam = &S.camera;
         }
@@ -1165,7 +1174,7 @@ __global__ void k_wf_film_adaptive(Wf w) {
         float3 f = w.film[q];
         bool done = false;
         for (int k = 0; k < w.spp_pass && !done; k++) {
-            float4 r = w.result[(size_t) k * na + a];
+            float4 r = w.result[(size_t) a * w.spp_pass + k];
             if (isnan(r.x) || isnan(r.y) || isnan(r.z))
                 r = make_float4(0.f, 0.f, 0.f, 0.f);
             f.x += r.x;
@@ -1236,7 +1245,7 @@ __global__ void k_wf_film_multi(Wf w, int64_t total_pixels) {
         float3 &film = R.film[(size_t) y * R.ww + x]; // row order
         float3 f = film;
         for (int s = 0; s < R.nspp; s++) {
-            const float4 v = w.result[R.path_base + (int64_t) s * R.npix + q];
+            const float4 v = w.result[R.path_base + (int64_t) q * R.nspp + s];
             if (!(isnan(v.x) || isnan(v.y) || isnan(v.z))) {
                 f.x += v.x;
                 f.y += v.y;
@@ -1252,7 +1261,7 @@ __global__ void k_wf_film(Wf w) {
     if (q < w.npix) {
         float3 f = w.film[q];
         for (int s = 0; s < w.spp_pass; s++) {
-            const float4 r = w.result[(size_t) s * w.npix + q];
+            const float4 r = w.result[(size_t) q * w.spp_pass + s];
             // a NaN sample is zeroed before accumulation (Renderer.cpp:78-83)
             if (!(isnan(r.x) || isnan(r.y) || isnan(r.z))) {
                 f.x += r.x;

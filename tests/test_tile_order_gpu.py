@@ -25,3 +25,17 @@ def test_ragged_windows(cuda, window):
     out = torch.empty_like(a)
     srv.wait(srv.submit(srv.add_scene(s), 6, 4, seed=3, window=window, out=out))
     assert np.array_equal(a.cpu().numpy().view(np.uint32), out.cpu().numpy().view(np.uint32))
+
+
+@pytest.mark.parametrize("spp, paths", [(1, 0), (5, 0), (32, 0), (33, 0), (12, 3 * 37 * 21),
+                                        (7, 1)])
+def test_samples_of_a_pixel_in_a_row(cuda, spp, paths):
+    """A pixel's samples are neighbouring paths, in one pass or several: the
+    film is the plain renderer's, fixed and adaptive."""
+    s = prr.Scene.from_desc(scenes.cornell_box(37, 21))
+    s.set_wavefront(paths_per_pass=paths)
+    for kw in (dict(), dict(min_spp=1, threshold=0.2)):
+        a, na = s.render(spp, 4, seed=5, mode="plain", slices=1, **kw)
+        b, nb = s.render(spp, 4, seed=5, mode="wavefront", **kw)
+        assert np.array_equal(a.cpu().numpy().view(np.uint32), b.cpu().numpy().view(np.uint32))
+        assert torch.equal(na, nb)
