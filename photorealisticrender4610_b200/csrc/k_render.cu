@@ -26,6 +26,7 @@ struct RenderArgs {
     int x0, y0, ww, wh;
     int spp_begin, spp_end; // samples [begin, end) of the fixed mode
     int slices;
+    int group_log2; // slices of a pixel side by side in a warp: 1 << group_log2
     int min_spp, max_spp;
     float threshold;
     int max_depth;
@@ -51,32 +52,46 @@ __device__ __forceinline__ void count_rays(unsigned long long *rays, const PathC
     }
 }
 
+// A block's threads are (1 << tile_w_log2) x tile_h pixels times 1 << group_log2 slices of
+// each, a pixel's slices side by side: its samples leave through the same
+// pixel and meet the same surfaces first.
+__host__ __device__ constexpr int tile_w_log2(int group_log2) {
+    return 4 - (group_log2 + 1) / 2;
+}
+static_assert(kTileW == 1 << tile_w_log2(0));
+__host__ __device__ constexpr int tile_h(int h, int group_log2) { return h >> (group_log2 / 2); }
+
 // SYNC: blocks of 16x24 pixels whose warps start each path segment together
-// (cast_ray); a slice's samples are as many for every pixel, so all threads
-// make the same calls. 384 threads at 80 registers, 2 blocks per SM: 128, 256
+// (cast_ray); the slices of a block have as many samples each (launch_plain), so
+// all threads make the same calls. 384 threads at 80 registers, 2 blocks per SM: 128, 256
 // and 512 threads gave 1.91, 1.63 and 1.44 ms on the Cornell box, 512 less than
 // 384 on every other scene.
 constexpr int kSyncTileH = 24;
 constexpr int kSyncDepth = 9; // levels of the deepest mesh it is used for
 
-template <bool SYNC>
+// GROUP: the slices of a pixel share warps (launch_plain); without it group_log2
+// is 0, known to the compiler (3% on one sample of the Cornell box).
+template <bool SYNC, bool GROUP>
 __global__ void __launch_bounds__(kTileW *(SYNC ? kSyncTileH : kTileH))
     k_render_plain(DevScene S, RenderArgs a) {
     extern __shared__ uint2 smem[];
     SmemStack tst{smem + threadIdx.x, (int) blockDim.x, 0, S.tlas_depth + 1, S.check};
     SmemStack bst{smem + (size_t) a.tlas_cap * blockDim.x + threadIdx.x, (int) blockDim.x, 0,
                   S.blas_depth + 1, S.check};
-    const int tiles_x = (a.ww + kTileW - 1) / kTileW;
+    const int g = GROUP ? a.group_log2 : 0;
+    const int tw_log2 = tile_w_log2(g), th = tile_h(SYNC ? kSyncTileH : kTileH, g);
+    const int tiles_x = (a.ww + (1 << tw_log2) - 1) >> tw_log2;
     const int tile = blockIdx.x;
-    const int lx = (tile % tiles_x) * kTileW + (int) (threadIdx.x % kTileW);
-    const int ly = (tile / tiles_x) * (SYNC ? kSyncTileH : kTileH) + (int) (threadIdx.x / kTileW);
+    const int in_tile = (int) threadIdx.x >> g;
+    const int lx = ((tile % tiles_x) << tw_log2) + (in_tile & ((1 << tw_log2) - 1));
+    const int ly = (tile / tiles_x) * th + (in_tile >> tw_log2);
     const bool active = lx < a.ww && ly < a.wh;
     PathCounters cnt{0, 0};
     if (SYNC || active) {
         const int i = a.x0 + lx, j = a.y0 + ly;
         const uint32_t m = (uint32_t) i + (uint32_t) j * (uint32_t) a.W;
         const int q = lx + ly * a.ww;
-        const int slice = blockIdx.y;
+        const int slice = (int) ((blockIdx.y << g) + (threadIdx.x & ((1u << g) - 1u)));
         const int total = a.spp_end - a.spp_begin;
         const int s0 = a.spp_begin + (int) ((int64_t) total * slice / a.slices);
         const int s1 = a.spp_begin + (int) ((int64_t) total * (slice + 1) / a.slices);
@@ -166,9 +181,21 @@ __global__ void k_render_resolve(const float3 *__restrict__ partial, int npix, i
 // levels a mesh), 1,920 triangles 6.4 -> 6.1 (8), but 7,680 triangles 7.1 -> 7.2
 // (10), 30,720 triangles 7.8 -> 8.3 (12); Cornell box 256x256 2.06 -> 1.44, and
 // 61x47, 3 spp, 0.163 -> 0.202. Their stacks are three times a small block's.
-int launch_plain(const DevScene &S, const RenderArgs &a, cudaStream_t st) {
+//
+// The slices of a pixel go side by side into a warp where every SM has more
+// blocks than it holds at once: 480x270, 16 spp, on museum-like scenes of 480
+// to 491,520 triangles 5.44 -> 4.70, 6.17 -> 5.19, 7.13 -> 6.17, 8.61 -> 7.16,
+// 9.26 -> 7.71 ms; 320x180, 7 spp 2.68 -> 2.24; Cornell box 256x256 1.446 ->
+// 1.407. A single wave is as slow as its slowest warp, and the long paths of a
+// difficult pixel then share one: 97x61, 16 spp 0.72 -> 0.76 ms. Slices of
+// uneven shares would leave threads that keep step idle (Cornell box 640x360,
+// 7 spp in 6 slices 2.13 -> 2.38), so there each stays in its own blocks.
+int launch_plain(const DevScene &S, RenderArgs a, cudaStream_t st) {
+    a.group_log2 = 0;
     const auto blocks = [&](int h) {
-        return (int64_t) ((a.ww + kTileW - 1) / kTileW) * ((a.wh + h - 1) / h) * a.slices;
+        const int tw = 1 << tile_w_log2(a.group_log2), th = tile_h(h, a.group_log2);
+        return (int64_t) ((a.ww + tw - 1) / tw) * ((a.wh + th - 1) / th) *
+               (a.slices >> a.group_log2);
     };
     const auto stacks = [&](int h) {
         return (size_t) (a.tlas_cap + S.blas_depth + 1) * kTileW * h * sizeof(uint2);
@@ -176,12 +203,18 @@ int launch_plain(const DevScene &S, const RenderArgs &a, cudaStream_t st) {
     const bool sync = S.blas_depth <= kSyncDepth && stacks(kSyncTileH) <= 96 * 1024 &&
                       blocks(kSyncTileH) >= 2 * device_sm_count();
     const int h = sync ? kSyncTileH : kTileH;
+    const bool even = (a.spp_end - a.spp_begin) % a.slices == 0;
+    if (blocks(kTileH) >= 8 * device_sm_count() && (even || !sync))
+        while (a.group_log2 < 5 && (a.slices & ((2 << a.group_log2) - 1)) == 0)
+            a.group_log2++;
+    const int groups = a.slices >> a.group_log2;
     const size_t smem = stacks(h);
-    auto kern = sync ? k_render_plain<true> : k_render_plain<false>;
+    auto kern = a.group_log2 ? (sync ? k_render_plain<true, true> : k_render_plain<false, true>)
+                             : (sync ? k_render_plain<true, false> : k_render_plain<false, false>);
     if (smem > 48 * 1024)
         PRR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int) smem));
-    kern<<<dim3((unsigned) (blocks(h) / a.slices), a.slices), kTileW * h, smem, st>>>(S, a);
+    kern<<<dim3((unsigned) (blocks(h) / groups), groups), kTileW * h, smem, st>>>(S, a);
     PRR_CUDA_TRY(cudaGetLastError());
     return PRR_OK;
 }

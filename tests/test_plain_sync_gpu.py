@@ -26,3 +26,27 @@ def test_large_window_equals_small_ones(cuda, make, size):
             part, _ = s.render(8, 6, seed=5, mode="plain", slices=4, window=win)
             assert np.array_equal(part.cpu().numpy().view(np.uint32),
                                   np.ascontiguousarray(whole[y:win[3], x:win[2]]).view(np.uint32))
+
+
+@pytest.mark.parametrize("size, spp, slices", [((161, 121), 16, 16), ((161, 121), 17, 16),
+                                               ((161, 121), 12, 6), ((161, 121), 66, 33),
+                                               ((161, 121), 64, 64), ((321, 203), 6, 4),
+                                               ((1, 4001), 32, 32), ((4001, 1), 32, 8)])
+@pytest.mark.parametrize("small", [True, False])
+def test_slices_side_by_side(cuda, size, spp, slices, small):
+    """A pixel's slices share a warp: the image is the float32 sum, slice after
+    slice, of the slices rendered alone, bit for bit."""
+    w, h = size
+    s = prr.Scene.from_desc(scenes.cornell_box(w, h) if small else
+                            scenes.museum_like(w, h, level=3, env_size=(8, 4)))
+    got, _ = s.render(spp, 3, seed=2, mode="plain", slices=slices)
+    acc = None
+    for k in range(slices):
+        a, b = spp * k // slices, spp * (k + 1) // slices
+        part = np.zeros((h, w, 3), np.float32)
+        for n in range(a, b):
+            one, _ = s.render(1, 3, seed=2, mode="plain", slices=1, sample_offset=n)
+            part = part + one.cpu().numpy()
+        acc = part if acc is None else acc + part
+    want = acc / np.float32(spp)
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
