@@ -239,10 +239,13 @@ __global__ void __maxnreg__(64) k_mesh_closest_refill(const __grid_constant__ Me
 }
 
 // For batches that give each ray a lane of its own: the walk that keeps more
-// loads under way (92 registers, 5 blocks). 10,000 triangles, 4,099 rays 76 ->
-// 67 us, 40,000 rays 157 -> 126; 300,000 triangles, 1,000 rays 196 -> 161,
-// 40,000 rays 340 -> 285.
-__global__ void k_mesh_closest_few(const __grid_constant__ MeshArgs a) {
+// loads under way (90 registers, 5 blocks of 128). 10,000 triangles, 4,099 rays
+// 76 -> 67 us, 40,000 rays 157 -> 126; 300,000 triangles, 1,000 rays 196 -> 161,
+// 40,000 rays 340 -> 285. An SM's registers hold blocks of up to kFewBlock
+// threads of it; larger ones take the form above.
+constexpr int kFewBlock = 640;
+__global__ void __launch_bounds__(kFewBlock)
+    k_mesh_closest_few(const __grid_constant__ MeshArgs a) {
     extern __shared__ uint2 smem[];
     MeshClosest<true> b(a, smem);
     trace_rays(b, a.n, a.c);
@@ -929,13 +932,6 @@ bool capturing(cudaStream_t st) {
 // traced launch after launch on their stream.
 constexpr int64_t kMaxLaunch = int64_t(1) << 31;
 
-// Blocks of a kernel resident per SM (0 blocks_per_sm: what its occupancy is).
-int resident_blocks(const void *fn, int block, size_t smem) {
-    int bps = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, block, smem);
-    return std::max(1, bps);
-}
-
 // Batches traced by the FEW form of a kernel: up to 640 rays per SM, what its
 // residents (5 blocks of 128) hold at once. Closest hit on one mesh takes it up
 // to twice that, its rays being slower apart than the larger batch's queueing
@@ -965,7 +961,12 @@ int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, 
         return fail(PRR_ERR_UNSUPPORTED, "BVH too deep for the shared-memory stack");
     if (int rc = set_smem(fn, L.smem))
         return rc;
-    const int bps = blocks_per_sm > 0 ? blocks_per_sm : resident_blocks(fn, block, L.smem);
+    int bps = 0; // blocks resident per SM
+    PRR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, block, L.smem));
+    if (bps == 0)
+        return fail(PRR_ERR_INTERNAL, "no block of the query kernel fits an SM");
+    if (blocks_per_sm > 0)
+        bps = blocks_per_sm;
     const int64_t resident = (int64_t) device_sm_count() * bps;
     const int64_t warps = resident * (block / 32);
     c.share = (uint32_t) ((n + warps - 1) / warps);
@@ -1032,7 +1033,7 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     // allocate nothing; every other call gets its own
     if (in_capture && mode > 0 && !counter)
         counter = (unsigned *) s.d_counter.ptr;
-    const bool few = mode == 0 && few_rays(n, 1280);
+    const bool few = mode == 0 && block <= kFewBlock && few_rays(n, 1280);
     const void *fn = mode == 1   ? (const void *) k_mesh_closest_persistent
                      : mode == 3 ? (const void *) k_mesh_closest_phased
                      : few         ? (const void *) k_mesh_closest_few
