@@ -43,12 +43,19 @@ __device__ double tri_t64(const float *__restrict__ v, const RayD &r) {
 // What every query kernel needs besides its rays and outputs.
 struct TraceCfg {
     unsigned *counter;           // next ray to hand out (nullptr: fixed shares)
-    void *spill;                 // global part of the stacks
+    void *spill;                 // global part of the stacks (nullptr: local_stack serves)
     uint32_t share;              // rays of a warp's share: n over the grid's warps
     int lanes;                   // lanes of a warp that take rays: share, at most 32
     int refill;                  // idle lanes that trigger a refill (at most lanes)
     int stack_sm, stack_cap;     // stack entries: in shared memory, in all
 };
+
+// Stack entries of a thread's own local memory, beyond those in shared memory:
+// enough for a four-wide walk of any tree whose binary walk's stack (one entry
+// per level) fits where kStackSm shared entries do, without a buffer that
+// captured calls, whose replays may overlap, would have to share.
+constexpr int kLocalStack = 24;
+template <class E> using QueryStack = StackCol<E, kLocalStack>;
 
 struct MeshArgs {
     const QNode *nodes;
@@ -144,7 +151,7 @@ __device__ __forceinline__ void trace_rays(Body &b, uint32_t n, const TraceCfg &
 // asks for the children it pushes.
 template <bool FEW> struct MeshClosest {
     const MeshArgs &a;
-    const StackCol<uint2> col;
+    const QueryStack<uint2> col;
     uint32_t idx = 0;
     RayD r;
     RayPair p;
@@ -153,8 +160,8 @@ template <bool FEW> struct MeshClosest {
     uint32_t ref = 0; // next node, or the leaf triangles left to test (a leaf reference)
     uint32_t top = 0;
 
-    __device__ __forceinline__ MeshClosest(const MeshArgs &args, uint2 *smem)
-        : a(args), col(smem, (uint2 *) args.c.spill, args.c.stack_sm, args.c.stack_cap,
+    __device__ __forceinline__ MeshClosest(const MeshArgs &args, uint2 *smem, uint2 *own)
+        : a(args), col(smem, (uint2 *) args.c.spill, own, args.c.stack_sm, args.c.stack_cap,
                        args.B.check) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
@@ -234,12 +241,13 @@ template <bool FEW> struct MeshClosest {
 // against 3.09 for one ray per thread over the binary nodes.
 __global__ void __maxnreg__(64) k_mesh_closest_refill(const __grid_constant__ MeshArgs a) {
     extern __shared__ uint2 smem[];
-    MeshClosest<false> b(a, smem);
+    uint2 own[kLocalStack];
+    MeshClosest<false> b(a, smem, own);
     trace_rays(b, a.n, a.c);
 }
 
 // For batches that give each ray a lane of its own: the walk that keeps more
-// loads under way (90 registers, 5 blocks of 128). 10,000 triangles, 4,099 rays
+// loads under way (96 registers, 5 blocks of 128). 10,000 triangles, 4,099 rays
 // 76 -> 67 us, 40,000 rays 157 -> 126; 300,000 triangles, 1,000 rays 196 -> 161,
 // 40,000 rays 340 -> 285. An SM's registers hold blocks of up to kFewBlock
 // threads of it; larger ones take the form above.
@@ -247,15 +255,23 @@ constexpr int kFewBlock = 640;
 __global__ void __launch_bounds__(kFewBlock)
     k_mesh_closest_few(const __grid_constant__ MeshArgs a) {
     extern __shared__ uint2 smem[];
-    MeshClosest<true> b(a, smem);
+    uint2 own[kLocalStack];
+    MeshClosest<true> b(a, smem, own);
     trace_rays(b, a.n, a.c);
 }
 
 // Persistent: each warp takes the next 32 rays from the counter until none
-// are left. The counter is zeroed on the stream before the launch.
-__global__ void k_mesh_closest_persistent(MeshArgs a) {
+// are left. The counter is zeroed on the stream before the launch. 55 registers
+// (61 without the bound), so the 9 blocks of 128 that the stacks leave room for:
+// 4,194,304 rays on 10,000, 300,000 and 1,000,000 triangles 4.08, 7.65 and 5.64
+// ms; whole stacks in shared memory 3.94, 7.44 and 5.76, but 30 and 34 entries
+// are more than blocks of 1,024 have room for.
+__global__ void __maxnreg__(56)
+    k_mesh_closest_persistent(const __grid_constant__ MeshArgs a) {
     extern __shared__ uint2 smem[];
-    SmemStack st{smem + threadIdx.x, (int) blockDim.x, 0, a.c.stack_cap, a.B.check};
+    uint2 own[kLocalStack];
+    const QueryStack<uint2> st(smem, (uint2 *) a.c.spill, own, a.c.stack_sm, a.c.stack_cap,
+                               a.B.check);
     const int lane = threadIdx.x & 31;
     for (;;) {
         uint32_t base = 0;
@@ -291,9 +307,12 @@ __global__ void k_mesh_closest_persistent(MeshArgs a) {
 
 constexpr uint32_t kNoRef = 0xFFFFFFFFu;
 
-__global__ void __maxnreg__(64) k_mesh_closest_phased(MeshArgs a, int refill, int tri_min) {
+__global__ void __maxnreg__(64)
+    k_mesh_closest_phased(const __grid_constant__ MeshArgs a, int refill, int tri_min) {
     extern __shared__ uint2 smem[];
-    const StackCol<uint2> col(smem, (uint2 *) a.c.spill, a.c.stack_sm, a.c.stack_cap, a.B.check);
+    uint2 own[kLocalStack];
+    const QueryStack<uint2> col(smem, (uint2 *) a.c.spill, own, a.c.stack_sm, a.c.stack_cap,
+                                a.B.check);
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     int64_t idx = -1;
@@ -392,7 +411,7 @@ template <bool FEW> struct MeshAny {
     const float *tmaxs;
     uint8_t *out;
     const float *box; // the mesh's root box
-    const StackCol<uint32_t> col;
+    const QueryStack<uint32_t> col;
     uint32_t idx = 0;
     RayD r;
     RayPair p;
@@ -402,9 +421,11 @@ template <bool FEW> struct MeshAny {
     bool occluded = false;
 
     __device__ __forceinline__ MeshAny(const MeshArgs &args, const float *root_box,
-                                       const float *tmax_, uint8_t *hit, uint32_t *smem)
+                                       const float *tmax_, uint8_t *hit, uint32_t *smem,
+                                       uint32_t *own)
         : a(args), tmaxs(tmax_), out(hit), box(root_box),
-          col(smem, (uint32_t *) args.c.spill, args.c.stack_sm, args.c.stack_cap, args.B.check) {}
+          col(smem, (uint32_t *) args.c.spill, own, args.c.stack_sm, args.c.stack_cap,
+              args.B.check) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
@@ -474,7 +495,8 @@ __global__ void __maxnreg__(FEW ? 128 : 64) k_mesh_occluded(const __grid_constan
                                                 const __grid_constant__ MeshBox box,
                                                 const float *tmax, uint8_t *out) {
     extern __shared__ uint32_t smem32[];
-    MeshAny<FEW> b(a, box.b, tmax, out, smem32);
+    uint32_t own[kLocalStack];
+    MeshAny<FEW> b(a, box.b, tmax, out, smem32, own);
     trace_rays(b, a.n, a.c);
 }
 
@@ -485,9 +507,10 @@ struct SceneArgs {
     TraceCfg c;
 };
 
-template <class E> __device__ __forceinline__ StackCol<E> scene_col(const DevScene &S,
-                                                                    const TraceCfg &c, E *smem) {
-    return StackCol<E>(smem, (E *) c.spill, c.stack_sm, c.stack_cap, S.check);
+template <class E>
+__device__ __forceinline__ QueryStack<E> scene_col(const DevScene &S, const TraceCfg &c, E *smem,
+                                                   E *own) {
+    return QueryStack<E>(smem, (E *) c.spill, own, c.stack_sm, c.stack_cap, S.check);
 }
 
 // 2,000,003 rays on 122,880 triangles with geometry, half of them incoherent:
@@ -498,15 +521,15 @@ template <bool FEW> struct SceneClosest {
     int32_t *out_obj, *out_prim;
     float *out_t;
     bool raw; // out_prim takes the leaf-order triangle index (k_scene_finish resolves it)
-    const StackCol<uint2> col;
+    const QueryStack<uint2> col;
     uint32_t idx = 0;
     ClosestWalk<FEW> w;
 
     __device__ __forceinline__ SceneClosest(const DevScene &scene, const SceneArgs &args,
                                             int32_t *obj, int32_t *prim, float *t, bool leaf_order,
-                                            uint2 *smem)
+                                            uint2 *smem, uint2 *own)
         : S(scene), a(args), out_obj(obj), out_prim(prim), out_t(t), raw(leaf_order),
-          col(scene_col(scene, args.c, smem)) {}
+          col(scene_col(scene, args.c, smem, own)) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
@@ -531,7 +554,8 @@ __global__ void __maxnreg__(FEW ? 128 : 64)
     k_scene_closest(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
                     int32_t *out_obj, int32_t *out_prim, float *out_t, bool raw) {
     extern __shared__ uint2 smem[];
-    SceneClosest<FEW> b(S, a, out_obj, out_prim, out_t, raw, smem);
+    uint2 own[kLocalStack];
+    SceneClosest<FEW> b(S, a, out_obj, out_prim, out_t, raw, smem, own);
     trace_rays(b, a.n, a.c);
 }
 
@@ -604,13 +628,14 @@ template <bool FEW> struct SceneAny {
     const SceneArgs &a;
     const float *tmaxs;
     uint8_t *out;
-    const StackCol<uint32_t> col;
+    const QueryStack<uint32_t> col;
     uint32_t idx = 0;
     AnyWalk<FEW> w;
 
     __device__ __forceinline__ SceneAny(const DevScene &scene, const SceneArgs &args,
-                                        const float *tmax, uint8_t *hit, uint32_t *smem)
-        : S(scene), a(args), tmaxs(tmax), out(hit), col(scene_col(scene, args.c, smem)) {}
+                                        const float *tmax, uint8_t *hit, uint32_t *smem,
+                                        uint32_t *own)
+        : S(scene), a(args), tmaxs(tmax), out(hit), col(scene_col(scene, args.c, smem, own)) {}
 
     __device__ __forceinline__ bool start(uint32_t i) {
         idx = i;
@@ -628,7 +653,8 @@ __global__ void __maxnreg__(FEW ? 128 : 64)
     k_scene_occluded(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
                      const float *tmax, uint8_t *out) {
     extern __shared__ uint32_t smem32[];
-    SceneAny<FEW> b(S, a, tmax, out, smem32);
+    uint32_t own[kLocalStack];
+    SceneAny<FEW> b(S, a, tmax, out, smem32, own);
     trace_rays(b, a.n, a.c);
 }
 
@@ -894,10 +920,12 @@ int device_sm_count() {
 
 namespace {
 
-// Mesh-stack entries a query kernel keeps in shared memory: 9 blocks of 128
+// Stack entries a query kernel keeps in shared memory: 9 blocks of 128
 // threads, what its registers allow, fill an SM's shared memory at 24 entries
-// of 8 bytes. Deeper entries go to a per-call global buffer.
+// of 8 bytes. Deeper entries go to local memory, or, where kLocalStack are too
+// few, to a per-call global buffer.
 constexpr int kStackSm = 24;
+constexpr size_t kMaxSmem = 227 * 1024; // shared memory of a block at most
 
 // Device scratch of one call, from the library's stream-ordered pool and given
 // back on the stream: concurrent calls on other streams get their own.
@@ -918,7 +946,8 @@ struct CallScratch {
 };
 
 // True while the stream is being captured into a graph: such calls allocate
-// nothing and keep no counter, as a replayed graph may overlap other calls.
+// nothing and keep no counter, as a replayed graph may overlap other calls. The
+// entries of a stack that local memory does not hold are then all shared.
 bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
@@ -953,11 +982,14 @@ int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, 
                int64_t n, int blocks_per_sm, int refill, bool counter_always,
                unsigned *counter, bool in_capture, cudaStream_t st) {
     c.stack_cap = cap;
-    c.stack_sm = in_capture ? cap : std::min(cap, kStackSm);
+    c.stack_sm = std::min(cap, kStackSm);
+    if (in_capture)
+        c.stack_sm = std::max(c.stack_sm, cap - kLocalStack);
+    const bool local = cap - c.stack_sm <= kLocalStack;
     c.counter = nullptr;
     c.spill = nullptr;
     L.smem = (size_t) c.stack_sm * block * entry;
-    if (L.smem > 227 * 1024)
+    if (L.smem > kMaxSmem)
         return fail(PRR_ERR_UNSUPPORTED, "BVH too deep for the shared-memory stack");
     if (int rc = set_smem(fn, L.smem))
         return rc;
@@ -977,12 +1009,12 @@ int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, 
     const bool count = counter_always || (n > warps * 32 && !in_capture);
     size_t bytes = count && !counter ? 256 : 0;
     const size_t spill_at = bytes;
-    if (cap > c.stack_sm)
+    if (!local)
         bytes += (size_t) (cap - c.stack_sm) * L.grid * block * entry;
     if (bytes)
         if (int rc = L.scratch.alloc(bytes, st))
             return rc;
-    if (cap > c.stack_sm)
+    if (!local)
         c.spill = L.scratch.ptr + spill_at;
     if (count) {
         c.counter = counter ? counter : (unsigned *) L.scratch.ptr;
@@ -1034,17 +1066,16 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     if (in_capture && mode > 0 && !counter)
         counter = (unsigned *) s.d_counter.ptr;
     const bool few = mode == 0 && block <= kFewBlock && few_rays(n, 1280);
+    const int cap = stack_cap(obj.qstack);
     const void *fn = mode == 1   ? (const void *) k_mesh_closest_persistent
                      : mode == 3 ? (const void *) k_mesh_closest_phased
-                     : few         ? (const void *) k_mesh_closest_few
+                     : few       ? (const void *) k_mesh_closest_few
                                  : (const void *) k_mesh_closest_refill;
     const int refill = mode >= 2 && cfg->batch > 0 ? std::min(cfg->batch, 32) : 8;
-    const int cap = stack_cap(obj.qstack);
     TraceLaunch L;
-    // mode 1 keeps its whole stack in shared memory
     if (int rc = plan_trace(L, a.c, fn, block, cap, sizeof(uint2), n,
                             mode > 0 ? cfg->blocks_per_sm : 0, refill, mode > 0, counter,
-                            in_capture || mode == 1, st))
+                            in_capture, st))
         return rc;
     CallScratch order;
     if (sort > 0 && n < (int64_t(1) << 31)) {

@@ -366,8 +366,8 @@ __device__ __forceinline__ int lanes_used(int n) {
 // This thread's stack: tlas_cap + blas_sm entries in shared memory, the rest in
 // the spill buffer.
 template <class E> __device__ __forceinline__ StackCol<E> path_stack(const Wf &w, E *smem) {
-    return StackCol<E>(smem, (E *) w.spill, w.tlas_cap + w.blas_sm, w.tlas_cap + w.blas_cap,
-                       w.check);
+    return StackCol<E>(smem, (E *) w.spill, nullptr, w.tlas_cap + w.blas_sm,
+                       w.tlas_cap + w.blas_cap, w.check);
 }
 
 template <bool MULTI>

@@ -497,26 +497,33 @@ __device__ __forceinline__ void lds(uint32_t a, uint32_t &v) {
 // Per-thread stack with a bounded shared-memory part. A position is the byte
 // address `top` of the next free entry of the thread's shared-memory column
 // (step bytes apart, [entry][thread], so a warp's pushes hit distinct banks);
-// positions at `limit` and beyond stand for entries of a global buffer laid
-// out [entry - cap][grid thread], so a warp's spills are coalesced. The bound
-// on a walk's entries is found when its tree is packed; the global part is
+// positions at `limit` and beyond stand for entries of a buffer that lies
+// outside: LOCAL entries of the thread's local memory, or, where those are too
+// few (or none, LOCAL = 0), a global buffer laid out [entry - cap][grid thread].
+// A warp's spills are coalesced in both. The bound
+// on a walk's entries is found when its tree is packed; the outer part is
 // only reached deep in unbalanced subtrees and stays in L1/L2, and the code
 // for it sits behind one comparison per step. Fewer shared entries leave more
 // of the SM's L1 for node and triangle fetches and let more blocks be
 // resident.
-template <class E> struct StackCol {
+template <class E, int LOCAL = 0> struct StackCol {
     uint32_t base, step, limit;
-    E *gl;
+    E *gl;                   // global part (LOCAL > 0: nullptr where `local` serves)
+    E *local = nullptr;      // LOCAL entries of the thread's own
     int total = 1 << 30;     // entries in both parts (tested by the checked build)
     uint32_t *check = nullptr;
-    __device__ __forceinline__ StackCol(E *sm, E *global, int cap, int total_, uint32_t *check_)
+    __device__ __forceinline__ StackCol(E *sm, E *global, E *own, int cap, int total_,
+                                        uint32_t *check_)
         : base((uint32_t) __cvta_generic_to_shared(sm) + threadIdx.x * (uint32_t) sizeof(E)),
-          step(blockDim.x * (uint32_t) sizeof(E)), gl(global), total(total_), check(check_) {
+          step(blockDim.x * (uint32_t) sizeof(E)), gl(global), local(own), total(total_),
+          check(check_) {
         limit = base + (uint32_t) cap * step;
     }
     __device__ __forceinline__ E *spill_at(uint32_t top) const {
-        return gl + (size_t) ((top - limit) / step) * (gridDim.x * blockDim.x) +
-               blockIdx.x * blockDim.x + threadIdx.x;
+        const size_t k = (top - limit) / step;
+        if (LOCAL > 0 && !gl)
+            return local + k;
+        return gl + k * (gridDim.x * blockDim.x) + blockIdx.x * blockDim.x + threadIdx.x;
     }
     __device__ __forceinline__ bool ok(uint32_t top) const {
 #ifdef PRR_CHECKED
@@ -562,7 +569,8 @@ template <class E> struct StackCol {
 
 // Push a node's entered children but the first (closest hit: with their entry
 // distances; any hit: references alone).
-__device__ __forceinline__ void push_rest(const StackCol<uint2> &st, uint32_t &top,
+template <int LOCAL>
+__device__ __forceinline__ void push_rest(const StackCol<uint2, LOCAL> &st, uint32_t &top,
                                           const QuadOrder &q, float best) {
     if (st.room3(top))
         q.rest(best, [&](uint32_t c, float t) {
@@ -573,7 +581,8 @@ __device__ __forceinline__ void push_rest(const StackCol<uint2> &st, uint32_t &t
             st.put(top, make_uint2(c, __float_as_uint(t)));
         });
 }
-__device__ __forceinline__ void push_rest(const StackCol<uint32_t> &st, uint32_t &top,
+template <int LOCAL>
+__device__ __forceinline__ void push_rest(const StackCol<uint32_t, LOCAL> &st, uint32_t &top,
                                           const QuadOrder &q, float tmax) {
     if (st.room3(top))
         q.rest(tmax, [&](uint32_t c, float) { st.put_sm(top, c); });
@@ -623,21 +632,23 @@ struct WalkCounts {
 // four-wide nodes. best_t enters as +inf (every mesh-level search starts
 // fresh, BVH.cpp:331). Returns the winning triangle's global leaf-order index,
 // or -1.
+template <int LOCAL>
 __device__ __forceinline__ int blas_closest_quad(const QNode *__restrict__ nodes,
-                                            const Tri *__restrict__ tris,
-                                            const float *__restrict__ e2z, uint32_t root,
-                                            const RayD &r, const RayPre &p, SmemStack &st,
-                                            float &best_t, float &best_u, float &best_v,
-                                            const TraceBounds &B) {
+                                                 const Tri *__restrict__ tris,
+                                                 const float *__restrict__ e2z, uint32_t root,
+                                                 const RayD &r, const RayPre &p,
+                                                 const StackCol<uint2, LOCAL> &st, float &best_t,
+                                                 float &best_u, float &best_v,
+                                                 const TraceBounds &B) {
     if (!(root & kLeafBit) && no_slab(p))
         return -1;
-    const int sp0 = st.sp;
+    uint32_t top = st.base;
     uint32_t ref = root;
     int hit = -1;
     for (;;) {
         if (!(ref & kLeafBit)) {
             const QuadOrder q = quad_order(load_quad(nodes, ref, B), p);
-            q.rest(best_t, [&](uint32_t c, float t) { st.push(c, t); });
+            push_rest(st, top, q, best_t);
             if (q.any(best_t)) {
                 ref = q.next(best_t);
                 continue;
@@ -658,9 +669,9 @@ __device__ __forceinline__ int blas_closest_quad(const QNode *__restrict__ nodes
         }
         // pop the next entry whose box is still nearer than the closest hit
         for (;;) {
-            if (st.sp == sp0)
+            if (st.empty(top))
                 return hit;
-            const uint2 e = st.pop();
+            const uint2 e = st.pop(top);
             if (__uint_as_float(e.y) < best_t) {
                 ref = e.x;
                 break;

@@ -35,8 +35,9 @@ template <bool FEW = false> struct ClosestWalk {
     uint32_t top, floor;
 
     // false when the ray is over at once (a miss)
+    template <int LOCAL>
     __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray,
-                                          const StackCol<uint2> &st) {
+                                          const StackCol<uint2, LOCAL> &st) {
         r = ray;
         p = precompute(ray);
         best = closest = kInf;
@@ -76,7 +77,8 @@ template <bool FEW = false> struct ClosestWalk {
     }
 
     // one unit of work; true when the walk is over
-    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint2> &st) {
+    template <int LOCAL>
+    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint2, LOCAL> &st) {
         bool down = false;
         uint32_t x = 0;
         if (FEW && (ref & kLeafBit)) {
@@ -155,8 +157,9 @@ template <bool FEW = false> struct AnyWalk {
     bool in_mesh, occluded;
 
     // false when the walk is over at once (nothing in the way, or a sphere)
+    template <int LOCAL>
     __device__ __forceinline__ bool start(const DevScene &S, const RayD &ray, float t_max,
-                                          const StackCol<uint32_t> &st) {
+                                          const StackCol<uint32_t, LOCAL> &st) {
         r = ray;
         p = precompute_pair(ray);
         tmax = t_max;
@@ -191,7 +194,8 @@ template <bool FEW = false> struct AnyWalk {
     }
 
     // one unit of work; true when the walk is over (result in `occluded`)
-    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint32_t> &st) {
+    template <int LOCAL>
+    __device__ __forceinline__ bool step(const DevScene &S, const StackCol<uint32_t, LOCAL> &st) {
         bool down = false;
         uint32_t x = 0;
         if (FEW && (ref & kLeafBit)) {

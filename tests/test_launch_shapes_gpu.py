@@ -27,3 +27,79 @@ def test_default_mode_block_sizes(port, cuda, block, rays):
     got = s.mesh_intersect(0, torch.from_numpy(o).to(cuda), torch.from_numpy(d).to(cuda),
                            config={"block_size": block})
     equal(got, port.mesh(v).intersect(o, d))
+
+
+def captured(fn):
+    """fn's outputs as a replayed CUDA graph leaves them."""
+    fn()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = fn()
+    for x in out:
+        x.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    return out
+
+
+MODES = [{}, {"persistent": 1}, {"persistent": 2}, {"persistent": 3}]
+
+
+@pytest.mark.parametrize("rays", [5_000, 200_000])
+def test_largest_blocks_on_a_large_mesh(port, cuda, rays):
+    """300,000 triangles: 21 entries for the binary walk's stack, about 30 for
+    the four-wide one's, of which a block of 1,024 has shared memory for 28."""
+    v, o, d = scenes.query_set(300_000, rays, seed=4)
+    want = port.mesh(v).intersect(o, d)
+    s = prr.Scene.single_mesh(v)
+    to, td = torch.from_numpy(o).to(cuda), torch.from_numpy(d).to(cuda)
+    for cfg in MODES:
+        cfg = {**cfg, "block_size": 1024}
+        equal(s.mesh_intersect(0, to, td, config=cfg), want)
+        equal(captured(lambda: s.mesh_intersect(0, to, td, config=cfg)), want)
+
+
+def spiral(base, n):
+    """Triangles growing geometrically: a deep, one-sided tree."""
+    x = base ** np.arange(n) * 1e-3
+    v = np.zeros((n, 9))
+    for a in range(3):
+        v[:, 3 * a] = x * (1 + 0.01 * a)
+        if a:
+            v[:, 3 * a + a] = x * 0.01
+    return v.astype(np.float32)
+
+
+@pytest.mark.parametrize("base, n", [(1.5, 60), (1.4, 100), (1.3, 150), (1.2, 260), (1.15, 600)])
+def test_stacks_beyond_shared_memory(cuda, base, n):
+    """Trees of more levels than a block's share of shared memory holds, and
+    rays that enter every box (a component without a bound on each axis but
+    one): all modes and block sizes agree, captured or not."""
+    verts = spiral(base, n)
+    s = prr.Scene.single_mesh(verts)
+    rng = np.random.default_rng(n)
+    tri = verts.reshape(-1, 3, 3)[rng.integers(0, n, 4000)]
+    target = (tri * rng.dirichlet([1, 1, 1], 4000)[:, :, None]).sum(1)
+    o = np.where(rng.random((4000, 1)) < 0.5, -target, target * 0.5)
+    d = target - o
+    d = d / np.linalg.norm(d, axis=1, keepdims=True)
+    d[::8] = [np.inf, np.nan, 1.0]
+    to = torch.from_numpy(o.astype(np.float32)).to(cuda)
+    td = torch.from_numpy(d.astype(np.float32)).to(cuda)
+    tm = torch.full((4000,), np.inf, device=cuda)
+    hid, t = s.mesh_intersect(0, to, td)
+    want = (hid.cpu().numpy(), t.cpu().numpy())
+    assert (want[0] >= 0).sum() > 200
+    for cfg in MODES:
+        for block in (32, 128, 256):
+            cfg = {**cfg, "block_size": block}
+            equal(s.mesh_intersect(0, to, td, config=cfg), want)
+            equal(captured(lambda: s.mesh_intersect(0, to, td, config=cfg)), want)
+    ob, prim, st = s.intersect(to, td)
+    equal((prim, st), want)
+    equal(captured(lambda: s.intersect(to, td)[1:]), want)
+    for fn in (lambda: s.mesh_occluded(0, to, td, tm), lambda: s.intersectP(to, td, tm)):
+        occ = fn().cpu().numpy() > 0
+        assert np.array_equal(occ, want[0] >= 0)
+        assert np.array_equal(captured(lambda: (fn(),))[0].cpu().numpy() > 0, occ)
