@@ -60,7 +60,7 @@ struct Wf {
     float clamp;
     uint64_t seed;
     int tlas_cap, blas_cap; // stack entries a walk may need at the scene and mesh level
-    int blas_sm;            // mesh-stack entries kept in shared memory
+    int stack_sm;           // entries of the two kept in shared memory
     int count_stack;        // binary-walk entries of the counting variants, both levels
     void *spill;            // global part of the stacks ([entry][grid thread])
     // path state
@@ -363,11 +363,11 @@ __device__ __forceinline__ int lanes_used(int n) {
 // ---- extend: closest hit of the queued rays, then sort by material class.
 // Persistent: a lane whose ray is finished takes the next queued ray once
 // `refill` lanes of its warp are idle (one atomic per refill).
-// This thread's stack: tlas_cap + blas_sm entries in shared memory, the rest in
-// the spill buffer.
+// This thread's stack: stack_sm entries in shared memory, the rest in the spill
+// buffer.
 template <class E> __device__ __forceinline__ StackCol<E> path_stack(const Wf &w, E *smem) {
-    return StackCol<E>(smem, (E *) w.spill, nullptr, w.tlas_cap + w.blas_sm,
-                       w.tlas_cap + w.blas_cap, w.check);
+    return StackCol<E>(smem, (E *) w.spill, nullptr, w.stack_sm, w.tlas_cap + w.blas_cap,
+                       w.check);
 }
 
 template <bool MULTI>
@@ -1397,16 +1397,14 @@ template <bool MULTI>
 int wf_shape(Wf &w, int block_req, int stack_req, int refill_req, WfShape &L) {
     const int sms = device_sm_count();
     L.block = block_req > 0 ? block_req : 128;
-    // Stacks: the scene-level one wholly in shared memory, the mesh one up to
-    // stack_req entries (0: all of it) within 96 KB per block; its deeper
-    // entries go to the global spill buffer.
+    // Stacks: the entries of both levels lie in one. The scene's and the mesh's up
+    // to stack_req (0: all of them) are kept in shared memory, within 96 KB per
+    // block; deeper ones go to the global spill buffer.
     const int max_sm_entries = (96 * 1024) / (L.block * (int) sizeof(uint2));
-    if (w.tlas_cap + 1 > max_sm_entries)
-        return fail(PRR_ERR_UNSUPPORTED, "scene BVH too deep for the shared-memory stack");
-    w.blas_sm = stack_req > 0 ? std::min(stack_req, w.blas_cap) : w.blas_cap;
-    w.blas_sm = std::max(1, std::min(w.blas_sm, max_sm_entries - w.tlas_cap));
-    L.smem_ext = (size_t) (w.tlas_cap + w.blas_sm) * L.block * sizeof(uint2);
-    L.smem_sh = (size_t) (w.tlas_cap + w.blas_sm) * L.block * sizeof(uint32_t);
+    const int blas_sm = stack_req > 0 ? std::min(stack_req, w.blas_cap) : w.blas_cap;
+    w.stack_sm = std::min(w.tlas_cap + blas_sm, max_sm_entries);
+    L.smem_ext = (size_t) w.stack_sm * L.block * sizeof(uint2);
+    L.smem_sh = (size_t) w.stack_sm * L.block * sizeof(uint32_t);
     L.ext = k_wf_extend<MULTI>;
     L.sh = k_wf_shadow<MULTI>;
     if constexpr (!MULTI) {
@@ -1446,7 +1444,7 @@ int wf_shape(Wf &w, int block_req, int stack_req, int refill_req, WfShape &L) {
                                                   L.smem_sh);
     L.g_ext = sms * std::max(1, occ_ext);
     L.g_sh = sms * std::max(1, occ_sh);
-    const size_t spill_entries = (size_t) (w.blas_cap - w.blas_sm);
+    const size_t spill_entries = (size_t) (w.tlas_cap + w.blas_cap - w.stack_sm);
     L.spill_bytes =
         spill_entries * std::max((size_t) L.g_ext * L.block * sizeof(uint2),
                                  (size_t) L.g_sh * L.block * sizeof(uint32_t));
@@ -1622,7 +1620,7 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     uint64_t key = (uint64_t) (uintptr_t) s.d_wavefront.ptr;
     key = mix64(key ^ ((uint64_t) w.P << 20) ^ ((uint64_t) w.max_depth << 8) ^
                 (uint64_t) L.block ^ ((uint64_t) L.refill << 50));
-    key = mix64(key ^ (uint64_t) (uintptr_t) w.spill ^ ((uint64_t) w.blas_sm << 32) ^
+    key = mix64(key ^ (uint64_t) (uintptr_t) w.spill ^ ((uint64_t) w.stack_sm << 32) ^
                 ((uint64_t) w.ordered << 60));
     key = mix64(key ^ ((uint64_t) w.adaptive << 7) ^ ((uint64_t) w.min_spp << 24) ^
                 ((uint64_t) float_bits(w.threshold) << 28) ^ (uint64_t) w.max_spp);

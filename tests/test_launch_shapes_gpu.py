@@ -103,3 +103,28 @@ def test_stacks_beyond_shared_memory(cuda, base, n):
         occ = fn().cpu().numpy() > 0
         assert np.array_equal(occ, want[0] >= 0)
         assert np.array_equal(captured(lambda: (fn(),))[0].cpu().numpy() > 0, occ)
+
+
+def clutter(objects, size):
+    """Many small meshes: a scene tree of 17 levels for 20,000."""
+    rng = np.random.default_rng(1)
+    desc = scenes.SceneDesc(width=size, height=size, name="clutter")
+    m = desc.add_material(scenes.Material(scenes.DIFFUSE, (0.7, 0.6, 0.5), 0.6, 0.0))
+    c = rng.uniform(0, 1, (objects, 1, 3))
+    for tri in (c + rng.normal(0, 0.01, (objects, 6, 3))).astype(np.float32).reshape(-1, 2, 9):
+        desc.objects.append(scenes.MeshObject(tri, m))
+    desc.background = (0.3, 0.5, 0.8)
+    desc.camera = scenes.Camera(eye=(2.2, 1.6, 2.4), target=(0.5, 0.5, 0.5), fovv=40, fovh=45)
+    return desc
+
+
+def test_wavefront_blocks_on_a_deep_scene_tree(cuda):
+    """The scene level's entries alone exceed the 24 a block of 512 has shared
+    memory for: they spill as the mesh level's do."""
+    s = prr.Scene.from_desc(clutter(20_000, 64))
+    assert s.stats()["tlas_depth"] >= 16
+    want, spp = s.render(2, 4, mode="plain")
+    for block, stack in ((512, 0), (512, 8), (512, 1), (256, 0), (64, 8)):
+        s.set_wavefront(block_size=block, stack_smem=stack)
+        got, n = s.render(2, 4, mode="wavefront")
+        assert torch.equal(got, want) and torch.equal(n, spp), (block, stack)
