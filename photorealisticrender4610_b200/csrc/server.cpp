@@ -63,7 +63,9 @@ struct Server {
     std::vector<Scene *> scenes;
     std::vector<size_t> scene_bytes;
     DevBuf d_scenes; // DevScene per scene
-    int tlas_cap = 1, blas_cap = 1;
+    // stack entries a walk may need, largest over the scenes: of the binary nodes
+    // (megakernel steps) and of the four-wide ones (wavefront steps)
+    int tlas_cap = 1, blas_cap = 1, quad_tlas_cap = 1, quad_blas_cap = 1;
 
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
@@ -300,8 +302,8 @@ int run_step_wavefront(Server &S) {
     const double t0 = now_s();
     int64_t launches = 0;
     if (int rc = wavefront_step_multi(S.wf, S.wf_reqs.data(), (int) S.wf_reqs.size(),
-                                      S.cfg.paths_per_launch, S.tlas_cap, S.blas_cap, S.p_rays,
-                                      S.st, &launches))
+                                      S.cfg.paths_per_launch, S.quad_tlas_cap, S.quad_blas_cap,
+                                      S.p_rays, S.st, &launches))
         return rc;
     PRR_CUDA_TRY(cudaStreamSynchronize(S.st));
     S.busy += now_s() - t0;
@@ -525,8 +527,10 @@ int prr_server_add_scene(prr_server *server, prr_scene *scene, int *out_id) {
     S.scenes.push_back(&sc);
     S.scene_bytes.push_back(sc.device_bytes);
     S.used += sc.device_bytes;
-    S.tlas_cap = std::max(S.tlas_cap, std::max(sc.dev.tlas_depth, sc.dev.tlas_stack) + 1);
-    S.blas_cap = std::max(S.blas_cap, std::max(sc.dev.blas_depth, sc.dev.blas_stack) + 1);
+    S.tlas_cap = std::max(S.tlas_cap, sc.dev.tlas_depth + 1);
+    S.blas_cap = std::max(S.blas_cap, sc.dev.blas_depth + 1);
+    S.quad_tlas_cap = std::max(S.quad_tlas_cap, sc.dev.tlas_stack + 1);
+    S.quad_blas_cap = std::max(S.quad_blas_cap, sc.dev.blas_stack + 1);
     std::vector<DevScene> all;
     for (Scene *p : S.scenes)
         all.push_back(p->dev);
