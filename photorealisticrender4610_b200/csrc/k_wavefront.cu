@@ -1296,12 +1296,6 @@ __global__ void k_wf_rays_out(const unsigned *cnt, unsigned long long *out) {
     out[1] = *reinterpret_cast<const unsigned long long *>(cnt + kCntShadowRays);
 }
 
-uint32_t float_bits(float f) {
-    uint32_t u;
-    std::memcpy(&u, &f, sizeof(u));
-    return u;
-}
-
 template <class T> T *carve(char *&p, size_t n) {
     T *r = reinterpret_cast<T *>(p);
     p += (n * sizeof(T) + 255) & ~size_t(255);
@@ -1310,17 +1304,21 @@ template <class T> T *carve(char *&p, size_t n) {
 
 } // namespace
 
+// One captured pass and everything it was captured with: the kernels' arguments
+// and launch shapes, byte for byte.
 struct WavefrontPlan {
-    // one captured pass per (scene, window, spp_pass, depth, block shape)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    uint64_t key = 0;
-    ~WavefrontPlan() {
+    std::vector<unsigned char> inputs;
+    void release() {
         if (exec)
             cudaGraphExecDestroy(exec);
         if (graph)
             cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
     }
+    ~WavefrontPlan() { release(); }
 };
 
 namespace {
@@ -1546,7 +1544,10 @@ int wf_enqueue_bounces(const DevScene &S, const Wf &w, const WfShape &L, const W
 int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, int32_t *out_spp,
                      unsigned long long *out_rays, cudaStream_t st) {
     const DevScene &S = s.dev;
-    Wf w{};
+    Wf w;
+    WfShape L;
+    std::memset(&w, 0, sizeof(w)); // padding too: the bytes are compared (WavefrontPlan)
+    std::memset(&L, 0, sizeof(L));
     w.W = s.width;
     w.x0 = rs.x0;
     w.y0 = rs.y0;
@@ -1567,7 +1568,6 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     w.threshold = rs.variance_threshold;
     w.stats = s.wf_stats;
     w.check = S.check;
-    WfShape L{};
     // Paths per pass: whole samples of the window, by default at most 32M in
     // flight (10 GB of path state): every bounce of a pass ends in a tail of
     // long rays, so fewer and larger passes pay it less often (museum-like
@@ -1617,30 +1617,18 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
         return PRR_OK;
     };
     const int passes = rs.max_spp / spp_pass;
-    uint64_t key = (uint64_t) (uintptr_t) s.d_wavefront.ptr;
-    key = mix64(key ^ ((uint64_t) w.P << 20) ^ ((uint64_t) w.max_depth << 8) ^
-                (uint64_t) L.block ^ ((uint64_t) L.refill << 50));
-    key = mix64(key ^ (uint64_t) (uintptr_t) w.spill ^ ((uint64_t) w.stack_sm << 32) ^
-                ((uint64_t) w.ordered << 60));
-    key = mix64(key ^ ((uint64_t) w.adaptive << 7) ^ ((uint64_t) w.min_spp << 24) ^
-                ((uint64_t) float_bits(w.threshold) << 28) ^ (uint64_t) w.max_spp);
-    key = mix64(key ^ ((uint64_t) (uint32_t) w.x0 << 32 | (uint32_t) w.y0) ^
-                ((uint64_t) (uint32_t) w.ww << 16) ^ (uint64_t) (uint32_t) w.wh ^ rs.seed ^
-                ((uint64_t) rs.sample_offset << 40) ^
-                (uint64_t) float_bits(w.clamp));
     if (!s.wf_plan)
         s.wf_plan = std::make_shared<WavefrontPlan>();
     WavefrontPlan &plan = *s.wf_plan;
     if (s.wf_graphs && passes > 1 && !w.stats) {
-        if (plan.key != key || !plan.exec) {
-            if (plan.exec) {
-                cudaGraphExecDestroy(plan.exec);
-                plan.exec = nullptr;
-            }
-            if (plan.graph) {
-                cudaGraphDestroy(plan.graph);
-                plan.graph = nullptr;
-            }
+        // the scene (its background may change after the build), the window, seed
+        // and sampling, the buffers, the launch shapes
+        std::vector<unsigned char> inputs(sizeof(S) + sizeof(w) + sizeof(L));
+        std::memcpy(inputs.data(), &S, sizeof(S));
+        std::memcpy(inputs.data() + sizeof(S), &w, sizeof(w));
+        std::memcpy(inputs.data() + sizeof(S) + sizeof(w), &L, sizeof(L));
+        if (!plan.exec || plan.inputs != inputs) {
+            plan.release();
             cudaStream_t cap;
             PRR_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
             PRR_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
@@ -1654,7 +1642,7 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
                 return fail(PRR_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
             plan.graph = g;
             PRR_CUDA_TRY(cudaGraphInstantiate(&plan.exec, g, 0));
-            plan.key = key;
+            plan.inputs = std::move(inputs);
         }
         for (int k = 0; k < passes; k++)
             PRR_CUDA_TRY(cudaGraphLaunch(plan.exec, st));
