@@ -992,7 +992,17 @@ struct PartSpec {
     int concat;
     int count_slot[8];  // counter slot receiving bucket b's size (-1: none)
     int total_slot;     // counter slot receiving the total (-1: none)
+    int from[2];        // counters of the items that may carry a tag (-1: none is kept)
 };
+
+// No item carries a tag: a bounce without paths (the passes after an adaptive
+// frame's last pixel has stopped, the last bounces of most passes), whose
+// partitions then leave the P tags unread. 960x540, up to 256 spp, every pixel
+// stopped in the first of 16 passes: 26.0 -> 17.1 ms.
+__device__ __forceinline__ bool part_empty(const Wf &w, const PartSpec &ps) {
+    return ps.from[0] >= 0 && w.cnt[ps.from[0]] == 0 &&
+           (ps.from[1] < 0 || w.cnt[ps.from[1]] == 0);
+}
 
 // How many of the 16 tag bytes in v equal b.
 __device__ __forceinline__ unsigned count_tag(const uint4 &v, unsigned b) {
@@ -1003,6 +1013,8 @@ __device__ __forceinline__ unsigned count_tag(const uint4 &v, unsigned b) {
 
 __global__ void __launch_bounds__(kPartThreads) k_part_count(Wf w, PartSpec ps) {
     stage_begin();
+    if (part_empty(w, ps))
+        return;
     const int nb = ps.nb;
     __shared__ unsigned c[8];
     if (threadIdx.x < 8)
@@ -1025,6 +1037,13 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(Wf w, PartSpec ps) 
 // thread per round. Tile counts become the tiles' first output slots.
 __global__ void __launch_bounds__(1024) k_part_scan(Wf w, int ntiles, PartSpec ps) {
     stage_begin();
+    if (part_empty(w, ps)) {
+        if (threadIdx.x < 8 && ps.count_slot[threadIdx.x] >= 0)
+            w.cnt[ps.count_slot[threadIdx.x]] = 0;
+        if (threadIdx.x == 8 && ps.total_slot >= 0)
+            w.cnt[ps.total_slot] = 0;
+        return;
+    }
     __shared__ unsigned wsum[32][8];
     __shared__ unsigned carry[8];
     __shared__ unsigned total[8];
@@ -1115,6 +1134,8 @@ __global__ void __launch_bounds__(1024) k_part_scan(Wf w, int ntiles, PartSpec p
 
 __global__ void __launch_bounds__(kPartThreads) k_part_scatter(Wf w, PartSpec ps) {
     stage_begin();
+    if (part_empty(w, ps))
+        return;
     __shared__ unsigned wsum[kPartThreads / 32][8];
     __shared__ unsigned base[8][kPartThreads];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1455,22 +1476,27 @@ int wf_shape(Wf &w, int block_req, int stack_req, int refill_req, WfShape &L) {
 
 // The stable partitions of the ordered queues.
 struct WfParts {
-    PartSpec cls, ray[2], act;
+    PartSpec cls[2], ray[2], act; // cls and ray: by the ray queue they read and write
 };
 WfParts wf_parts(const Wf &w) {
     WfParts P;
     // hit classes -> miss / delta / surface queues
-    P.cls = PartSpec{};
-    P.cls.tag = w.tag;
-    P.cls.q[0] = w.qmiss;
-    P.cls.q[1] = w.qdelta;
-    P.cls.q[2] = w.qsurf;
-    P.cls.nb = 3;
-    P.cls.concat = 0;
-    P.cls.count_slot[0] = kCntMiss;
-    P.cls.count_slot[1] = kCntDelta;
-    P.cls.count_slot[2] = kCntSurf;
-    P.cls.total_slot = -1;
+    for (int r = 0; r < 2; r++) {
+        PartSpec &c = P.cls[r] = PartSpec{};
+        c.tag = w.tag;
+        c.q[0] = w.qmiss;
+        c.q[1] = w.qdelta;
+        c.q[2] = w.qsurf;
+        c.nb = 3;
+        c.concat = 0;
+        std::fill(c.count_slot, c.count_slot + 8, -1);
+        c.count_slot[0] = kCntMiss;
+        c.count_slot[1] = kCntDelta;
+        c.count_slot[2] = kCntSurf;
+        c.total_slot = -1;
+        c.from[0] = kCntRay0 + r;
+        c.from[1] = -1;
+    }
     // next rays -> the ray queue, direction octant major
     for (int r = 0; r < 2; r++) {
         P.ray[r] = PartSpec{};
@@ -1481,6 +1507,8 @@ WfParts wf_parts(const Wf &w) {
         for (int b = 0; b < 8; b++)
             P.ray[r].count_slot[b] = -1;
         P.ray[r].total_slot = kCntRay0 + r;
+        P.ray[r].from[0] = kCntDelta;
+        P.ray[r].from[1] = kCntSurf;
     }
     // adaptive: the pixels still active -> the next pass's active list
     P.act = PartSpec{};
@@ -1489,8 +1517,9 @@ WfParts wf_parts(const Wf &w) {
     P.act.q[0] = w.act_next;
     P.act.nb = 1;
     P.act.concat = 1;
-    P.act.count_slot[0] = -1;
+    std::fill(P.act.count_slot, P.act.count_slot + 8, -1);
     P.act.total_slot = kCntActive;
+    P.act.from[0] = P.act.from[1] = -1;
     return P;
 }
 
@@ -1526,7 +1555,7 @@ int wf_enqueue_bounces(const DevScene &S, const Wf &w, const WfShape &L, const W
         launch_stage(k_wf_begin, 1, 32, 0, cs, w, it);
         launch_stage(L.ext, L.g_ext, L.block, L.smem_ext, cs, S, w, it, L.refill);
         if (w.ordered)
-            wf_partition(w, parts.cls, L.ntiles, cs);
+            wf_partition(w, parts.cls[it & 1], L.ntiles, cs);
         launch_stage(k_wf_miss<MULTI>, L.g_shade, 128, 0, cs, S, w);
         launch_stage(k_wf_delta<MULTI>, L.g_shade, 128, 0, cs, S, w, it + 1);
         launch_stage(k_wf_surface<MULTI>, device_sm_count() * 2, kSurfaceBlock, 0, cs, S, w, it + 1);

@@ -22,3 +22,15 @@ def test_adaptive_passes_do_not_grow_with_the_budget(cuda):
     assert launches(s) == 2 + 13 * 3 + 1
     s.render(1024, 2, mode="wavefront", min_spp=1, threshold=1e9)
     assert launches(s) == 4 * (6 + 13 * 3) + 2
+
+
+@pytest.mark.parametrize("ordered", [True, False])
+@pytest.mark.parametrize("threshold", [1e9, 0.5])
+def test_passes_after_the_last_pixel_stopped(cuda, ordered, threshold):
+    """Passes, and bounces of a pass, without paths: image and sample counts are
+    the plain adaptive renderer's."""
+    s = prr.Scene.from_desc(scenes.cornell_box(96, 64))
+    s.set_wavefront(paths_per_pass=96 * 64 * 4, stack_smem=8, ordered=ordered)
+    got, n = s.render(32, 12, mode="wavefront", min_spp=1, threshold=threshold)
+    want, m = s.render(32, 12, mode="plain", min_spp=1, threshold=threshold)
+    assert torch.equal(n, m) and torch.equal(got, want)
