@@ -116,8 +116,9 @@ typedef struct prr_render_settings {
 
 /* Wavefront launch shape (chosen by prr_autotune; zero fields = defaults). */
 typedef struct prr_wavefront_config {
-    int64_t paths_per_pass; /* paths in flight per pass (0: up to 32M, fewer where device
-                               memory is short, 8M for adaptive sampling; at most 2^30; about 320 bytes of device
+    int64_t paths_per_pass; /* paths in flight per pass (0: up to 32M, fewer where they would
+                               take over a quarter of the free device memory, and 8M for
+                               adaptive sampling; at most 2^30; about 320 bytes of device
                                memory each) */
     int block_size;         /* threads per block of the traversal stages (0: 128) */
     int use_graphs;         /* 1: replay each pass from one captured CUDA graph */

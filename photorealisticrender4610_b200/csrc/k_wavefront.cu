@@ -1600,29 +1600,46 @@ int render_wavefront(Scene &s, const prr_render_settings &rs, float *out_rgb, in
     // Paths per pass: whole samples of the window, by default at most 32M in
     // flight (10 GB of path state): every bounce of a pass ends in a tail of
     // long rays, so fewer and larger passes pay it less often.
-    // Where that much memory is not free, half as much, down to 8M.
     // Adaptive renders take 8M: all samples of a pass are traced, also those past
     // a pixel's stop. Museum-like scene at 480x270, up to 256 spp, 8M and 32M: all
     // pixels stopped after one sample 17.2 and 34.9 ms, after 3 20.9 and 35.0,
     // but 56.7 and 49.4 where they take nearly all 256.
     const int64_t kDefaultPaths = (int64_t) 1 << 25, kLeastPaths = (int64_t) 1 << 23;
+    const bool automatic = s.wf_paths <= 0;
+    int64_t target = s.wf_paths;
+    if (automatic)
+        target = w.adaptive ? kLeastPaths : s.wf_fit > 0 ? s.wf_fit : kDefaultPaths;
     int spp_pass = 1;
-    for (int64_t target = s.wf_paths > 0 ? s.wf_paths : w.adaptive ? kLeastPaths : kDefaultPaths;;
-         target >>= 1) {
+    for (;; target >>= 1) {
         spp_pass = (int) std::max<int64_t>(1, target / std::max(1, w.npix));
         spp_pass = std::min(spp_pass, rs.max_spp);
         while (rs.max_spp % spp_pass)
             spp_pass--;
         w.spp_pass = spp_pass;
         w.P = spp_pass * w.npix;
-        int rc = wf_shape<false>(w, s.wf_block, s.wf_stack, s.wf_refill, L);
-        if (rc == PRR_OK)
-            rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix, L.spill_bytes);
+        if (int rc = wf_shape<false>(w, s.wf_block, s.wf_stack, s.wf_refill, L))
+            return rc;
+        // More than the least is taken only where it leaves other users of the
+        // device three quarters of the free memory, looked up when the buffer has
+        // to grow; a smaller size that had to do is kept for the next renders.
+        const bool shrinks = automatic && target > kLeastPaths;
+        const size_t held = s.d_wavefront.bytes;
+        const size_t need = wf_bytes((size_t) w.P, w.npix, L.spill_bytes);
+        if (shrinks && need > held) {
+            size_t free_bytes = 0, total_bytes = 0;
+            PRR_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+            if (need > (free_bytes + held) / 4) {
+                s.wf_fit = target >> 1;
+                continue;
+            }
+        }
+        const int rc = wf_layout(s.d_wavefront, w, (size_t) w.P, w.npix, L.spill_bytes);
         if (rc == PRR_OK)
             break;
-        if (rc != PRR_ERR_OUT_OF_MEMORY || s.wf_paths > 0 || target <= kLeastPaths)
+        if (rc != PRR_ERR_OUT_OF_MEMORY || !shrinks)
             return rc;
         cudaGetLastError(); // the failed allocation
+        s.wf_fit = target >> 1;
     }
     const WfParts parts = wf_parts(w);
 

@@ -125,6 +125,7 @@ struct Scene {
     DevBuf d_wavefront;    // wavefront path state, queues, film and stack spill
     std::shared_ptr<WavefrontPlan> wf_plan; // captured pass graph
     int64_t wf_paths = 0;  // paths in flight per pass (0 = automatic)
+    int64_t wf_fit = 0;    // the automatic pass size that device memory allowed (0 = the largest)
     int wf_block = 0;      // extend / shadow block size (0 = 128)
     int wf_refill = 0;     // idle lanes that trigger a refill (0 = 12)
     bool wf_graphs = true; // replay passes from a captured CUDA graph

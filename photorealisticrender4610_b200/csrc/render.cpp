@@ -117,6 +117,7 @@ extern "C" int prr_scene_set_wavefront(prr_scene *scene, const prr_wavefront_con
     Scene &s = *reinterpret_cast<Scene *>(scene);
     std::lock_guard<std::mutex> g(s.mu);
     s.wf_paths = config->paths_per_pass;
+    s.wf_fit = 0;
     s.wf_block = config->block_size;
     s.wf_graphs = config->use_graphs != 0;
     s.wf_stack = config->stack_smem;

@@ -34,3 +34,29 @@ def test_passes_after_the_last_pixel_stopped(cuda, ordered, threshold):
     got, n = s.render(32, 12, mode="wavefront", min_spp=1, threshold=threshold)
     want, m = s.render(32, 12, mode="plain", min_spp=1, threshold=threshold)
     assert torch.equal(n, m) and torch.equal(got, want)
+
+
+def test_default_pass_leaves_memory_to_others(cuda):
+    """With 24 GB free a frame of 33.5M paths (10.7 GB of path state) is split:
+    no more than a quarter of the free memory is taken, and the image stays."""
+    s = prr.Scene.from_desc(scenes.cornell_box(1024, 1024))
+    want = s.render(32, 2, mode="plain", slices=1)[0]
+    torch.cuda.synchronize()
+    ballast = []
+    try:
+        spare = torch.cuda.mem_get_info()[0] - (24 << 30)
+        while spare > 0:
+            ballast.append(torch.empty(min(spare, 16 << 30), dtype=torch.uint8, device=cuda))
+            spare -= 16 << 30
+        free = torch.cuda.mem_get_info()[0]
+        got = s.render(32, 2, mode="wavefront")[0]
+        torch.cuda.synchronize()
+        taken = free - torch.cuda.mem_get_info()[0]
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    assert taken <= free / 4 + (64 << 20)  # and the image's own block
+    assert launches(s) > 2 + 13 * 3 + 1
+    assert torch.equal(got, want)
+    again = s.render(32, 2, mode="wavefront")[0]
+    assert torch.equal(again, want)
