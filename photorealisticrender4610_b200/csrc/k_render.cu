@@ -68,6 +68,7 @@ __host__ __device__ constexpr int tile_h(int h, int group_log2) { return h >> (g
 // 384 on every other scene.
 constexpr int kSyncTileH = 24;
 constexpr int kSyncDepth = 9; // levels of the deepest mesh it is used for
+constexpr int kSyncSceneDepth = 4; // and of the scene's tree
 
 // GROUP: the slices of a pixel share warps (launch_plain); without it group_log2
 // is 0, known to the compiler (3% on one sample of the Cornell box).
@@ -181,6 +182,13 @@ __global__ void k_render_resolve(const float3 *__restrict__ partial, int npix, i
 // levels a mesh), 1,920 triangles 6.4 -> 6.1 (8), but 7,680 triangles 7.1 -> 7.2
 // (10), 30,720 triangles 7.8 -> 8.3 (12); Cornell box 256x256 2.06 -> 1.44, and
 // 61x47, 3 spp, 0.163 -> 0.202. Their stacks are three times a small block's.
+// The deeper the meshes, the more uneven the walks and the more samples it takes
+// to even them out (m meshes of 12 triangles, 3 levels, apart / in step: m = 4,
+// 97x61, 16 spp 0.28 / 0.33 ms, 256x256, 16 spp 0.79 / 0.76; museum-like, 8
+// levels, 320x180, 7 spp 1.37 / 1.49, 640x360, 16 spp 10.1 / 9.1), and over many
+// objects they do not pay at any size (m = 30, scene tree of 6 levels, 256x256
+// 1.83 / 2.07; m = 100, 8 levels, 640x360 24.0 / 28.2; 300 spheres and meshes,
+// 10 levels, 97x61 0.42 / 0.56).
 //
 // The slices of a pixel go side by side into a warp where every SM has more
 // blocks than it holds at once: 480x270, 16 spp, on museum-like scenes of 480
@@ -200,10 +208,13 @@ int launch_plain(const DevScene &S, RenderArgs a, cudaStream_t st) {
     const auto stacks = [&](int h) {
         return (size_t) (a.tlas_cap + S.blas_depth + 1) * kTileW * h * sizeof(uint2);
     };
-    const bool sync = S.blas_depth <= kSyncDepth && stacks(kSyncTileH) <= 96 * 1024 &&
-                      blocks(kSyncTileH) >= 2 * device_sm_count();
+    const int spp = a.spp_end - a.spp_begin;
+    const int64_t fill = 2 * device_sm_count(); // blocks resident at once
+    const bool sync = S.blas_depth <= kSyncDepth && S.tlas_depth <= kSyncSceneDepth &&
+                      stacks(kSyncTileH) <= 96 * 1024 && blocks(kSyncTileH) >= fill &&
+                      blocks(kSyncTileH) / a.slices * spp >= fill * (1 + S.blas_depth);
     const int h = sync ? kSyncTileH : kTileH;
-    const bool even = (a.spp_end - a.spp_begin) % a.slices == 0;
+    const bool even = spp % a.slices == 0;
     if (blocks(kTileH) >= 8 * device_sm_count() && (even || !sync))
         while (a.group_log2 < 5 && (a.slices & ((2 << a.group_log2) - 1)) == 0)
             a.group_log2++;

@@ -50,3 +50,18 @@ def test_slices_side_by_side(cuda, size, spp, slices, small):
         acc = part if acc is None else acc + part
     want = acc / np.float32(spp)
     assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("level", [1, 2])
+def test_large_window_of_a_scene_with_deeper_meshes(cuda, level):
+    """Enough blocks for meshes of 6 and 8 levels to keep step (32 slices)."""
+    w, h = 330, 200
+    s = prr.Scene.from_desc(scenes.museum_like(w, h, level=level, env_size=(64, 32)))
+    whole, _ = s.render(32, 4, seed=5, mode="plain", slices=32)
+    whole = whole.cpu().numpy()
+    for y in range(0, h, 26):
+        for x in range(0, w, 50):
+            win = (x, y, min(x + 50, w), min(y + 26, h))
+            part, _ = s.render(32, 4, seed=5, mode="plain", slices=32, window=win)
+            assert np.array_equal(part.cpu().numpy().view(np.uint32),
+                                  np.ascontiguousarray(whole[y:win[3], x:win[2]]).view(np.uint32))
