@@ -513,74 +513,14 @@ __device__ __forceinline__ QueryStack<E> scene_col(const DevScene &S, const Trac
     return QueryStack<E>(smem, (E *) c.spill, own, c.stack_sm, c.stack_cap, S.check);
 }
 
-// 2,000,003 rays on 122,880 triangles with geometry, half of them incoherent:
-// 0.50 ms against 0.74 for one ray per thread; any hit 0.35 against 0.81.
-template <bool FEW> struct SceneClosest {
-    const DevScene &S;
-    const SceneArgs &a;
-    int32_t *out_obj, *out_prim;
-    float *out_t;
-    bool raw; // out_prim takes the leaf-order triangle index (k_scene_finish resolves it)
-    const QueryStack<uint2> col;
-    uint32_t idx = 0;
-    ClosestWalk<FEW> w;
-
-    __device__ __forceinline__ SceneClosest(const DevScene &scene, const SceneArgs &args,
-                                            int32_t *obj, int32_t *prim, float *t, bool leaf_order,
-                                            uint2 *smem, uint2 *own)
-        : S(scene), a(args), out_obj(obj), out_prim(prim), out_t(t), raw(leaf_order),
-          col(scene_col(scene, args.c, smem, own)) {}
-
-    __device__ __forceinline__ bool start(uint32_t i) {
-        idx = i;
-        if (w.start(S, load_ray(a.O, a.D, i), col))
-            return true;
-        finish();
-        return false;
-    }
-    __device__ __forceinline__ bool step() { return w.step(S, col); }
-    __device__ __forceinline__ void finish() {
-        out_obj[idx] = w.hit_obj;
-        out_t[idx] = w.best;
-        int prim = w.hit_tri;
-        if (!raw && w.hit_obj >= 0)
-            prim = prim >= 0 ? __ldg(&S.tri_meta[prim].id) : 0;
-        out_prim[idx] = prim;
-    }
-};
-
-template <bool FEW>
-__global__ void __maxnreg__(FEW ? 128 : 64)
-    k_scene_closest(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
-                    int32_t *out_obj, int32_t *out_prim, float *out_t, bool raw) {
-    extern __shared__ uint2 smem[];
-    uint2 own[kLocalStack];
-    SceneClosest<FEW> b(S, a, out_obj, out_prim, out_t, raw, smem, own);
-    trace_rays(b, a.n, a.c);
-}
-
-// Hit geometry of a scene query, one thread per ray, so its loads and stores
-// are coalesced: in the tracing kernel they would be made by a few lanes at a
-// time while the rest of their warp waits. out_prim holds leaf-order triangle
-// indices (-1 for a sphere) and is resolved here.
-__global__ void __launch_bounds__(256)
-    k_scene_finish(const __grid_constant__ DevScene S, const float *O, const float *D, int64_t n,
-                   const int32_t *obj, int32_t *prim, const float *ts, float *geo) {
-    const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const int ob = obj[i];
-    if (ob < 0)
-        return; // a miss: prim is -1, its geometry is left as it was
-    const int tri = prim[i];
-    const float ht = ts[i];
-    const RayD r = load_ray(O, D, i);
-    const DevObject &o = S.objects[ob];
+// Coordinates and normal of the hit of ray r on object ob at ht (tri: leaf-order
+// triangle index, of a mesh).
+__device__ __forceinline__ void hit_geometry(const DevScene &S, const RayD &r, const DevObject &o,
+                                             int tri, float ht, float *geo) {
     // hit coords (Triangle.cpp:37 / Sphere.hpp:37): origin + direction * t
     const float cx = r.ox + r.dx * ht, cy = r.oy + r.dy * ht, cz = r.oz + r.dz * ht;
     float nx, ny, nz;
     if (o.kind == kObjMesh) {
-        prim[i] = __ldg(&S.tri_meta[tri].id);
         nx = S.normals[(size_t) tri * 3 + 0];
         ny = S.normals[(size_t) tri * 3 + 1];
         nz = S.normals[(size_t) tri * 3 + 2];
@@ -602,7 +542,6 @@ __global__ void __launch_bounds__(256)
             }
         }
     } else {
-        prim[i] = 0;
         // normalize(coords - center) (Vector.hpp:103-111)
         nx = cx - o.cx;
         ny = cy - o.cy;
@@ -615,12 +554,83 @@ __global__ void __launch_bounds__(256)
             nz = nz * inv;
         }
     }
-    geo[i * 6 + 0] = cx;
-    geo[i * 6 + 1] = cy;
-    geo[i * 6 + 2] = cz;
-    geo[i * 6 + 3] = nx;
-    geo[i * 6 + 4] = ny;
-    geo[i * 6 + 5] = nz;
+    geo[0] = cx;
+    geo[1] = cy;
+    geo[2] = cz;
+    geo[3] = nx;
+    geo[4] = ny;
+    geo[5] = nz;
+}
+
+// 2,000,003 rays on 122,880 triangles with geometry, half of them incoherent:
+// 0.50 ms against 0.74 for one ray per thread; any hit 0.35 against 0.81.
+// Geometry: the FEW form writes it as a ray ends, which saves a launch (1,000 rays
+// with geometry in the museum-like scene of 7,680 triangles 61.8 -> 56.9 us, in
+// the Cornell box 40.4 -> 36.6). The other leaves it to k_scene_finish, as here a
+// few lanes at a time would make its loads and stores while the rest of their
+// warp waits.
+template <bool FEW> struct SceneClosest {
+    const DevScene &S;
+    const SceneArgs &a;
+    int32_t *out_obj, *out_prim;
+    float *out_t, *out_geo;
+    const QueryStack<uint2> col;
+    uint32_t idx = 0;
+    ClosestWalk<FEW> w;
+
+    __device__ __forceinline__ SceneClosest(const DevScene &scene, const SceneArgs &args,
+                                            int32_t *obj, int32_t *prim, float *t, float *geo,
+                                            uint2 *smem, uint2 *own)
+        : S(scene), a(args), out_obj(obj), out_prim(prim), out_t(t), out_geo(geo),
+          col(scene_col(scene, args.c, smem, own)) {}
+
+    __device__ __forceinline__ bool start(uint32_t i) {
+        idx = i;
+        if (w.start(S, load_ray(a.O, a.D, i), col))
+            return true;
+        finish();
+        return false;
+    }
+    __device__ __forceinline__ bool step() { return w.step(S, col); }
+    __device__ __forceinline__ void finish() {
+        out_obj[idx] = w.hit_obj;
+        out_t[idx] = w.best;
+        int prim = w.hit_tri;
+        if ((FEW || !out_geo) && w.hit_obj >= 0) {
+            prim = prim >= 0 ? __ldg(&S.tri_meta[prim].id) : 0;
+            if (FEW && out_geo)
+                hit_geometry(S, w.r, S.objects[w.hit_obj], w.hit_tri, w.best,
+                             out_geo + (size_t) idx * 6);
+        }
+        out_prim[idx] = prim;
+    }
+};
+
+template <bool FEW>
+__global__ void __maxnreg__(FEW ? 128 : 64)
+    k_scene_closest(const __grid_constant__ DevScene S, const __grid_constant__ SceneArgs a,
+                    int32_t *out_obj, int32_t *out_prim, float *out_t, float *geo) {
+    extern __shared__ uint2 smem[];
+    uint2 own[kLocalStack];
+    SceneClosest<FEW> b(S, a, out_obj, out_prim, out_t, geo, smem, own);
+    trace_rays(b, a.n, a.c);
+}
+
+// Hit geometry of a large scene query, one thread per ray, so its loads and
+// stores are coalesced. out_prim holds leaf-order triangle indices (-1 for a
+// sphere) and is resolved here.
+__global__ void __launch_bounds__(256)
+    k_scene_finish(const __grid_constant__ DevScene S, const float *O, const float *D, int64_t n,
+                   const int32_t *obj, int32_t *prim, const float *ts, float *geo) {
+    const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const int ob = obj[i];
+    if (ob < 0)
+        return; // a miss: prim is -1, its geometry is left as it was
+    const int tri = prim[i];
+    prim[i] = tri >= 0 ? __ldg(&S.tri_meta[tri].id) : 0;
+    hit_geometry(S, load_ray(O, D, i), S.objects[ob], tri, ts[i], geo + i * 6);
 }
 
 template <bool FEW> struct SceneAny {
@@ -1145,13 +1155,14 @@ int launch_scene_closest(const Scene &s, const float *o, const float *d, int64_t
     const int block = 128;
     SceneArgs a{o, d, (uint32_t) n, {}};
     TraceLaunch L;
-    auto kern = few_rays(n) ? k_scene_closest<true> : k_scene_closest<false>;
+    const bool few = few_rays(n);
+    auto kern = few ? k_scene_closest<true> : k_scene_closest<false>;
     if (int rc = plan_trace(L, a.c, (const void *) kern, block,
                             stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
                             sizeof(uint2), n, 0, 8, false, nullptr, capturing(st), st))
         return rc;
-    kern<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo != nullptr);
-    if (geo)
+    kern<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo);
+    if (geo && !few)
         k_scene_finish<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(s.dev, o, d, n, obj, prim, t,
                                                                      geo);
     PRR_CUDA_TRY(cudaGetLastError());
