@@ -11,7 +11,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <limits>
+#include <system_error>
 #include <thread>
 
 namespace prr {
@@ -182,8 +184,12 @@ void pack_quads(const FlatBVH &f, bool object_leaves, int tri_base, std::vector<
 // Appends one mesh's four-wide nodes, packed with references from 0, to the
 // scene's: moves node references by the nodes before them and leaf references
 // by the mesh's first triangle.
-void append_quads(const std::vector<QNode> &quads, uint32_t &root_ref, int tri_base,
+void append_quads(std::vector<QNode> &quads, uint32_t &root_ref, int tri_base,
                   std::vector<QNode> &out) {
+    if (out.empty() && tri_base == 0) { // nothing moves
+        out.swap(quads);
+        return;
+    }
     const uint32_t node_base = (uint32_t) out.size(), leaf_base = (uint32_t) tri_base << 2;
     auto moved = [&](uint32_t r) { return r + ((r & kLeafBit) ? leaf_base : node_base); };
     root_ref = moved(root_ref);
@@ -275,6 +281,11 @@ int build_scene(Scene &s, cudaStream_t st) {
         if (s.objects[k].kind == kObjMesh)
             meshes.push_back((int) k);
     const int hw = (int) std::max(1u, std::thread::hardware_concurrency());
+    // The four-wide nodes of large meshes are packed aside while the triangles
+    // are laid out below (1,000,000 triangles: 36 ms of packing; the build 313 ->
+    // 297 ms, 289 without those nodes). Small meshes' are packed by the threads
+    // that build them: six of 81,920 took 88 ms so and 108 aside.
+    std::vector<std::future<void>> packing(s.objects.size());
     auto build_one = [&](int k, int threads) {
         HostObject &o = s.objects[k];
         std::vector<PrimBox> pb;
@@ -288,7 +299,15 @@ int build_scene(Scene &s, cudaStream_t st) {
         for (float x : pa)
             a += x;
         o.area = a;
-        pack_quads(o.bvh, false, 0, o.quads, o.qroot, o.qstack);
+        auto pack = [&o] { pack_quads(o.bvh, false, 0, o.quads, o.qroot, o.qstack); };
+        if (threads > 1) {
+            try {
+                packing[k] = std::async(std::launch::async, pack);
+                return;
+            } catch (const std::system_error &) { // no thread to be had
+            }
+        }
+        pack();
     };
     {
         // big meshes get the threads; small ones run side by side
@@ -392,6 +411,8 @@ int build_scene(Scene &s, cudaStream_t st) {
         }
         if (int rc = pack_tree(o.bvh, false, base, nodes, o.root))
             return rc;
+        if (packing[k].valid())
+            packing[k].get();
         append_quads(o.quads, o.qroot, base, qnodes);
         std::vector<QNode>().swap(o.quads);
         blas_stack = std::max(blas_stack, o.qstack);
