@@ -1061,6 +1061,8 @@ __device__ float warp_estimate(const GridView &v, V3 pos, int k, int found, Warp
         __syncwarp();
         if (found < 0) { // the walk at t = r: every photon inside
             found = c;
+            if (c == 0) // whatever the disc's area rounds to
+                return 0.f;
             if (c <= k) { // the fixed-radius estimate (k <= kMaxK fit)
                 for (int base = 0; base < c; base += 32) {
                     const int q = base + lane;

@@ -455,3 +455,16 @@ def test_caustic_film_of_any_sample_count(cuda, spp):
         torch.cuda.synchronize()
         acc += one.cpu().numpy()
     assert np.array_equal(got.view(np.uint32), (acc / np.float32(spp)).view(np.uint32))
+
+
+@pytest.mark.parametrize("k", [0, 8])
+def test_gather_without_photons_is_zero_at_any_radius(cuda, k):
+    """A radius whose disc's area rounds to 0: still 0 where no photon lies."""
+    rng = np.random.default_rng(6)
+    rec = np.zeros((500, 9), np.float32)
+    rec[:, 0:3] = rng.uniform(-1, 1, (500, 3))
+    rec[:, 4] = -1.0
+    rec[:, 6:9] = 1.0
+    pm = prr.PhotonMap().set(rec).build(1e-24)
+    q = rng.uniform(-1, 1, (300, 3)).astype(np.float32)
+    assert not pm.gather(q, k_nearest=k).cpu().numpy().any()
