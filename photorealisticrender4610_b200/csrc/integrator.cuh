@@ -92,10 +92,6 @@ __device__ __forceinline__ V3 clamp_indirect(V3 c, float clamp) {
     return (lum > clamp) ? c * (clamp / lum) : c;
 }
 
-#ifndef CAST_OUTLINE
-#define CAST_OUTLINE true
-#endif
-constexpr bool kCastOutline = CAST_OUTLINE;
 struct PathCounters {
     uint32_t closest, shadow; // rays traced by this path
 };
@@ -198,7 +194,7 @@ static __device__ V3 cast_ray(const DevScene &S, Ray3 ray, int max_depth, float 
         const V3 gn = in.n;
         const bool delta = m.kind == kMatMirror || m.kind == kMatGlass;
         const V3 sn = delta || dot(cur.d, gn) < 0.f ? gn : -gn;
-        const Shading sd = build_shading<kCastOutline>(S, m, sn, in.a);
+        const Shading sd = build_shading<true>(S, m, sn, in.a);
         const V3 wo = -cur.d;
         if (delta) {
             // delta chain (Integrator.cpp:143-169)

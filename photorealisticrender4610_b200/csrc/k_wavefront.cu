@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(kSurfaceBlock, 2)
                 const V3 cd = ld3(w.rd, p);
                 const V3 hp = in.p;
                 const V3 sn = dot(cd, in.n) < 0.f ? in.n : -in.n;
-                const Shading sd = build_shading<kCastOutline>(S, m, sn, in.a);
+                const Shading sd = build_shading<true>(S, m, sn, in.a);
                 const V3 wo = -cd;
                 const float indirect = it > 0 ? 1.f : 0.f;
                 // The three directions that leave the hit: towards an emitter,
