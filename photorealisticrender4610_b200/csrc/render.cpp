@@ -201,9 +201,9 @@ extern "C" int prr_autotune(prr_scene *scene, const prr_render_settings *setting
     if (rc == PRR_OK)
         trial(prr_wavefront_config{shape2.paths_per_pass, shape2.block_size, 1,
                                    shape2.stack_smem, 0, 0});
-    // stage 4: the refill threshold of the traversal stages (so far the default, 12)
+    // stage 4: the refill threshold of the traversal stages
     const prr_wavefront_config shape3 = best;
-    for (int rf : {4, 8, 16})
+    for (int rf : {4, 12, 16})
         if (rc == PRR_OK)
             trial(prr_wavefront_config{shape3.paths_per_pass, shape3.block_size, 1,
                                        shape3.stack_smem, shape3.ordered, rf});
