@@ -186,14 +186,16 @@ def parse_launch(text):
 
 
 def traversal_work(verts, o, d, threads):
-    """Mean interior visits I and triangle tests T per ray, counted by the
-    oracle's traversal on the same rays (sample of 2^20 rays)."""
+    """Mean interior visits I, those I4 at every other level (what the kernels'
+    four-wide nodes, two levels in one, are visited) and triangle tests T per
+    ray, counted by the oracle's traversal on the same rays (2^20 of them)."""
     from oracle.loader import PortOracle
     port = PortOracle()
     m = port.mesh(verts)
     k = min(len(o), 1 << 20)
     _, _, _, vis, tst = m.intersect(o[:k], d[:k], threads=threads, stats=True)
-    return float(vis.mean()), float(tst.mean())
+    even = m.even_visits(o[:k], d[:k], threads=threads)
+    return float(vis.mean()), float(even.mean()), float(tst.mean())
 
 
 _CPU_MESH = {}
@@ -385,8 +387,8 @@ def run_ours(args, rank, world, on):
     if rank != 0:
         return 0
     threads = os.cpu_count() or 1
-    I, T = traversal_work(verts, o, d, threads)
-    bytes_per_ray = 24 + 8 + 64 * I + 36 * T
+    I, I4, T = traversal_work(verts, o, d, threads)
+    bytes_per_ray = 24 + 8 + 112 * I4 + 36 * T
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_ray * N_RAYS / (float(np.mean(kernel_ms)) * 1e-3) / 1e9
     traffic = profiled_traffic("k_mesh_closest")
@@ -411,7 +413,8 @@ def run_ours(args, rank, world, on):
                                 "stay in L2 (DRAM a few % busy), about 12 of 32 lanes active "
                                 "per warp instruction",
                      "peak_source": f"{peak_kind} hbm_gbs",
-                     "bytes_per_ray": bytes_per_ray, "interior_visits": I, "tri_tests": T},
+                     "bytes_per_ray": bytes_per_ray, "four_wide_visits": I4,
+                     "binary_visits": I, "tri_tests": T},
         "cpu_baseline": {"value": cpu_rate, "unit": "Mrays/s", "cores": threads,
                          "kind": cpu_kind, "sample": f"all {N_RAYS} query rays, one pass",
                          "one_core": {"value": cpu_rate_1, "sample": "first 131072 query rays"}},
@@ -463,8 +466,8 @@ RENDER_WORKLOADS = {
 }
 
 
-# Algorithmic bytes of a wavefront frame, per unit of work counted by
-# prr_render_counts: a closest-hit ray reads its origin and direction (24 B)
+# Algorithmic bytes of a wavefront frame over the binary trees, per unit of work
+# counted by prr_render_counts: a closest-hit ray reads its origin and direction (24 B)
 # and writes its hit record (16 B); a shadow ray reads origin, direction and
 # tmax (28 B) and writes its visibility byte; each interior node visited reads
 # the two child boxes of one 64 B node, each triangle test the 36 B of v0, e1,
@@ -590,13 +593,15 @@ def render_result(args, rank, world, on, workload, steps, warmup, crop_check=Fal
         return None
     peak, peak_kind = measured_peaks()
     alg = frame_bytes(counts, npix)
-    achieved = alg / (wf_step * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": None,
+    # no rate: the counts are of the binary trees, the timed stages walk four-wide
+    # nodes and fetch less
+    roofline = {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s",
+                "frac": None, "traffic": None,
                 "peak_source": f"{peak_kind} hbm_gbs",
-                "basis": "algorithmic bytes of the whole wavefront frame (traversal steps "
-                         "and hit classes counted by prr_render_counts, bytes per unit in "
-                         "bench.FRAME_BYTES) / frame time",
+                "basis": "bytes_per_frame: algorithmic bytes of the whole wavefront frame over "
+                         "the binary trees (traversal steps and hit classes counted by "
+                         "prr_render_counts, bytes per unit in bench.FRAME_BYTES); the "
+                         "timed stages walk four-wide nodes, so it gives no rate of theirs",
                 "bytes_per_frame": alg, "bytes_per_unit": FRAME_BYTES,
                 "counts": counts,
                 "nodes_per_closest_ray": counts["closest_nodes"] / max(1, counts["closest_rays"]),

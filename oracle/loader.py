@@ -89,6 +89,8 @@ class PortOracle:
                                             C.c_void_p, C.c_void_p]
         L.prr_oracle_mesh_intersect.argtypes = [C.c_void_p, _f32p, _f32p, C.c_int64, _i32p, _f32p,
                                                 C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]
+        L.prr_oracle_mesh_even_visits.argtypes = [C.c_void_p, _f32p, _f32p, C.c_int64, _i32p,
+                                                  C.c_int]
         L.prr_oracle_mesh_occluded.argtypes = [C.c_void_p, _f32p, _f32p, _f32p, C.c_int64, _u8p,
                                                C.c_int]
         L.prr_oracle_tonemap.argtypes = [C.c_int, C.c_float, _f32p, C.c_int64, _f32p, _u8p]
@@ -185,6 +187,15 @@ class PortMesh:
         if stats:
             return hid, t, t64, vis, tst
         return hid, t, t64
+
+    def even_visits(self, o, d, threads=0):
+        """Interior nodes each ray visits at even levels of the tree."""
+        o = _c(o, np.float32).reshape(-1, 3)
+        d = _c(d, np.float32).reshape(-1, 3)
+        vis = np.empty(len(o), np.int32)
+        self.port.L.prr_oracle_mesh_even_visits(self.h, o, d, len(o), vis,
+                                                threads or os.cpu_count())
+        return vis
 
     def occluded(self, o, d, tmax, threads=0):
         o = _c(o, np.float32).reshape(-1, 3)

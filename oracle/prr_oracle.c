@@ -573,7 +573,7 @@ static double tri_t64(const float *p, v3 of, v3 df) {
 
 /* BVHAccel::Intersect, triangle fast path (BVH.cpp:311-415). */
 static int32_t closest(const prr_oracle_mesh *m, v3 o, v3 d, float *tout, int32_t *nvis,
-                       int32_t *ntest) {
+                       int32_t *neven, int32_t *ntest) {
     if (m->nnodes == 0) {
         *tout = INFINITY;
         return -1;
@@ -581,11 +581,12 @@ static int32_t closest(const prr_oracle_mesh *m, v3 o, v3 d, float *tout, int32_
     rdata rd = precompute(o, d);
     uint32_t st_idx[64];
     float st_t[64];
-    int sp = 0;
+    uint8_t st_odd[64];
+    int sp = 0, odd = 0; /* level of ni, modulo 2 */
     uint32_t ni = 0;
     float closest_t = INFINITY;
     int64_t hit = -1;
-    int32_t vis = 0, tst = 0;
+    int32_t vis = 0, even = 0, tst = 0;
     for (;;) {
         uint32_t meta = m->meta[ni];
         uint32_t cnt = meta & 0x00FFFFFFu;
@@ -601,6 +602,7 @@ static int32_t closest(const prr_oracle_mesh *m, v3 o, v3 d, float *tout, int32_
             }
         } else {
             vis++;
+            even += !odd;
             uint32_t left = ni + 1, right = m->fc[ni];
             float tl = node_isect(m->nb + (size_t) left * 6, &rd);
             float tr = node_isect(m->nb + (size_t) right * 6, &rd);
@@ -608,18 +610,22 @@ static int32_t closest(const prr_oracle_mesh *m, v3 o, v3 d, float *tout, int32_
                 if (tl < closest_t) {
                     if (tr < closest_t) {
                         st_idx[sp] = right;
+                        st_odd[sp] = (uint8_t) !odd;
                         st_t[sp++] = tr;
                     }
                     ni = left;
+                    odd = !odd;
                     continue;
                 }
             } else {
                 if (tr < closest_t) {
                     if (tl < closest_t) {
                         st_idx[sp] = left;
+                        st_odd[sp] = (uint8_t) !odd;
                         st_t[sp++] = tl;
                     }
                     ni = right;
+                    odd = !odd;
                     continue;
                 }
             }
@@ -628,6 +634,7 @@ static int32_t closest(const prr_oracle_mesh *m, v3 o, v3 d, float *tout, int32_
             if (sp == 0)
                 goto done;
             ni = st_idx[--sp];
+            odd = st_odd[sp];
             if (st_t[sp] < closest_t)
                 break;
         }
@@ -636,6 +643,8 @@ done:
     *tout = closest_t;
     if (nvis)
         *nvis = vis;
+    if (neven)
+        *neven = even;
     if (ntest)
         *ntest = tst;
     return hit < 0 ? -1 : m->tris[hit].id;
@@ -650,7 +659,7 @@ void prr_oracle_mesh_intersect(const prr_oracle_mesh *m, const float *o, const f
         v3 dd = mk(d[i * 3], d[i * 3 + 1], d[i * 3 + 2]);
         float tt;
         int32_t nv = 0, nt = 0;
-        int32_t h = closest(m, oo, dd, &tt, &nv, &nt);
+        int32_t h = closest(m, oo, dd, &tt, &nv, NULL, &nt);
         id[i] = h;
         t[i] = tt;
         if (t64)
@@ -659,6 +668,19 @@ void prr_oracle_mesh_intersect(const prr_oracle_mesh *m, const float *o, const f
             visits[i] = nv;
         if (tests)
             tests[i] = nt;
+    }
+}
+
+/* Interior nodes visited at even levels: the nodes a walk over two levels of
+ * the tree at a time visits (the root, its grandchildren and so on). */
+void prr_oracle_mesh_even_visits(const prr_oracle_mesh *m, const float *o, const float *d,
+                                 int64_t n, int32_t *visits, int nthreads) {
+#pragma omp parallel for schedule(dynamic, 1024) num_threads(nthreads > 0 ? nthreads : 1)
+    for (int64_t i = 0; i < n; i++) {
+        float tt;
+        visits[i] = 0;
+        closest(m, mk(o[i * 3], o[i * 3 + 1], o[i * 3 + 2]),
+                mk(d[i * 3], d[i * 3 + 1], d[i * 3 + 2]), &tt, NULL, &visits[i], NULL);
     }
 }
 

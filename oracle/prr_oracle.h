@@ -48,6 +48,10 @@ int64_t prr_oracle_mesh_nodes(const prr_oracle_mesh *m, float *bounds, uint32_t 
 void prr_oracle_mesh_intersect(const prr_oracle_mesh *m, const float *o, const float *d,
                                int64_t n, int32_t *id, float *t, double *t64, int32_t *visits,
                                int32_t *tests, int nthreads);
+/* visits: interior nodes visited at even levels (root 0), what a walk over two
+ * levels at a time visits. */
+void prr_oracle_mesh_even_visits(const prr_oracle_mesh *m, const float *o, const float *d,
+                                 int64_t n, int32_t *visits, int nthreads);
 void prr_oracle_mesh_occluded(const prr_oracle_mesh *m, const float *o, const float *d,
                               const float *tmax, int64_t n, uint8_t *hit, int nthreads);
 
