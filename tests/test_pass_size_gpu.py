@@ -26,13 +26,16 @@ def test_adaptive_passes_do_not_grow_with_the_budget(cuda):
 
 @pytest.mark.parametrize("ordered", [True, False])
 @pytest.mark.parametrize("threshold", [1e9, 0.5])
-def test_passes_after_the_last_pixel_stopped(cuda, ordered, threshold):
+@pytest.mark.parametrize("per_pass", [4, 85, 86, 256])
+def test_passes_after_the_last_pixel_stopped(cuda, ordered, threshold, per_pass):
     """Passes, and bounces of a pass, without paths: image and sample counts are
-    the plain adaptive renderer's."""
+    the plain adaptive renderer's. (From 128 tiles of 4,096 paths on, 85.3
+    samples of 96x64, partitions look for that.)"""
     s = prr.Scene.from_desc(scenes.cornell_box(96, 64))
-    s.set_wavefront(paths_per_pass=96 * 64 * 4, stack_smem=8, ordered=ordered)
-    got, n = s.render(32, 12, mode="wavefront", min_spp=1, threshold=threshold)
-    want, m = s.render(32, 12, mode="plain", min_spp=1, threshold=threshold)
+    s.set_wavefront(paths_per_pass=96 * 64 * per_pass, stack_smem=8, ordered=ordered)
+    spp = 4 * per_pass
+    got, n = s.render(spp, 12, mode="wavefront", min_spp=1, threshold=threshold)
+    want, m = s.render(spp, 12, mode="plain", min_spp=1, threshold=threshold)
     assert torch.equal(n, m) and torch.equal(got, want)
 
 
