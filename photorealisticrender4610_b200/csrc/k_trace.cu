@@ -972,11 +972,14 @@ bool capturing(cudaStream_t st) {
 constexpr int64_t kMaxLaunch = int64_t(1) << 31;
 
 // Batches traced by the FEW form of a kernel: up to 640 rays per SM, what its
-// residents (5 blocks of 128) hold at once. Closest hit on one mesh takes it up
-// to twice that, its rays being slower apart than the larger batch's queueing
-// (100,000 triangles: 140,000 rays 454 -> 386 us, 180,000 479 -> 448, 250,000
-// 552 -> 546, 400,000 722 -> 753; scene level 100,000 rays 115 -> 108, 140,000
-// 115 -> 122).
+// residents (4 or 5 blocks of 128) hold at once or little more. Closest hit on
+// one mesh takes it to 740, and on large meshes (walks of 24 stack entries and
+// more, from about 50,000 triangles on) to 1,280, their rays being slower apart
+// than the larger batch's queueing. Times of the form over the other's, at
+// 110,000, 130,000 and 160,000 rays: 1,000 triangles 1.03, 1.10, 1.13; 10,000
+// 0.97, 1.05, 1.05; 100,000 0.83, 0.84, 0.90; 1,000,000 0.87, 0.89, 0.88 (250,000
+// rays 0.96); scene level, museum-like of 1,920 to 491,520 triangles, 94,000
+// rays 0.89 to 0.84, 130,000 1.06 to 0.93.
 bool few_rays(int64_t n, int per_sm = 640) { return n <= (int64_t) device_sm_count() * per_sm; }
 
 // Launch shape of a query kernel over n rays: shared memory, grid, and the
@@ -988,8 +991,16 @@ struct TraceLaunch {
     CallScratch scratch;
 };
 
+//
+// A counter costs a call an allocation, a clear and the atomics, so rays are
+// counted out only when a warp's share is more than a few rounds of its lanes
+// (count_from). Closest hit on one mesh: one round, 32 (10,000 triangles,
+// 200,000 rays 260 us, 275 with fixed shares of two). The other queries, whose
+// rays differ less: two, 64 (94,000 rays, counted / fixed: any hit on 10,000
+// triangles 40.9 / 35.5 us, closest hit in the Cornell box 18.4 / 15.0, in the
+// museum-like scene of 30,720 triangles 78.9 / 74.5, of 491,520 105 / 107).
 int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, size_t entry,
-               int64_t n, int blocks_per_sm, int refill, bool counter_always,
+               int64_t n, int blocks_per_sm, int refill, int count_from, bool counter_always,
                unsigned *counter, bool in_capture, cudaStream_t st) {
     c.stack_cap = cap;
     c.stack_sm = std::min(cap, kStackSm);
@@ -1016,7 +1027,7 @@ int plan_trace(TraceLaunch &L, TraceCfg &c, const void *fn, int block, int cap, 
     c.refill = std::min(refill, c.lanes);
     const int64_t per_block = (int64_t) c.lanes * (block / 32);
     L.grid = (unsigned) std::min<int64_t>(resident, (n + per_block - 1) / per_block);
-    const bool count = counter_always || (n > warps * 32 && !in_capture);
+    const bool count = counter_always || (n > warps * count_from && !in_capture);
     size_t bytes = count && !counter ? 256 : 0;
     const size_t spill_at = bytes;
     if (!local)
@@ -1075,7 +1086,8 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     // allocate nothing; every other call gets its own
     if (in_capture && mode > 0 && !counter)
         counter = (unsigned *) s.d_counter.ptr;
-    const bool few = mode == 0 && block <= kFewBlock && few_rays(n, 1280);
+    const bool few =
+        mode == 0 && block <= kFewBlock && few_rays(n, obj.qstack >= 24 ? 1280 : 740);
     const int cap = stack_cap(obj.qstack);
     const void *fn = mode == 1   ? (const void *) k_mesh_closest_persistent
                      : mode == 3 ? (const void *) k_mesh_closest_phased
@@ -1084,7 +1096,7 @@ int launch_mesh_closest(const Scene &s, int object, const float *o, const float 
     const int refill = mode >= 2 && cfg->batch > 0 ? std::min(cfg->batch, 32) : 8;
     TraceLaunch L;
     if (int rc = plan_trace(L, a.c, fn, block, cap, sizeof(uint2), n,
-                            mode > 0 ? cfg->blocks_per_sm : 0, refill, mode > 0, counter,
+                            mode > 0 ? cfg->blocks_per_sm : 0, refill, 32, mode > 0, counter,
                             in_capture, st))
         return rc;
     CallScratch order;
@@ -1136,7 +1148,7 @@ int launch_mesh_occluded(const Scene &s, int object, const float *o, const float
     TraceLaunch L;
     auto kern = few_rays(n) ? k_mesh_occluded<true> : k_mesh_occluded<false>;
     if (int rc = plan_trace(L, a.c, (const void *) kern, block, stack_cap(obj.qstack),
-                            sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
+                            sizeof(uint32_t), n, 0, 8, 64, false, nullptr, capturing(st), st))
         return rc;
     kern<<<L.grid, block, L.smem, st>>>(a, box, tmax, hit);
     PRR_CUDA_TRY(cudaGetLastError());
@@ -1159,7 +1171,7 @@ int launch_scene_closest(const Scene &s, const float *o, const float *d, int64_t
     auto kern = few ? k_scene_closest<true> : k_scene_closest<false>;
     if (int rc = plan_trace(L, a.c, (const void *) kern, block,
                             stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
-                            sizeof(uint2), n, 0, 8, false, nullptr, capturing(st), st))
+                            sizeof(uint2), n, 0, 8, 64, false, nullptr, capturing(st), st))
         return rc;
     kern<<<L.grid, block, L.smem, st>>>(s.dev, a, obj, prim, t, geo);
     if (geo && !few)
@@ -1183,7 +1195,7 @@ int launch_scene_occluded(const Scene &s, const float *o, const float *d, const 
     auto kern = few_rays(n) ? k_scene_occluded<true> : k_scene_occluded<false>;
     if (int rc = plan_trace(L, a.c, (const void *) kern, block,
                             stack_cap(s.dev.blas_stack + s.dev.tlas_stack),
-                            sizeof(uint32_t), n, 0, 8, false, nullptr, capturing(st), st))
+                            sizeof(uint32_t), n, 0, 8, 64, false, nullptr, capturing(st), st))
         return rc;
     kern<<<L.grid, block, L.smem, st>>>(s.dev, a, tmax, hit);
     PRR_CUDA_TRY(cudaGetLastError());

@@ -128,3 +128,26 @@ def test_wavefront_blocks_on_a_deep_scene_tree(cuda):
         s.set_wavefront(block_size=block, stack_smem=stack)
         got, n = s.render(2, 4, mode="wavefront")
         assert torch.equal(got, want) and torch.equal(n, spp), (block, stack)
+
+
+# where the scene and any-hit queries change kernels (640 rays per SM), and
+# where they begin to hand out rays from a counter (64 rays a warp: 2 x 75,776
+# for the 4 resident blocks of the small batches' form, 2 x 151,552 for 8)
+@pytest.mark.parametrize("rays", [75_777, 94_720, 94_721, 151_553, 303_104, 303_105, 340_993])
+def test_scene_and_any_hit_batch_sizes(port, cuda, rays):
+    v, o, d = scenes.query_set(400, rays, seed=2)
+    tmax = np.linspace(0.05, 2, rays, dtype=np.float32)
+    m = port.mesh(v)
+    want = m.intersect(o, d)
+    occ = np.asarray(m.occluded(o, d, tmax)) > 0
+    s = prr.Scene.single_mesh(v)
+    to, td, tm = (torch.from_numpy(a).to(cuda) for a in (o, d, tmax))
+    ob, prim, t, geo = s.intersect(to, td, geo=True)
+    equal((prim, t), want)
+    hit = want[0] >= 0
+    # coords as Triangle::finalize forms them: origin + direction * t
+    coords = o + d * want[1][:, None]
+    assert np.array_equal(geo.cpu().numpy()[hit, :3].view(np.uint32),
+                          coords[hit].view(np.uint32))
+    assert np.array_equal(s.mesh_occluded(0, to, td, tm).cpu().numpy() > 0, occ)
+    assert np.array_equal(s.intersectP(to, td, tm).cpu().numpy() > 0, occ)
