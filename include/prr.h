@@ -114,7 +114,10 @@ typedef struct prr_render_settings {
     int slices;               /* plain fixed-spp mode: threads per pixel (0 = automatic) */
 } prr_render_settings;
 
-/* Wavefront launch shape (chosen by prr_autotune; zero fields = defaults). */
+/* Wavefront launch shape (chosen by prr_autotune; zero fields mean what their
+ * comments say). Before the first prr_scene_set_wavefront or prr_autotune a scene
+ * has paths_per_pass 0, block_size 0, use_graphs 1, stack_smem 8, ordered 1 and
+ * refill 0. */
 typedef struct prr_wavefront_config {
     int64_t paths_per_pass; /* paths in flight per pass (0: up to 32M, fewer where they would
                                take over a quarter of the free device memory, and 8M for
@@ -122,8 +125,9 @@ typedef struct prr_wavefront_config {
                                memory each) */
     int block_size;         /* threads per block of the traversal stages (0: 128) */
     int use_graphs;         /* 1: replay each pass from one captured CUDA graph */
-    int stack_smem;         /* mesh-BVH stack entries per thread kept in shared memory;
-                               deeper entries spill to a global buffer (0: the whole stack) */
+    int stack_smem;         /* mesh-BVH stack entries per thread kept in shared memory, as far
+                               as 96 KB a block allow; deeper entries spill to a global
+                               buffer (0: the whole stack) */
     int ordered;            /* 1: rebuild the stage queues in path order (stable partition,
                                next rays grouped by direction octant); 0: append order */
     int refill;             /* traversal stages: a warp takes new rays from its queue once

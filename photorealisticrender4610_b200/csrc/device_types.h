@@ -94,7 +94,8 @@ enum MaterialKind : int32_t { kMatDiffuse = 0, kMatEmissive = 1, kMatMirror = 2,
 struct alignas(16) DevObject {
     int32_t kind;
     int32_t material;
-    uint32_t root;      // mesh: root reference into nodes/tris (light sampling)
+    uint32_t root;      // mesh: root reference into nodes/tris (light sampling, and the walks
+                        // of kernels that run a whole path per thread)
     int32_t tri_base;   // mesh: first triangle (global index)
     float root_box[6];  // own bounds (IntersectP tests the root box first)
     float area;         // MeshTriangle::area or Sphere::area
@@ -104,7 +105,7 @@ struct alignas(16) DevObject {
     int32_t depth;      // max leaf depth of the mesh BVH (stack bound)
     int32_t attr;       // mesh: kAttr* bits of the per-corner data it carries
     int32_t attr_base;  // mesh: its first record in DevScene::attr
-    uint32_t qroot;     // mesh: root reference into qnodes/tris (the traversals')
+    uint32_t qroot;     // mesh: root reference into qnodes/tris (batch queries, wavefront)
     int32_t pad[1];
 };
 

@@ -780,9 +780,6 @@ __device__ __noinline__ V3 knn_estimate(const GridView &v, const GatherBox &b, V
 
 constexpr int kMaxK = 64;
 
-// Caustic render: per (pixel, sample), follow the camera ray through the
-// specular chain as castRay does (Integrator.cpp:143-169) and, at the first
-// non-delta hit, estimate the caustic radiance baseColor/pi * E(x).
 // Division of n < 2^31 by a fixed d >= 1: with s = ceil(log2 d) and m =
 // ceil(2^(31 + s) / d) < 2^32, n / d = (n m) >> (31 + s) (Granlund and
 // Montgomery 1994, theorem 4.2 for 31-bit n: m d - 2^(31 + s) < d <= 2^s). The
@@ -804,6 +801,9 @@ struct FastDiv {
     }
 };
 
+// Caustic render: per (pixel, sample), follow the camera ray through the
+// specular chain as castRay does (Integrator.cpp:143-169) and, at the first
+// non-delta hit, estimate the caustic radiance baseColor/pi * E(x).
 struct CausticArgs {
     FastDiv by_chunk, by_ww;
     int W, x0, y0, ww, wh, spp, max_depth, k_nearest, tlas_cap;

@@ -102,8 +102,8 @@ __device__ __forceinline__ void write_hit(const MeshArgs &a, int64_t i, const Ra
 // 174 with 32 rays a warp over the binary nodes; 20,000 rays on 300,000: 320
 // against 444).
 //
-// Rays come from the counter, or, without one (small batches, where a share
-// is a single round, and calls under stream capture, which allocate nothing),
+// Rays come from the counter, or, without one (batches of one or two rounds of
+// the grid's lanes, and calls under stream capture, which allocate nothing),
 // from a contiguous share per warp.
 template <class Body>
 __device__ __forceinline__ void trace_rays(Body &b, uint32_t n, const TraceCfg &c) {

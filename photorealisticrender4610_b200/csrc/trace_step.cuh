@@ -1,10 +1,11 @@
 // Two-level scene traversal as resumable per-lane state machines, for
 // persistent kernels whose lanes take new rays as soon as theirs finish.
 // Each call to step() does one unit of work -- one four-wide node of either
-// level, or one triangle -- and leaves are taken in exactly the order of the
-// walks in trace.cuh (scene_closest / scene_occluded, which restate
-// BVH.cpp:311-473 over MeshTriangle and Sphere leaves), so results are
-// identical; only the scheduling of rays onto lanes changes.
+// level, or one triangle. Results are those of the walks in trace.cuh
+// (scene_closest / scene_occluded, which restate BVH.cpp:311-473 over
+// MeshTriangle and Sphere leaves): closest hit takes the leaves in exactly their
+// order; any hit takes the same leaves, near ones first, and its answer does not
+// depend on the order.
 //
 // Both levels are four-wide nodes, and one stack holds the entries of both:
 // those of the mesh being walked lie above the scene's (from `floor` up). So a
